@@ -119,7 +119,8 @@ int walk_sorted(mb2_state* s, const std::vector<double>& u, uint64_t* basis) {
     auto* dev_basis = reinterpret_cast<uint64_t*>(base + al_u);
     MB2_CUDA(s->ctx, cudaMemcpyAsync(dev_u, u.data(), shots * 8, cudaMemcpyHostToDevice, s->stream));
     const int rc =
-        mb2::launch_sample(s->amps, s->n, dev_u, shots, base + 2 * al_u, dev_basis, s->stream, s->precision);
+        mb2::launch_sample(s->amps, s->n, dev_u, shots, nullptr, nullptr, base + 2 * al_u, dev_basis, s->stream,
+                           s->precision);
     if (rc != MB2_OK) return fail(s->ctx, rc, std::string("sample launch: ") + mb2::last_cuda_error_string());
     MB2_CUDA(s->ctx, cudaMemcpyAsync(basis, dev_basis, shots * 8, cudaMemcpyDeviceToHost, s->stream));
     MB2_CUDA(s->ctx, cudaStreamSynchronize(s->stream));
@@ -199,8 +200,12 @@ uint64_t scratch_bound(uint32_t n, const mb2_op* ops, uint32_t num_ops, uint64_t
     uint64_t program = 4 * 256;
     for (uint32_t i = 0; i < num_ops; ++i)
         if (ops[i].opcode != MB2_MEASURE) program += 144 + (16ull << (2 * ops[i].num_qubits));
-    // The sampler (walk_sorted): uniforms, per-shot basis, the walk's scratch.
-    const uint64_t sample = shots == 0 ? 0 : 2 * up(8 * shots) + sample_scratch_bytes(n, shots);
+    // The sampler (device_counts): uniforms, per-shot basis, the walk's
+    // scratch, and the sort's or the counts'.
+    const uint64_t sample =
+        shots == 0 ? 0
+                   : 2 * up(8 * shots) + sample_scratch_bytes(n, shots) +
+                         std::max<uint64_t>(uniforms_scratch_bytes(shots), up(8 * shots) + runs_scratch_bytes(shots));
     // The expectation (mb2_expectation): masks, partials, results, the
     // groups' span vectors (at most 2^kPauliMaxSpan per group) and terms.
     const uint64_t t = terms;
@@ -1051,6 +1056,18 @@ std::vector<double> sorted_uniforms(uint64_t shots, uint64_t seed) {
     return u;
 }
 
+// Whether every qubit is read into the clbit of its own number: the outcome
+// of a basis state is the state itself.
+bool identity_targets(uint32_t n, const uint32_t* targets, uint32_t num_targets) {
+    if (num_targets != n) return false;
+    uint64_t seen = 0;
+    for (uint32_t t = 0; t < num_targets; ++t) {
+        if (targets[2 * t] != targets[2 * t + 1]) return false;
+        seen |= uint64_t{1} << targets[2 * t];
+    }
+    return seen == ((n >= 64) ? ~uint64_t{0} : ((uint64_t{1} << n) - 1));
+}
+
 // The walk's basis states (non-decreasing) as counts of the measured
 // outcomes, ascending: mb2_sample's output.
 int histogram(mb2_context* ctx, uint32_t n, const std::vector<uint64_t>& basis, const uint32_t* targets,
@@ -1063,18 +1080,12 @@ int histogram(mb2_context* ctx, uint32_t n, const std::vector<uint64_t>& basis, 
     // Outcome of a basis index: one table per byte of the index (the OR of
     // the target bits that byte carries), or the index itself when every
     // qubit is read into the clbit of its own number.
-    bool identity = num_targets == n;
+    const bool identity = identity_targets(n, targets, num_targets);
     std::vector<uint64_t> table(8 * 256, 0);
     for (uint32_t t = 0; t < num_targets; ++t) {
         const uint32_t q = targets[2 * t], c = targets[2 * t + 1];
-        if (q != c) identity = false;
         for (uint32_t v = 0; v < 256; ++v)
             if ((v >> (q & 7u)) & 1u) table[(q >> 3) * 256 + v] |= uint64_t{1} << c;
-    }
-    if (identity) {
-        uint64_t seen = 0;
-        for (uint32_t t = 0; t < num_targets; ++t) seen |= uint64_t{1} << targets[2 * t];
-        identity = seen == ((n >= 64) ? ~uint64_t{0} : ((uint64_t{1} << n) - 1));
     }
     const uint32_t nbytes = (n + 7) / 8;
     auto outcome_of = [&](uint64_t b) {
@@ -1109,6 +1120,60 @@ int histogram(mb2_context* ctx, uint32_t n, const std::vector<uint64_t>& basis, 
     return MB2_OK;
 }
 
+// `shots` draws from `seed` as counts of the measured outcomes, the state on
+// the device from the uniforms to the counts: walk(draw, u, sort, scratch,
+// basis) queues the walk (walk_bytes of scratch) of the sorted uniforms u,
+// which it draws into u itself where draw is not null (sort: scratch of the
+// sort's).  n: the qubits that a basis index holds.  Outcomes that are not the basis states
+// themselves are counted on the host (their order need not be the walk's).
+template <typename WALK>
+int device_counts(mb2_state* s, uint32_t n, uint64_t shots, uint64_t seed, const uint32_t* targets,
+                  uint32_t num_targets, uint64_t* outcomes, uint64_t* counts, uint64_t* num_outcomes,
+                  size_t walk_bytes, WALK walk) {
+    if (shots > uint64_t{1} << 40) return fail(s->ctx, MB2_ERR_RESOURCE, "too many shots");
+    const size_t al_u = (shots * 8 + 255) & ~size_t{255};
+    const size_t other = std::max(mb2::uniforms_scratch_bytes(shots), al_u + mb2::runs_scratch_bytes(shots));
+    // Where the device has no room for the sort (a state that nearly fills
+    // it), the uniforms are sorted and the outcomes counted on the host.
+    const int room = ensure_scratch(s, 2 * al_u + walk_bytes + other);
+    if (room != MB2_OK && room != MB2_ERR_RESOURCE) return room;
+    const bool on_device = room == MB2_OK;
+    if (!on_device)
+        if (int e = ensure_scratch(s, 2 * al_u + walk_bytes); e != MB2_OK) return e;
+    auto* base = static_cast<unsigned char*>(s->scratch);
+    auto* dev_u = reinterpret_cast<double*>(base);
+    auto* dev_basis = reinterpret_cast<uint64_t*>(base + al_u);
+    unsigned char* const rest = base + 2 * al_u + walk_bytes;
+    int rc;
+    std::vector<double> u;  // until the stream is synchronised
+    if (!on_device) {
+        u = sorted_uniforms(shots, seed);
+        MB2_CUDA(s->ctx, cudaMemcpyAsync(dev_u, u.data(), shots * 8, cudaMemcpyHostToDevice, s->stream));
+    }
+    rc = walk(on_device ? &seed : nullptr, dev_u, rest, base + 2 * al_u, dev_basis);
+    if (rc != MB2_OK) return fail(s->ctx, rc, std::string("sample launch: ") + mb2::last_cuda_error_string());
+    if (!on_device || !identity_targets(n, targets, num_targets)) {
+        std::vector<uint64_t> basis(shots);
+        MB2_CUDA(s->ctx, cudaMemcpyAsync(basis.data(), dev_basis, shots * 8, cudaMemcpyDeviceToHost, s->stream));
+        MB2_CUDA(s->ctx, cudaStreamSynchronize(s->stream));
+        return histogram(s->ctx, n, basis, targets, num_targets, outcomes, counts, num_outcomes);
+    }
+    auto* dev_outcomes = reinterpret_cast<uint64_t*>(dev_u);  // the uniforms have been placed
+    auto* dev_counts = reinterpret_cast<uint64_t*>(rest);
+    const uint64_t* dev_runs = nullptr;
+    rc = mb2::launch_runs(dev_basis, shots, rest + al_u, dev_outcomes, dev_counts, &dev_runs, s->stream);
+    if (rc != MB2_OK) return fail(s->ctx, rc, std::string("sample launch: ") + mb2::last_cuda_error_string());
+    uint64_t d = 0;
+    MB2_CUDA(s->ctx, cudaMemcpyAsync(&d, dev_runs, sizeof(d), cudaMemcpyDeviceToHost, s->stream));
+    MB2_CUDA(s->ctx, cudaStreamSynchronize(s->stream));
+    if (d > *num_outcomes) return fail(s->ctx, MB2_ERR_INVALID, "outcome capacity too small");
+    MB2_CUDA(s->ctx, cudaMemcpyAsync(outcomes, dev_outcomes, d * 8, cudaMemcpyDeviceToHost, s->stream));
+    MB2_CUDA(s->ctx, cudaMemcpyAsync(counts, dev_counts, d * 8, cudaMemcpyDeviceToHost, s->stream));
+    MB2_CUDA(s->ctx, cudaStreamSynchronize(s->stream));
+    *num_outcomes = d;
+    return MB2_OK;
+}
+
 }  // namespace
 
 namespace mb2 {
@@ -1131,10 +1196,11 @@ int mb2_sample(mb2_state* s, uint64_t shots, uint64_t seed, const uint32_t* targ
         *num_outcomes = 0;
         return MB2_OK;
     }
-    const std::vector<double> u = sorted_uniforms(shots, seed);
-    std::vector<uint64_t> basis(shots);
-    if (int e = walk_sorted(s, u, basis.data()); e != MB2_OK) return e;
-    return histogram(s->ctx, s->n, basis, targets, num_targets, outcomes, counts, num_outcomes);
+    return device_counts(s, s->n, shots, seed, targets, num_targets, outcomes, counts, num_outcomes,
+                         mb2::sample_scratch_bytes(s->n, shots), [&](const uint64_t* draw, double* u, void* sort, void* scratch, uint64_t* basis) {
+                             return mb2::launch_sample(s->amps, s->n, u, shots, draw, sort, scratch, basis, s->stream,
+                                                       s->precision);
+                         });
 }
 
 int mb2_sample_basis(mb2_state* s, const double* uniforms, uint64_t n, uint64_t* basis_out) {
@@ -1323,18 +1389,14 @@ int mb2_dm_sample(mb2_state* rho, uint32_t n, uint64_t shots, uint64_t seed, con
         *num_outcomes = 0;
         return MB2_OK;
     }
-    const std::vector<double> u = sorted_uniforms(shots, seed);
-    const size_t al_u = (shots * 8 + 255) & ~size_t{255};
-    if (int e = ensure_scratch(rho, 2 * al_u); e != MB2_OK) return e;
-    auto* base = static_cast<unsigned char*>(rho->scratch);
-    MB2_CUDA(rho->ctx, cudaMemcpyAsync(base, u.data(), shots * 8, cudaMemcpyHostToDevice, rho->stream));
-    const int rc = mb2::launch_dm_walk(rho->amps, n, reinterpret_cast<const double*>(base), shots,
-                                       reinterpret_cast<uint64_t*>(base + al_u), rho->stream);
-    if (rc != MB2_OK) return fail(rho->ctx, rc, std::string("walk launch: ") + mb2::last_cuda_error_string());
-    std::vector<uint64_t> basis(shots);
-    MB2_CUDA(rho->ctx, cudaMemcpyAsync(basis.data(), base + al_u, shots * 8, cudaMemcpyDeviceToHost, rho->stream));
-    MB2_CUDA(rho->ctx, cudaStreamSynchronize(rho->stream));
-    return histogram(rho->ctx, n, basis, targets, num_targets, outcomes, counts, num_outcomes);
+    return device_counts(rho, n, shots, seed, targets, num_targets, outcomes, counts, num_outcomes, 0,
+                         [&](const uint64_t* draw, double* u, void* sort, void*, uint64_t* basis) {
+                             if (draw != nullptr)
+                                 if (int rc = mb2::launch_sorted_uniforms(shots, *draw, sort, u, rho->stream);
+                                     rc != MB2_OK)
+                                     return rc;
+                             return mb2::launch_dm_walk(rho->amps, n, u, shots, basis, rho->stream);
+                         });
 }
 
 int mb2_norm_exact(mb2_state* s, double* out) {

@@ -383,8 +383,27 @@ size_t sample_scratch_bytes(uint32_t n, uint64_t shots);
 // The reference's sequential FP64 sum of |a_i|^2 over the state, bit for bit
 // (the sampler's exact chain; scratch: sample_scratch_bytes(n, 0)); synchronises.
 int launch_exact_norm(const void* amps, uint32_t n, void* scratch, double* host_total, void* stream, int precision);
-int launch_sample(const void* amps, uint32_t n, const double* dev_uniforms_sorted, uint64_t shots, void* scratch,
-                  uint64_t* dev_basis, void* stream, int precision = MB2_C128);
+// The same for `batch` states back to back, left on the device: state t's at
+// (*norms)[t * *pitch], in scratch (norms_scratch_bytes).
+size_t norms_scratch_bytes(uint32_t n, uint32_t batch);
+int launch_norms(const void* amps, uint32_t n, uint32_t batch, void* scratch, const double** norms, uint64_t* pitch,
+                 void* stream, int precision = MB2_C128);
+// draw == nullptr: dev_u holds the sorted uniforms.  Otherwise they are drawn
+// from the seed *draw into dev_u on the way (sort_scratch:
+// uniforms_scratch_bytes), the generator beside the chunk sums.
+int launch_sample(const void* amps, uint32_t n, double* dev_u, uint64_t shots, const uint64_t* draw,
+                  void* sort_scratch, void* scratch, uint64_t* dev_basis, void* stream, int precision = MB2_C128);
+// The reference's `shots` uniforms from `seed`, sorted, in device memory
+// (kernels_uniforms.cu; scratch: uniforms_scratch_bytes).
+size_t uniforms_scratch_bytes(uint64_t shots);
+int launch_sorted_uniforms(uint64_t shots, uint64_t seed, void* scratch, double* dev_u, void* stream);
+// The second half of it: the generator's words (at the head of scratch) sorted.
+int launch_sort_words(const uint64_t* words, uint64_t shots, void* scratch, double* dev_u, void* stream);
+// The distinct values of a non-decreasing list and how often each comes
+// (scratch: runs_scratch_bytes); *dev_runs: where their number is, on the device.
+size_t runs_scratch_bytes(uint64_t shots);
+int launch_runs(const uint64_t* dev_basis, uint64_t shots, void* scratch, uint64_t* dev_outcomes,
+                uint64_t* dev_counts, const uint64_t** dev_runs, void* stream);
 // complex64 precision path (kernels_c64.cu).
 constexpr uint32_t kMaxTileQubitsC64 = 13;
 // Default complex64 tile: 12 qubits, two CTAs per SM (measured faster per
@@ -462,7 +481,7 @@ int launch_expectation_finish(const double* dev_partials, uint32_t blocks, const
 // Density matrices (kernels_reduce.cu): rho as a 2n-qubit complex128 vector,
 // entry (r, c) at r | c << n.  Tr(P rho) per term (partials as
 // launch_expectation's, then the finish); the exact walk of the sorted
-// uniforms over rho's diagonal (one thread; n <= 15).
+// uniforms over rho's diagonal (one CTA; n <= 15).
 int launch_dm_trace(const void* rho, uint32_t n, const uint64_t* dev_x, const uint64_t* dev_z, uint32_t num_terms,
                     double* dev_partials, double* dev_out, void* stream);
 int launch_dm_walk(const void* rho, uint32_t n, const double* dev_uniforms_sorted, uint64_t shots,

@@ -44,6 +44,14 @@ class Counts(Mapping):
     def items(self):
         return zip(self.outcomes.tolist(), self.counts.tolist())
 
+    @classmethod
+    def of(cls, outcomes: np.ndarray, counts: np.ndarray, size: int) -> "Counts":
+        """The first `size` entries of a call's output arrays; copied only
+        where the arrays are much larger."""
+        if 2 * size < outcomes.size:
+            return cls(outcomes[:size].copy(), counts[:size].copy())
+        return cls(outcomes[:size], counts[:size])
+
     def to_dict(self) -> dict:
         return dict(self.items())
 
@@ -246,13 +254,13 @@ class DeviceState:
     def sample(self, shots: int, seed: int, targets) -> "Counts":
         t = np.ascontiguousarray(np.asarray(targets, np.uint32).ravel())
         cap = max(int(shots), 1)
-        outc = np.zeros(cap, np.uint64)
-        cnt = np.zeros(cap, np.uint64)
+        outc = np.empty(cap, np.uint64)
+        cnt = np.empty(cap, np.uint64)
         nout = C.c_uint64(cap)
         self._chk(lib().mb2_sample(self.h, shots, seed, t.ctypes.data if len(t) else None, len(t) // 2,
                                    outc.ctypes.data, cnt.ctypes.data, C.byref(nout)), "mb2_sample")
         d = nout.value
-        return Counts(outc[:d].copy(), cnt[:d].copy())
+        return Counts.of(outc, cnt, d)
 
     def copy_out(self) -> np.ndarray:
         dt = np.complex128 if self.precision == C128 else np.complex64
@@ -294,7 +302,7 @@ def trajectories(ctx: Context, circ: Circuit, count: int, seed: int, paulis=(), 
     d = nout.value if shots else 0
     return {"terms": means[:2 * T].view(np.complex128).copy() if T else None,
             "standard_error": se.value if T else None,
-            "counts": Counts(outc[:d].copy(), cnt[:d].copy()) if shots else None}
+            "counts": Counts.of(outc, cnt, d) if shots else None}
 
 
 class DensityMatrix:
@@ -341,8 +349,8 @@ class DensityMatrix:
         measurement of each target's clbit, mb2_dm_sample_readout)."""
         t = np.ascontiguousarray(np.asarray(targets, np.uint32).ravel())
         cap = max(int(shots), 1)
-        outc = np.zeros(cap, np.uint64)
-        cnt = np.zeros(cap, np.uint64)
+        outc = np.empty(cap, np.uint64)
+        cnt = np.empty(cap, np.uint64)
         nout = C.c_uint64(cap)
         if circuit is not None:
             arr, keep = to_mb2_ops(circuit)
@@ -356,7 +364,7 @@ class DensityMatrix:
                                           len(t) // 2, outc.ctypes.data, cnt.ctypes.data, C.byref(nout)),
                       "mb2_dm_sample")
         d = nout.value
-        return Counts(outc[:d].copy(), cnt[:d].copy())
+        return Counts.of(outc, cnt, d)
 
     def matrix(self) -> np.ndarray:
         """rho as a (2^n, 2^n) array, rho[r, c]."""
