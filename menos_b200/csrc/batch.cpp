@@ -22,8 +22,6 @@
 #include "mb2_internal.h"
 
 namespace mb2 {
-int launch_batch_init(void* amps, uint32_t n, uint64_t bindings, double re, double im, void* stream,
-                      int precision);
 int launch_batch_expect(const void* amps, uint32_t n, uint64_t bindings, const uint64_t* dev_x,
                         const uint64_t* dev_z, const double* dev_coefs, uint32_t num_terms, double* dev_out,
                         void* stream, int precision);

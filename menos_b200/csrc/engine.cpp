@@ -189,6 +189,66 @@ C64Choice c64_choice(const mb2_sweep_options& o, uint32_t n, uint32_t default_ti
     return {m, want_tc && m >= 11 && m <= 13};
 }
 
+// Pauli terms of an n-qubit state on the device: grouped so that each group
+// reads the state once (one launch per group); the fixed-order finish then
+// adds every term's partials.
+struct ExpectPlan {
+    uint32_t n, num_terms;
+    const uint64_t *xs, *zs;  // the caller's
+    mb2::PauliPlan plan;
+    size_t off_z, off_p, off_out, off_s, off_t;
+    std::vector<unsigned char> host;  // spans and terms, until the stream has copied them
+
+    ExpectPlan(uint32_t n_, const uint64_t* x, const uint64_t* z, uint32_t terms)
+        : n(n_), num_terms(terms), xs(x), zs(z), plan(mb2::plan_pauli_groups(x, z, terms, n_)) {
+        auto up = [](size_t v) { return (v + 255) & ~size_t{255}; };
+        const size_t span_bytes = plan.spans.size() * 8, term_bytes = plan.terms.size() * sizeof(mb2::PauliGroupTerm);
+        off_z = up(size_t{terms} * 8);
+        off_p = 2 * off_z;
+        off_out = off_p + size_t{terms} * mb2::kExpBlocks * 16;
+        off_s = up(off_out + size_t{terms} * 16);
+        off_t = off_s + up(span_bytes);
+        host.resize(off_t + term_bytes - off_s);
+        std::memcpy(host.data(), plan.spans.data(), span_bytes);
+        std::memcpy(host.data() + (off_t - off_s), plan.terms.data(), term_bytes);
+    }
+    size_t bytes() const { return off_s + host.size(); }
+    int upload(mb2_context* ctx, unsigned char* base, cudaStream_t s) const {
+        MB2_CUDA(ctx, cudaMemcpyAsync(base, xs, size_t{num_terms} * 8, cudaMemcpyHostToDevice, s));
+        MB2_CUDA(ctx, cudaMemcpyAsync(base + off_z, zs, size_t{num_terms} * 8, cudaMemcpyHostToDevice, s));
+        MB2_CUDA(ctx, cudaMemcpyAsync(base + off_s, host.data(), host.size(), cudaMemcpyHostToDevice, s));
+        return MB2_OK;
+    }
+    // dev_out: num_terms complex values.
+    int launch(mb2_context* ctx, const void* amps, int precision, unsigned char* base, double* dev_out,
+               cudaStream_t s) const {
+        const auto *dx = reinterpret_cast<const uint64_t*>(base), *dz = reinterpret_cast<const uint64_t*>(base + off_z);
+        auto* partials = reinterpret_cast<double*>(base + off_p);
+        int rc = MB2_OK;
+        for (const mb2::PauliGroupPlan& g : plan.groups) {
+            if (g.nterms == 1 || g.c + g.d < mb2::kPauliMinTileQubits) {
+                // Nothing to share (or a state too small for the grouped tiles):
+                // one streaming read per term, its partials in place.
+                for (uint32_t i = 0; i < g.nterms && rc == MB2_OK; ++i) {
+                    const uint32_t t = plan.terms[g.term_off + i].out;
+                    rc = mb2::launch_expectation_partials(
+                        amps, n, dx + t, dz + t, 1, partials + 2 * static_cast<size_t>(t) * mb2::kExpBlocks, s, precision);
+                }
+            } else {
+                rc = mb2::launch_pauli_group(amps, n, g.c, g.d,
+                                             reinterpret_cast<const uint64_t*>(base + off_s) + g.span_off, g.free_mask,
+                                             base + off_t + size_t{g.term_off} * sizeof(mb2::PauliGroupTerm), g.nterms,
+                                             partials, mb2::kExpBlocks, s, precision);
+            }
+            if (rc != MB2_OK) break;
+        }
+        if (rc == MB2_OK)
+            rc = mb2::launch_expectation_finish(partials, mb2::kExpBlocks, dx, dz, num_terms, dev_out, s);
+        if (rc != MB2_OK) return fail(ctx, rc, std::string("expectation launch: ") + mb2::last_cuda_error_string());
+        return MB2_OK;
+    }
+};
+
 }  // namespace
 
 namespace mb2 {
@@ -942,55 +1002,13 @@ int mb2_expectation(mb2_state* s, const uint64_t* x_masks, const uint64_t* z_mas
     const uint64_t lim = (s->n >= 64) ? ~uint64_t{0} : ((uint64_t{1} << s->n) - 1);
     for (uint32_t t = 0; t < num_terms; ++t)
         if ((x_masks[t] | z_masks[t]) & ~lim) return fail(s->ctx, MB2_ERR_INVALID, "Pauli mask beyond the state's qubits");
-    // Terms are grouped so that each group reads the state once (one launch
-    // per group); the fixed-order finish then adds every term's partials.
-    const mb2::PauliPlan plan = mb2::plan_pauli_groups(x_masks, z_masks, num_terms, s->n);
-    const size_t mask_bytes = size_t{num_terms} * 8;
-    const size_t part_bytes = size_t{num_terms} * mb2::kExpBlocks * 16;
-    const size_t out_bytes = size_t{num_terms} * 16;
-    const size_t span_bytes = plan.spans.size() * 8;
-    const size_t term_bytes = plan.terms.size() * sizeof(mb2::PauliGroupTerm);
-    auto up = [](size_t v) { return (v + 255) & ~size_t{255}; };
-    const size_t off_z = up(mask_bytes);
-    const size_t off_p = off_z + up(mask_bytes);
-    const size_t off_o = off_p + part_bytes;
-    const size_t off_s = up(off_o + out_bytes);
-    const size_t off_t = off_s + up(span_bytes);
-    if (int e = ensure_scratch(s, off_t + term_bytes); e != MB2_OK) return e;
+    const ExpectPlan plan(s->n, x_masks, z_masks, num_terms);
+    if (int e = ensure_scratch(s, plan.bytes()); e != MB2_OK) return e;
     auto* base = static_cast<unsigned char*>(s->scratch);
-    std::vector<unsigned char> host(off_t + term_bytes - off_s);
-    std::memcpy(host.data(), plan.spans.data(), span_bytes);
-    std::memcpy(host.data() + (off_t - off_s), plan.terms.data(), term_bytes);
-    MB2_CUDA(s->ctx, cudaMemcpyAsync(base, x_masks, mask_bytes, cudaMemcpyHostToDevice, s->stream));
-    MB2_CUDA(s->ctx, cudaMemcpyAsync(base + off_z, z_masks, mask_bytes, cudaMemcpyHostToDevice, s->stream));
-    MB2_CUDA(s->ctx, cudaMemcpyAsync(base + off_s, host.data(), host.size(), cudaMemcpyHostToDevice, s->stream));
-    auto* partials = reinterpret_cast<double*>(base + off_p);
-    for (const mb2::PauliGroupPlan& g : plan.groups) {
-        if (g.nterms == 1 || g.c + g.d < mb2::kPauliMinTileQubits) {
-            // Nothing to share (or a state too small for the grouped tiles):
-            // one streaming read per term, its partials in place.
-            for (uint32_t i = 0; i < g.nterms; ++i) {
-                const uint32_t t = plan.terms[g.term_off + i].out;
-                const int rc = mb2::launch_expectation_partials(
-                    s->amps, s->n, reinterpret_cast<const uint64_t*>(base) + t,
-                    reinterpret_cast<const uint64_t*>(base + off_z) + t, 1,
-                    partials + 2 * static_cast<size_t>(t) * mb2::kExpBlocks, s->stream, s->precision);
-                if (rc != MB2_OK)
-                    return fail(s->ctx, rc, std::string("expectation launch: ") + mb2::last_cuda_error_string());
-            }
-            continue;
-        }
-        const int rc = mb2::launch_pauli_group(
-            s->amps, s->n, g.c, g.d, reinterpret_cast<const uint64_t*>(base + off_s) + g.span_off, g.free_mask,
-            base + off_t + size_t{g.term_off} * sizeof(mb2::PauliGroupTerm), g.nterms, partials, mb2::kExpBlocks,
-            s->stream, s->precision);
-        if (rc != MB2_OK) return fail(s->ctx, rc, std::string("expectation launch: ") + mb2::last_cuda_error_string());
-    }
-    const int rc = mb2::launch_expectation_finish(partials, mb2::kExpBlocks, reinterpret_cast<const uint64_t*>(base),
-                                                  reinterpret_cast<const uint64_t*>(base + off_z), num_terms,
-                                                  reinterpret_cast<double*>(base + off_o), s->stream);
-    if (rc != MB2_OK) return fail(s->ctx, rc, std::string("expectation launch: ") + mb2::last_cuda_error_string());
-    MB2_CUDA(s->ctx, cudaMemcpyAsync(out, base + off_o, out_bytes, cudaMemcpyDeviceToHost, s->stream));
+    if (int e = plan.upload(s->ctx, base, s->stream); e != MB2_OK) return e;
+    auto* dev_out = reinterpret_cast<double*>(base + plan.off_out);
+    if (int e = plan.launch(s->ctx, s->amps, s->precision, base, dev_out, s->stream); e != MB2_OK) return e;
+    MB2_CUDA(s->ctx, cudaMemcpyAsync(out, dev_out, size_t{num_terms} * 16, cudaMemcpyDeviceToHost, s->stream));
     MB2_CUDA(s->ctx, cudaStreamSynchronize(s->stream));
     return MB2_OK;
 }
@@ -1494,10 +1512,14 @@ int histogram_words(mb2_context* ctx, std::vector<uint64_t> words, uint64_t* out
 
 struct TrajChannel {
     std::vector<uint32_t> qubits;
-    std::vector<std::vector<mb2::Cd>> kraus;     // each dim x dim, row-major
-    std::vector<std::vector<mb2::Cd>> products;  // K^dagger K, as the reference forms them
-    std::vector<uint64_t> xs, zs;                // the 4^k Pauli strings on the channel's qubits
+    uint32_t branches = 0;
+    size_t products = 0, kraus = 0;  // byte offsets in the uploaded data: K^dagger K as the reference forms them, K
 };
+
+// The most trajectories run at once, and the most memory their states take
+// together (a larger state runs alone).
+constexpr uint64_t kTrajBatch = 64;
+constexpr uint64_t kTrajBatchBytes = uint64_t{256} << 20;
 
 // K^dagger K (kraus_products, trajectory_engine.cpp:50-69).
 std::vector<mb2::Cd> kraus_product(const std::vector<mb2::Cd>& k, size_t dim) {
@@ -1542,12 +1564,30 @@ int mb2_trajectories_monitored(mb2_context* ctx, uint32_t n, const mb2_op* ops, 
         return fail(ctx, MB2_ERR_INVALID, "more shots than trajectories");
     for (uint32_t t = 0; t < num_targets; ++t)
         if (targets[2 * t] >= n || targets[2 * t + 1] >= 64) return fail(ctx, MB2_ERR_INVALID, "measure target out of range");
+    const uint64_t lim = (uint64_t{1} << n) - 1;
+    for (uint32_t t = 0; t < num_terms; ++t)
+        if ((x_masks[t] | z_masks[t]) & ~lim) return fail(ctx, MB2_ERR_INVALID, "Pauli mask beyond the state's qubits");
     // Segments: runs of gates (applied op by op, as the reference's
-    // apply_matrix per operation) and channels.
+    // apply_matrix per operation: a tiled program each, planned once for every
+    // trajectory) and channels.
     std::vector<std::vector<mb2_op>> gate_runs;
     std::vector<TrajChannel> channels;
     std::vector<std::pair<int, size_t>> steps;  // (0: gate run, 1: channel), index
     std::vector<uint64_t> step_end;             // operations done once the step is (measurements included)
+    std::vector<std::vector<mb2::Block>> run_blocks;
+    std::vector<mb2::TileProgram> programs;
+    struct RunOffsets {
+        size_t words, data, gdata;
+    };
+    std::vector<RunOffsets> program_at;
+    std::vector<unsigned char> upload;
+    auto put = [&](const void* p, size_t bytes) {
+        const size_t at = (upload.size() + 255) & ~size_t{255};
+        upload.resize(at + bytes);
+        if (bytes) std::memcpy(upload.data() + at, p, bytes);
+        return at;
+    };
+    const bool tiled = n >= mb2::kMinTileQubits;
     try {
         for (uint32_t i = 0; i < num_ops; ++i) {
             const mb2_op& op = ops[i];
@@ -1568,28 +1608,45 @@ int mb2_trajectories_monitored(mb2_context* ctx, uint32_t n, const mb2_op* ops, 
             const size_t dim = size_t{1} << k;
             TrajChannel ch;
             ch.qubits.assign(op.qubits, op.qubits + k);
-            for (uint32_t q : ch.qubits)
-                if (q >= n) return fail(ctx, MB2_ERR_INVALID, "operand out of range");
+            for (uint32_t j = 0; j < k; ++j) {
+                if (ch.qubits[j] >= n) return fail(ctx, MB2_ERR_INVALID, "operand out of range");
+                for (uint32_t l = 0; l < j; ++l)
+                    if (ch.qubits[l] == ch.qubits[j]) return fail(ctx, MB2_ERR_INVALID, "repeated operand");
+            }
+            ch.branches = op.reserved;
+            std::vector<mb2::Cd> kraus, products;
             for (uint32_t t = 0; t < op.reserved; ++t) {
                 std::vector<mb2::Cd> km(dim * dim);
                 for (size_t e = 0; e < dim * dim; ++e)
                     km[e] = mb2::Cd{op.matrix[2 * (t * dim * dim + e)], op.matrix[2 * (t * dim * dim + e) + 1]};
-                ch.products.push_back(kraus_product(km, dim));
-                ch.kraus.push_back(std::move(km));
+                const std::vector<mb2::Cd> pm = kraus_product(km, dim);
+                kraus.insert(kraus.end(), km.begin(), km.end());
+                products.insert(products.end(), pm.begin(), pm.end());
             }
-            for (uint64_t lx = 0; lx < dim; ++lx)
-                for (uint64_t lz = 0; lz < dim; ++lz) {
-                    uint64_t gx = 0, gz = 0;
-                    for (uint32_t j = 0; j < k; ++j) {
-                        if ((lx >> j) & 1u) gx |= uint64_t{1} << ch.qubits[j];
-                        if ((lz >> j) & 1u) gz |= uint64_t{1} << ch.qubits[j];
-                    }
-                    ch.xs.push_back(gx);
-                    ch.zs.push_back(gz);
-                }
+            ch.products = put(products.data(), products.size() * sizeof(mb2::Cd));
+            ch.kraus = put(kraus.data(), kraus.size() * sizeof(mb2::Cd));
             steps.emplace_back(1, channels.size());
             step_end.push_back(i + 1);
             channels.push_back(std::move(ch));
+        }
+        for (const std::vector<mb2_op>& run : gate_runs) {
+            for (const mb2_op& op : run) {
+                if (op.num_qubits == 0 || op.num_qubits > MB2_MAX_OP_QUBITS)
+                    return fail(ctx, MB2_ERR_INVALID, "operand count");
+                for (uint32_t j = 0; j < op.num_qubits; ++j) {
+                    if (op.qubits[j] >= n) return fail(ctx, MB2_ERR_INVALID, "operand out of range");
+                    for (uint32_t l = 0; l < j; ++l)
+                        if (op.qubits[l] == op.qubits[j]) return fail(ctx, MB2_ERR_INVALID, "repeated operand");
+                }
+            }
+            run_blocks.push_back(mb2::build_blocks(run.data(), static_cast<uint32_t>(run.size()), false));
+            if (!tiled) continue;
+            const std::vector<mb2::Block>& blocks = run_blocks.back();
+            const uint32_t m = tile_width(n <= 16 ? mb2::kMaxTileQubits : ctx->tile_c128.load(), n, blocks);
+            programs.push_back(mb2::plan_tile_program(blocks, n, m));
+            const mb2::TileProgram& p = programs.back();
+            program_at.push_back({put(p.words.data(), p.words.size() * 4), put(p.data.data(), p.data.size() * 8),
+                                  put(p.gdata.data(), p.gdata.size() * 8)});
         }
     } catch (const std::exception& e) {
         return fail(ctx, MB2_ERR_INVALID, e.what());
@@ -1597,15 +1654,54 @@ int mb2_trajectories_monitored(mb2_context* ctx, uint32_t n, const mb2_op* ops, 
     const std::vector<Readout> readouts =
         want_counts ? readout_targets(ops, num_ops, targets, num_targets) : std::vector<Readout>{};
     if (!readouts_valid(readouts)) return fail(ctx, MB2_ERR_INVALID, "readout error entries must lie in [0, 1]");
-    mb2_state* st = nullptr;
-    if (int e = mb2_state_alloc(ctx, n, MB2_C128, ~uint64_t{0}, &st); e != MB2_OK) return e;
-    struct Free {
-        mb2_state* s;
-        ~Free() { mb2_state_free(s); }
-    } guard{st};
-    const mb2_sweep_options one_by_one{0, 0, 0, 0, 0, 0};
+    // Trajectories run in batches, their states back to back, every launch for
+    // the whole batch; a monitored run one at a time.
+    const uint64_t state_amps = uint64_t{1} << n;
+    uint64_t batch = std::clamp<uint64_t>(kTrajBatchBytes / (16 * state_amps), 1, std::min(kTrajBatch, trajectories));
+    if (boundary != nullptr) batch = 1;
+    struct Work {  // the batch's states, as a state whose first 2^n amplitudes are trajectory 0's
+        mb2_state* s = nullptr;
+        void* extra = nullptr;
+        ~Work() {
+            if (s == nullptr) return;
+            if (extra != nullptr) cudaFreeAsync(extra, s->stream);
+            mb2_state_free(s);
+        }
+    } work;
+    if (int e = mb2_state_alloc(ctx, n, MB2_C128, ~uint64_t{0}, &work.s); e != MB2_OK) return e;
+    mb2_state* const st = work.s;
+    const cudaStream_t stream = st->stream;
+    if (batch > 1) {
+        MB2_CUDA(ctx, cudaFreeAsync(st->amps, stream));
+        if (cudaMallocAsync(&st->amps, batch * 16 * state_amps, stream) != cudaSuccess) {
+            cudaGetLastError();
+            batch = 1;
+            st->amps = nullptr;
+            MB2_CUDA(ctx, cudaMallocAsync(&st->amps, 16 * state_amps, stream));
+        }
+    }
+    const uint32_t B = static_cast<uint32_t>(batch), C = static_cast<uint32_t>(channels.size());
+    auto up = [](size_t v) { return (v + 255) & ~size_t{255}; };
+    const ExpectPlan terms(n, x_masks, z_masks, num_terms);
+    const size_t off_u = up(upload.size()), off_shot = off_u + up(size_t{B} * C * 8), off_err = off_shot + up(B * 8),
+                 off_basis = off_err + up(B * 4), off_vals = off_basis + up(B * 8),
+                 off_chan = off_vals + up(size_t{B} * num_terms * 16),
+                 off_norms = off_chan + up(mb2::traj_scratch_bytes(n, B)),
+                 off_terms = off_norms + up(mb2::norms_scratch_bytes(n, B)),
+                 bytes = off_terms + (want_exp ? terms.bytes() : 0);
+    MB2_CUDA(ctx, cudaMallocAsync(&work.extra, bytes, stream));
+    auto* const dev = static_cast<unsigned char*>(work.extra);
+    if (!upload.empty()) MB2_CUDA(ctx, cudaMemcpyAsync(dev, upload.data(), upload.size(), cudaMemcpyHostToDevice, stream));
+    if (want_exp)
+        if (int e = terms.upload(ctx, dev + off_terms, stream); e != MB2_OK) return e;
+    auto* const dev_err = reinterpret_cast<int*>(dev + off_err);
+    auto* const dev_vals = reinterpret_cast<double*>(dev + off_vals);
     std::vector<mb2::Cd> term_sums(num_terms, mb2::Cd{0.0, 0.0});
-    std::vector<double> vals(2 * std::max<uint32_t>(num_terms, 1));
+    std::vector<double> vals(size_t{2} * B * std::max<uint32_t>(num_terms, 1)), draws(size_t{B} * std::max<uint32_t>(C, 1)),
+        shot_draws(B);
+    std::vector<uint64_t> basis(B);
+    std::vector<int> errs(B);
+    std::vector<std::mt19937_64> rngs(B);
     uint64_t count = 0;  // Welford (trajectory_engine.cpp:244-265)
     mb2::Cd mean{0.0, 0.0};
     double ssd = 0.0;
@@ -1618,94 +1714,133 @@ int mb2_trajectories_monitored(mb2_context* ctx, uint32_t n, const mb2_op* ops, 
     auto cross = [&](uint64_t crossed) {
         return boundary == nullptr || boundary(user, crossed) == 0;
     };
-    for (uint64_t t = 0; t < trajectories; ++t) {
-        std::mt19937_64 rng(trajectory_seed(seed, t));
-        if (int e = mb2_init(st, 0.0); e != MB2_OK) return e;  // |0..0>, no global phase
+    auto launched = [&](int rc) {
+        return rc == MB2_OK ? MB2_OK
+                            : fail(ctx, rc, std::string("trajectory launch: ") + mb2::last_cuda_error_string());
+    };
+    // The first trajectory that went wrong, as the reference meets it.
+    auto check = [&](uint32_t nt) -> int {
+        MB2_CUDA(ctx, cudaMemcpyAsync(errs.data(), dev_err, nt * sizeof(int), cudaMemcpyDeviceToHost, stream));
+        MB2_CUDA(ctx, cudaStreamSynchronize(stream));
+        for (uint32_t t = 0; t < nt; ++t) {
+            if (errs[t] == mb2::kTrajNoBranch) return fail(ctx, MB2_ERR_INVALID, "every Kraus branch has probability 0");
+            if (errs[t] != 0) return fail(ctx, MB2_ERR_INVALID, "a chosen Kraus branch annihilated the state");
+        }
+        return MB2_OK;
+    };
+    for (uint64_t t0 = 0; t0 < trajectories; t0 += B) {
+        const uint32_t nt = static_cast<uint32_t>(std::min<uint64_t>(B, trajectories - t0));
+        // A trajectory draws one uniform per channel, then its shot's word and
+        // the readout errors'.
+        for (uint32_t t = 0; t < nt; ++t) {
+            rngs[t].seed(trajectory_seed(seed, t0 + t));
+            for (uint32_t c = 0; c < C; ++c) draws[size_t{t} * C + c] = word_to_uniform(rngs[t]());
+            if (want_counts && t0 + t < shots) shot_draws[t] = word_to_uniform(rngs[t]());
+        }
+        if (C != 0)
+            MB2_CUDA(ctx, cudaMemcpyAsync(dev + off_u, draws.data(), size_t{nt} * C * 8, cudaMemcpyHostToDevice, stream));
+        MB2_CUDA(ctx, cudaMemsetAsync(dev_err, 0, B * sizeof(int), stream));
+        // |0..0>, no global phase.
+        if (int e = launched(mb2::launch_batch_init(st->amps, n, nt, 1.0, 0.0, stream, MB2_C128)); e != MB2_OK) return e;
+        // psi /= ||psi|| with the reference's sequential norm (renormalize,
+        // :155-166), applied with the next step that reads the state.
+        mb2::TrajNorm pending;
+        auto settle = [&]() -> int {
+            if (pending.norms == nullptr) return MB2_OK;
+            const int rc = mb2::launch_traj_scale(st->amps, n, nt, pending, dev_err, stream);
+            pending = mb2::TrajNorm{};
+            return launched(rc);
+        };
         for (size_t si = 0; si < steps.size(); ++si) {
-            if (si > 0 && !cross(t * per_trajectory + step_end[si - 1]))
+            if (si > 0 && !cross(t0 * per_trajectory + step_end[si - 1]))
                 return fail(ctx, MB2_ERR_ABANDONED, "abandoned at a safe boundary");
             const auto& [kind, idx] = steps[si];
-            if (kind == 0) {
-                const std::vector<mb2_op>& run = gate_runs[idx];
-                if (int e = mb2_apply_program(st, run.data(), static_cast<uint32_t>(run.size()), &one_by_one); e != MB2_OK)
+            if (kind == 0 && tiled) {
+                if (int e = settle(); e != MB2_OK) return e;
+                const mb2::BatchLayout layout{nt, nullptr, 0};
+                for (const mb2::TilePass& pass : programs[idx].passes)
+                    if (int e = launched(mb2::launch_tile_pass(
+                            st->amps, n, pass, reinterpret_cast<const uint32_t*>(dev + program_at[idx].words),
+                            reinterpret_cast<const double*>(dev + program_at[idx].data),
+                            reinterpret_cast<const double*>(dev + program_at[idx].gdata), ctx->sm_count, stream, &layout));
+                        e != MB2_OK)
+                        return e;
+            } else if (kind == 0) {
+                // Too small for a tile: gate by gate, state by state.
+                if (int e = settle(); e != MB2_OK) return e;
+                void* const first = st->amps;
+                int rc = MB2_OK;
+                for (uint32_t t = 0; t < nt && rc == MB2_OK; ++t) {
+                    st->amps = static_cast<mb2::Cd*>(first) + t * state_amps;
+                    for (const mb2::Block& b : run_blocks[idx])
+                        if ((rc = apply_block(st, b.m.data(), b.q, b.k, false)) != MB2_OK) break;
+                }
+                st->amps = first;
+                if (rc != MB2_OK) return rc;
+            } else {
+                const TrajChannel& ch = channels[idx];
+                const mb2::TrajChannelData data{dev + ch.products, dev + ch.kraus, ch.branches,
+                                                reinterpret_cast<const double*>(dev + off_u) + idx, C};
+                if (int e = launched(mb2::launch_traj_channel(st->amps, n, nt, ch.qubits.data(),
+                                                              static_cast<uint32_t>(ch.qubits.size()), pending, data,
+                                                              dev + off_chan, dev_err, stream));
+                    e != MB2_OK)
                     return e;
-                continue;
-            }
-            const TrajChannel& ch = channels[idx];
-            const uint32_t k = static_cast<uint32_t>(ch.qubits.size());
-            const size_t dim = size_t{1} << k;
-            // rho_q from its Pauli expectations: rho = 2^-k sum_P <P> P,
-            // P = i^{|x&z|} X^x Z^z in the channel's local basis.
-            std::vector<double> pv(2 * ch.xs.size());
-            if (int e = mb2_expectation(st, ch.xs.data(), ch.zs.data(), static_cast<uint32_t>(ch.xs.size()), pv.data());
-                e != MB2_OK)
-                return e;
-            std::vector<mb2::Cd> rho(dim * dim, mb2::Cd{0.0, 0.0});
-            const mb2::Cd ipow[4] = {{1.0, 0.0}, {0.0, 1.0}, {-1.0, 0.0}, {0.0, -1.0}};
-            size_t pi = 0;
-            for (uint64_t lx = 0; lx < dim; ++lx)
-                for (uint64_t lz = 0; lz < dim; ++lz, ++pi) {
-                    const mb2::Cd v{pv[2 * pi], pv[2 * pi + 1]};
-                    const mb2::Cd ph = ipow[std::popcount(lx & lz) & 3];
-                    for (uint64_t c = 0; c < dim; ++c) {
-                        const double sgn = (std::popcount(c & lz) & 1) ? -1.0 : 1.0;
-                        rho[(c ^ lx) * dim + c] += v * ph * sgn;
-                    }
-                }
-            for (mb2::Cd& r : rho) r /= static_cast<double>(dim);
-            // The branch: the first with cumulative p_i = Re Tr(M_i rho) above
-            // u, else the last with p_i > 0 (choose_branch, :123-152).
-            const double u = word_to_uniform(rng());
-            double cumulative = 0.0;
-            int64_t branch = -1, last_positive = -1;
-            for (size_t b = 0; b < ch.products.size() && branch < 0; ++b) {
-                double p = 0.0;
-                for (size_t a = 0; a < dim; ++a)
-                    for (size_t c = 0; c < dim; ++c) p += (ch.products[b][a * dim + c] * rho[c * dim + a]).real();
-                if (p > 0.0) {
-                    last_positive = static_cast<int64_t>(b);
-                    cumulative += p;
-                    if (u < cumulative) branch = static_cast<int64_t>(b);
+                if (int e = launched(mb2::launch_norms(st->amps, n, nt, dev + off_norms, &pending.norms, &pending.pitch,
+                                                       stream));
+                    e != MB2_OK)
+                    return e;
+                if (boundary != nullptr) {
+                    if (int e = settle(); e != MB2_OK) return e;
+                    if (int e = check(nt); e != MB2_OK) return e;
                 }
             }
-            if (branch < 0) branch = last_positive;
-            if (branch < 0) return fail(ctx, MB2_ERR_INVALID, "every Kraus branch has probability 0");
-            const std::vector<mb2::Cd>& km = ch.kraus[static_cast<size_t>(branch)];
-            if (int e = mb2_apply_matrix(st, reinterpret_cast<const double*>(km.data()), ch.qubits.data(), k); e != MB2_OK)
-                return e;
-            // psi /= ||psi|| with the reference's sequential norm (renormalize, :155-166).
-            double norm_sq = 0.0;
-            if (int e = mb2_norm_exact(st, &norm_sq); e != MB2_OK) return e;
-            if (!(norm_sq > 0.0)) return fail(ctx, MB2_ERR_INVALID, "a chosen Kraus branch annihilated the state");
-            const double scale = 1.0 / std::sqrt(norm_sq);
-            const double sm[8] = {scale, 0.0, 0.0, 0.0, 0.0, 0.0, scale, 0.0};
-            const uint32_t q0 = 0;
-            if (int e = mb2_apply_matrix(st, sm, &q0, 1); e != MB2_OK) return e;
         }
-        if (want_exp) {
-            if (int e = mb2_expectation(st, x_masks, z_masks, num_terms, vals.data()); e != MB2_OK) return e;
-            mb2::Cd x{0.0, 0.0};
-            for (uint32_t i = 0; i < num_terms; ++i) {
-                const mb2::Cd v{vals[2 * i], vals[2 * i + 1]};
-                term_sums[i] += v;
-                x += mb2::Cd{coefs[2 * i], coefs[2 * i + 1]} * v;
+        if (int e = settle(); e != MB2_OK) return e;
+        const uint32_t ns = want_counts && t0 < shots ? static_cast<uint32_t>(std::min<uint64_t>(nt, shots - t0)) : 0;
+        if (want_exp)
+            for (uint32_t t = 0; t < nt; ++t)
+                if (int e = terms.launch(ctx, static_cast<mb2::Cd*>(st->amps) + t * state_amps, MB2_C128, dev + off_terms,
+                                         dev_vals + size_t{2} * t * num_terms, stream);
+                    e != MB2_OK)
+                    return e;
+        if (ns != 0) {
+            MB2_CUDA(ctx, cudaMemcpyAsync(dev + off_shot, shot_draws.data(), ns * 8, cudaMemcpyHostToDevice, stream));
+            for (uint32_t t = 0; t < ns; ++t)
+                if (int e = launched(mb2::launch_sample(static_cast<mb2::Cd*>(st->amps) + t * state_amps, n,
+                                                        reinterpret_cast<double*>(dev + off_shot) + t, 1, nullptr, nullptr,
+                                                        dev + off_norms, reinterpret_cast<uint64_t*>(dev + off_basis) + t,
+                                                        stream));
+                    e != MB2_OK)
+                    return e;
+            MB2_CUDA(ctx, cudaMemcpyAsync(basis.data(), dev + off_basis, ns * 8, cudaMemcpyDeviceToHost, stream));
+        }
+        if (want_exp)
+            MB2_CUDA(ctx, cudaMemcpyAsync(vals.data(), dev_vals, size_t{nt} * num_terms * 16, cudaMemcpyDeviceToHost, stream));
+        if (int e = check(nt); e != MB2_OK) return e;  // synchronises
+        for (uint32_t t = 0; t < nt; ++t) {
+            if (want_exp) {
+                mb2::Cd x{0.0, 0.0};
+                for (uint32_t i = 0; i < num_terms; ++i) {
+                    const double* const p = vals.data() + size_t{2} * (size_t{t} * num_terms + i);
+                    const mb2::Cd v{p[0], p[1]};
+                    term_sums[i] += v;
+                    x += mb2::Cd{coefs[2 * i], coefs[2 * i + 1]} * v;
+                }
+                ++count;
+                const mb2::Cd delta = x - mean;
+                mean += delta / static_cast<double>(count);
+                ssd += (std::conj(delta) * (x - mean)).real();
             }
-            ++count;
-            const mb2::Cd delta = x - mean;
-            mean += delta / static_cast<double>(count);
-            ssd += (std::conj(delta) * (x - mean)).real();
+            if (t < ns) {
+                // One word for the shot, then one per readout-errored target
+                // (trajectory_engine.cpp:465-471).
+                uint64_t o = outcome_word(basis[t], targets, num_targets);
+                apply_readout(o, readouts, rngs[t]);
+                shot_words.push_back(o);
+            }
         }
-        if (want_counts && t < shots) {
-            // One word for the shot, then one per readout-errored target
-            // (trajectory_engine.cpp:465-471).
-            const double u = word_to_uniform(rng());
-            uint64_t b = 0;
-            if (int e = mb2_sample_basis(st, &u, 1, &b); e != MB2_OK) return e;
-            uint64_t o = outcome_word(b, targets, num_targets);
-            apply_readout(o, readouts, rng);
-            shot_words.push_back(o);
-        }
-        if ((!steps.empty() && !cross(t * per_trajectory + num_ops)) || !cross((t + 1) * per_trajectory))
+        if ((!steps.empty() && !cross(t0 * per_trajectory + num_ops)) || !cross((t0 + 1) * per_trajectory))
             return fail(ctx, MB2_ERR_ABANDONED, "abandoned at a safe boundary");
     }
     if (want_exp) {

@@ -290,6 +290,8 @@ struct BatchLayout {
     const double* pdata = nullptr;
     uint32_t pstride = 0;
 };
+// Every binding's state to (re, im)|0..0> (kernels_batch.cu).
+int launch_batch_init(void* amps, uint32_t n, uint64_t bindings, double re, double im, void* stream, int precision);
 int launch_tile_pass(void* amps, uint32_t n, const TilePass& pass, const uint32_t* dev_words,
                      const double* dev_sdata, const double* dev_gdata, int sm_count, void* stream,
                      const BatchLayout* batch = nullptr);
@@ -388,6 +390,29 @@ int launch_exact_norm(const void* amps, uint32_t n, void* scratch, double* host_
 size_t norms_scratch_bytes(uint32_t n, uint32_t batch);
 int launch_norms(const void* amps, uint32_t n, uint32_t batch, void* scratch, const double** norms, uint64_t* pitch,
                  void* stream, int precision = MB2_C128);
+// A trajectory batch's channels (kernels_traj.cu): trajectory t's state at
+// amps + t * 2^n amplitudes.
+struct TrajQubits {
+    uint32_t q[3], sorted[3];  // the channel's operands, and ascending
+};
+struct TrajNorm {
+    const double* norms = nullptr;  // launch_norms' of states still to be scaled (null: none are)
+    uint64_t pitch = 0;
+};
+struct TrajChannelData {
+    const void* products;  // K^dagger K per branch, then the branches themselves, row-major complex
+    const void* kraus;
+    uint32_t branches;
+    const double* uniforms;  // trajectory t's at [t * pitch]
+    uint32_t pitch;
+};
+// err[t]: the first thing that went wrong in trajectory t, else 0.
+constexpr int kTrajNoBranch = 1, kTrajAnnihilated = 2;
+size_t traj_scratch_bytes(uint32_t n, uint32_t batch);
+// Scales the states where `norm` says so, then selects and applies a branch each.
+int launch_traj_channel(void* amps, uint32_t n, uint32_t batch, const uint32_t* qubits, uint32_t k,
+                        const TrajNorm& norm, const TrajChannelData& c, void* scratch, int* dev_err, void* stream);
+int launch_traj_scale(void* amps, uint32_t n, uint32_t batch, const TrajNorm& norm, int* dev_err, void* stream);
 // draw == nullptr: dev_u holds the sorted uniforms.  Otherwise they are drawn
 // from the seed *draw into dev_u on the way (sort_scratch:
 // uniforms_scratch_bytes), the generator beside the chunk sums.
