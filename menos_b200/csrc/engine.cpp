@@ -255,11 +255,12 @@ namespace mb2 {
 uint64_t scratch_bound(uint32_t n, const mb2_op* ops, uint32_t num_ops, uint64_t shots, uint32_t terms) {
     auto up = [](uint64_t v) { return (v + 255) & ~uint64_t{255}; };
     // The sweep's upload (mb2_apply_program_monitored): per block at most a
-    // phase record, a few gate words and pass padding (144 bytes) and its
-    // matrix (16 * 4^k, staged or global-only); blocks never outnumber ops.
+    // phase record and a store record of a mapped tile, a few gate words and
+    // pass padding (432 bytes) and its matrix (16 * 4^k, staged or
+    // global-only); blocks never outnumber ops.
     uint64_t program = 4 * 256;
     for (uint32_t i = 0; i < num_ops; ++i)
-        if (ops[i].opcode != MB2_MEASURE) program += 144 + (16ull << (2 * ops[i].num_qubits));
+        if (ops[i].opcode != MB2_MEASURE) program += 432 + (16ull << (2 * ops[i].num_qubits));
     // The sampler (device_counts): uniforms, per-shot basis, the walk's
     // scratch, and the sort's or the counts'.
     const uint64_t sample =
@@ -552,7 +553,7 @@ int mb2_apply_program_monitored(mb2_state* s, const mb2_op* ops, uint32_t num_op
                                                                          : static_cast<uint32_t>(o.low_qubits));
         // complex64 results are not bitwise the reference's: commuting
         // blocks may be reordered into fewer passes.
-        prog = mb2::plan_tile_program(blocks, s->n, m, low, nullptr, c64);
+        prog = mb2::plan_tile_program(blocks, s->n, m, low, nullptr, c64, !tc);
         if (tc) mb2::make_tensor_core_program(prog, blocks, mb2::tc_max_phases(m));
     } catch (const std::exception& e) {
         return fail(s->ctx, MB2_ERR_INVALID, e.what());
@@ -1989,7 +1990,7 @@ int mb2_debug_run_plan(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_opti
         m = std::min(std::max(m, mb2::kMinTileQubits), num_qubits);
         const uint32_t low = o.low_qubits < 0 ? 0u : (o.low_qubits == 0 ? mb2::kDefaultFixedLow
                                                                          : static_cast<uint32_t>(o.low_qubits));
-        mb2::TileProgram prog = mb2::plan_tile_program(blocks, num_qubits, m, low, nullptr, c64);
+        mb2::TileProgram prog = mb2::plan_tile_program(blocks, num_qubits, m, low, nullptr, c64, !tc);
         if (tc) mb2::make_tensor_core_program(prog, blocks, mb2::tc_max_phases(m));
         if (state != nullptr) mb2::run_program_on_host(prog, num_qubits, reinterpret_cast<mb2::Cd*>(state));
         if (stats != nullptr) {

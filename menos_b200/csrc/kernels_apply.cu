@@ -313,6 +313,7 @@ int launch_tile_pass(void* amps, uint32_t n, const TilePass& pass, const uint32_
     L.param_lo = pass.param_lo;
     L.param_len = pass.param_len;
     L.bshift = n - pass.m;
+    L.store_rec = pass.store_rec;
     L.stream = stream;
     L.threads = 1u << (pass.m - kRegQubits);
     // 12-qubit tiles keep three tile buffers (two tiles in flight), smaller

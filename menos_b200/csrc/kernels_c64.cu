@@ -70,26 +70,6 @@ __device__ __forceinline__ void g2(float2 (&a)[kNA], const float* md) {
     }
 }
 
-template <int P0, int P1, int KIND>
-__device__ __forceinline__ void perm2(float2 (&a)[kNA]) {
-    if constexpr (P0 == P1) {
-        return;
-    } else {
-        constexpr int lo = KIND == TK_SW23 ? 2 : 1;
-        constexpr int hi = KIND == TK_SW12 ? 2 : 3;
-#pragma unroll
-        for (int j = 0; j < kNA; ++j) {
-            if (j & ((1 << P0) | (1 << P1))) continue;
-            const int il = j | ((lo & 1) ? (1 << P0) : 0) | ((lo & 2) ? (1 << P1) : 0);
-            const int ih = j | ((hi & 1) ? (1 << P0) : 0) | ((hi & 2) ? (1 << P1) : 0);
-            const float2 t = a[il];
-            a[il] = a[ih];
-            a[ih] = t;
-        }
-    }
-}
-
-
 // One pass: the complex128 kernel's structure (persistent CTAs, tiles
 // `stages - 1` ahead in flight, masked-add tile bases, the pass's words and
 // data staged in shared memory, a batch's parametric slice per tile) with
@@ -104,7 +84,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
                     const uint32_t* __restrict__ words, uint32_t nwords, const double* __restrict__ sdata,
                     uint32_t nsdata, const double* __restrict__ gdata, uint64_t ntiles,
                     const double* __restrict__ pdata, uint32_t pstride, uint32_t param_lo, uint32_t param_len,
-                    uint32_t bshift, uint32_t stages) {
+                    uint32_t bshift, uint32_t store_rec, uint32_t stages) {
     extern __shared__ float2 smem_f[];
     const uint32_t m = MT > 0 ? static_cast<uint32_t>(MT) : m_rt;
     const uint32_t tid = threadIdx.x;
@@ -182,18 +162,25 @@ __global__ void __launch_bounds__(MAXT, MINB)
         while (pc < nwords) {
             const uint32_t w0 = sw[pc];
             const uint32_t op0 = w0 & 0xffu;
-            if (op0 == cop::kPhase) {
-                // The phase record (cop::kPhase), 8-byte slot offsets.
+            if (op0 == cop::kPhase || op0 == cop::kPhaseMap) {
+                // The phase record (cop::kPhase), 8-byte slot offsets; with a
+                // map of the tile (cop::kPhaseMap) the slot from a table.
+                const bool mapped = op0 == cop::kPhaseMap;
                 const uint32_t* rec = sw + pc;
-                pc += cop::kPhaseWords;
+                pc += mapped ? cop::phase_map_words(MT) : cop::phase_words(MT);
                 const uint16_t* et = reinterpret_cast<const uint16_t*>(rec + 5);
                 uint32_t tb = static_cast<uint32_t>(et[tid & 15u]) | static_cast<uint32_t>(et[16 + ((tid >> 4) & 15u)]);
-                if (MT == 0 || MT > 12) tb |= static_cast<uint32_t>(et[32 + ((tid >> 8) & 15u)]);
+                if (MT > 12) tb |= static_cast<uint32_t>(et[32 + ((tid >> 8) & 15u)]);
                 uint32_t rb[kR];
 #pragma unroll
                 for (int b = 0; b < kR; ++b) rb[b] = 1u << ((w0 >> (16 + 4 * b)) & 15u);
-                const uint32_t z0 = swz8(tb) << 3, z1 = rec[3] & 0xffffu, z2 = rec[3] >> 16, z3 = rec[4] & 0xffffu,
-                               z4 = rec[4] >> 16;
+                uint32_t z0 = swz8(tb) << 3;
+                if (mapped) {
+                    const uint16_t* pt = et + 16 * cop::phase_nibbles(MT);
+                    z0 = static_cast<uint32_t>(pt[tid & 15u]) ^ static_cast<uint32_t>(pt[16 + ((tid >> 4) & 15u)]);
+                    if (MT > 12) z0 ^= static_cast<uint32_t>(pt[32 + ((tid >> 8) & 15u)]);
+                }
+                const uint32_t z1 = rec[3] & 0xffffu, z2 = rec[3] >> 16, z3 = rec[4] & 0xffffu, z4 = rec[4] >> 16;
                 char* const tile_b = reinterpret_cast<char*>(tile);
                 auto at = [&](int j) -> float2& {
                     return *reinterpret_cast<float2*>(tile_b + (z0 ^ ((j & 1) ? z1 : 0u) ^ ((j & 2) ? z2 : 0u) ^
@@ -253,9 +240,6 @@ __global__ void __launch_bounds__(MAXT, MINB)
                             break;
                         MB2_CASE12(cop::kGen2, if constexpr (V >= 1) g2<P0, P1>(a, md))
                         MB2_CASE12(cop::kMono2, if constexpr (V == 2) { ++pc; g2<P0, P1>(a, md); })
-                        MB2_CASE12(cop::kSw12, if constexpr (V == 2) perm2<P0, P1, TK_SW12>(a))
-                        MB2_CASE12(cop::kSw13, if constexpr (V == 2) perm2<P0, P1, TK_SW13>(a))
-                        MB2_CASE12(cop::kSw23, if constexpr (V == 2) perm2<P0, P1, TK_SW23>(a))
                         MB2_CASE4(cop::kDs1R, (diag_regs<P, -1>(a, md, 1, aux, 0u, 0u)))
                         MB2_CASE12(cop::kDs2RR, (diag_regs<P0, P1>(a, md, 2, aux, 0u, 0u)))
 #undef MB2_CASE4
@@ -310,8 +294,18 @@ __global__ void __launch_bounds__(MAXT, MINB)
                         } break;
                     }
                 }
+                if (V == 2 && mapped && (w0 & (cop::kPhaseSettle << 8)) != 0) {
+                    // Back to the amplitudes' own index, once every thread has read.
+                    const uint32_t own = swz8(tb);
+                    __syncthreads();
 #pragma unroll
-                for (int j = 0; j < kNA; ++j) at(j) = a[j];
+                    for (int j = 0; j < kNA; ++j)
+                        tile[own ^ swz8(((j & 1) ? rb[0] : 0u) | ((j & 2) ? rb[1] : 0u) | ((j & 4) ? rb[2] : 0u) |
+                                        ((j & 8) ? rb[3] : 0u))] = a[j];
+                } else {
+#pragma unroll
+                    for (int j = 0; j < kNA; ++j) at(j) = a[j];
+                }
                 __syncthreads();
             } else if (V == 2 && op0 == cop::kSmem) {
                 const uint32_t k = (w0 >> 8) & 0xffu, dim = 1u << k;
@@ -345,8 +339,21 @@ __global__ void __launch_bounds__(MAXT, MINB)
             }
         }
         const IDX b0 = cbase + off_lo;
+        if (store_rec != 0) {  // the pass left the tile mapped
+            const uint32_t* rec = sw + store_rec;
+            const uint16_t* pt = reinterpret_cast<const uint16_t*>(rec + 2);
+            uint32_t z0 = static_cast<uint32_t>(pt[tid & 15u]) ^ static_cast<uint32_t>(pt[16 + ((tid >> 4) & 15u)]);
+            if (MT > 12) z0 ^= static_cast<uint32_t>(pt[32 + ((tid >> 8) & 15u)]);
+            const uint32_t z1 = rec[0] & 0xffffu, z2 = rec[0] >> 16, z3 = rec[1] & 0xffffu, z4 = rec[1] >> 16;
+            const char* const tile_b = reinterpret_cast<const char*>(tile);
 #pragma unroll
-        for (int j = 0; j < kNA; ++j) st[b0 + reg_off(j)] = tile[slot(j)];
+            for (int j = 0; j < kNA; ++j)
+                st[b0 + reg_off(j)] = *reinterpret_cast<const float2*>(
+                    tile_b + (z0 ^ ((j & 1) ? z1 : 0u) ^ ((j & 2) ? z2 : 0u) ^ ((j & 4) ? z3 : 0u) ^ ((j & 8) ? z4 : 0u)));
+        } else {
+#pragma unroll
+            for (int j = 0; j < kNA; ++j) st[b0 + reg_off(j)] = tile[slot(j)];
+        }
         cbase = advance(cbase);
         __syncthreads();
     }
@@ -371,7 +378,7 @@ int launch_c64_instance(const TileLaunch& L) {
     if (L.smem > dyn_max) return MB2_ERR_INVALID;
     k_tile_pass_c64<MAXT, MINB, MT, IDX, V><<<L.grid, L.threads, L.smem, static_cast<cudaStream_t>(L.stream)>>>(
         static_cast<float2*>(L.amps), L.n_all, L.m, L.smask, L.words, L.nwords, L.sdata, L.nsdata, L.gdata, L.ntiles,
-        L.pdata, L.pstride, L.param_lo, L.param_len, L.bshift, L.stages);
+        L.pdata, L.pstride, L.param_lo, L.param_len, L.bshift, L.store_rec, L.stages);
     return launch_status();
 }
 
@@ -406,6 +413,7 @@ int launch_tile_pass_c64(void* amps, uint32_t n, const TilePass& pass, const uin
     L.param_lo = pass.param_lo;
     L.param_len = pass.param_len;
     L.bshift = n - pass.m;
+    L.store_rec = pass.store_rec;
     L.stream = stream;
     L.threads = 1u << (pass.m - kRegQubits);
     // 13-qubit tiles (64 KiB): one CTA per SM with three buffers; smaller

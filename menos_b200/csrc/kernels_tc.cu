@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(1 << (MT - 4), MINB)
             if ((w0 & 0xffu) != cop::kPhase) break;  // padding after the last phase
             // The phase record (cop::kPhase), 8-byte slot offsets.
             const uint32_t* rec = sw + pc;
-            pc += cop::kPhaseWords;
+            pc += cop::phase_words(MT);
             const uint16_t* et = reinterpret_cast<const uint16_t*>(rec + 5);
             uint32_t tb = static_cast<uint32_t>(et[tid & 15u]) | static_cast<uint32_t>(et[16 + ((tid >> 4) & 15u)]);
             if (MT > 12) tb |= static_cast<uint32_t>(et[32 + ((tid >> 8) & 15u)]);

@@ -85,7 +85,8 @@ enum TileOp : uint8_t {
     TOP_G2 = 4,       // 2-qubit dense gate on register slots (pos[0], pos[1])
     TOP_DIAG = 5,     // diagonal on tile bits pos[0..k-1]
     TOP_SMEM = 6,     // k-qubit dense gate applied from shared memory (own phase)
-    TOP_MMA = 7       // tensor-core pass: the phase's composed 16x16 matrix number `aux` (tile_tc.cpp)
+    TOP_MMA = 7,      // tensor-core pass: the phase's composed 16x16 matrix number `aux` (tile_tc.cpp)
+    TOP_MOVE = 8      // exact permutation (kind) of tile bits pos[0..k-1]: the amplitudes stay, TileMap changes
 };
 enum TileKind : uint8_t {
     TK_GEN = 0,   // every entry general
@@ -116,6 +117,44 @@ static_assert(sizeof(TileInstr) == 32, "TileInstr is 32 bytes");
 constexpr uint32_t kMaxGlobalQubits = 16;
 constexpr uint32_t kGlobalPos0 = 16;
 
+// Where a tile's amplitudes lie while a pass runs: tile index L is kept at
+// place A L ^ c over GF(2), A's columns col[p] for tile bit p.  X, CX and SWAP
+// permute tile indices by such maps themselves, so a pass composes them here
+// and moves nothing: the phases after them read and write through the map.
+struct TileMap {
+    uint32_t col[16], c = 0;
+    // A CX whose control lies outside the tile: what is added to c in the tiles
+    // where outside qubit r (its rank) is 1.
+    uint32_t out[16] = {};
+    TileMap() {
+        for (uint32_t p = 0; p < 16; ++p) col[p] = 1u << p;
+    }
+    bool identity() const {
+        for (uint32_t p = 0; p < 16; ++p)
+            if (col[p] != 1u << p || out[p] != 0) return false;
+        return c == 0;
+    }
+    // The move takes index L to P L, P its own inverse: afterwards L is where P L was.
+    void move(const TileInstr& g) {
+        const uint32_t control = g.kind == TK_SW13 ? g.pos[0] : g.pos[1], target = g.kind == TK_SW13 ? g.pos[1] : g.pos[0];
+        if ((g.kind == TK_SW13 || g.kind == TK_SW23) && control >= kGlobalPos0) {
+            out[control - kGlobalPos0] ^= col[target];
+            return;
+        }
+        switch (g.kind) {
+            case TK_X: c ^= col[g.pos[0]]; break;
+            case TK_SW12: {
+                const uint32_t t = col[g.pos[0]];
+                col[g.pos[0]] = col[g.pos[1]];
+                col[g.pos[1]] = t;
+                break;
+            }
+            case TK_SW13: col[g.pos[0]] ^= col[g.pos[1]]; break;
+            default: col[g.pos[1]] ^= col[g.pos[0]]; break;  // TK_SW23
+        }
+    }
+};
+
 struct TilePass {
     uint32_t m = 0;          // tile qubits
     uint64_t smask = 0;      // global qubits in the tile
@@ -128,11 +167,12 @@ struct TilePass {
     // The complex128 kernel's compact stream (tile_encode.cpp).
     uint32_t word_begin = 0;
     uint32_t word_count = 0;
+    uint32_t store_rec = 0;  // word offset of the pass's store record (cop::kStoreWords), 0: none needed
     // Parametric data this pass reads from a binding's record: doubles
     // [param_lo, param_lo + param_len), staged after the pass's data.
     uint32_t param_lo = 0;
     uint32_t param_len = 0;
-    bool heavy = false;  // has two-qubit dense/monomial/permutation, kDiagK or kSmem words
+    bool heavy = false;  // has two-qubit dense/monomial, kDiagK or kSmem words
     bool mid = false;    // heavy, but only through general dense two-qubit words (kGen2)
     // Tensor-core form (complex64, tile_tc.cpp): the pass's composed phase
     // matrices are tcdata[tc_begin, tc_begin + tc_phases * kTcOperandWords).
@@ -156,9 +196,7 @@ constexpr uint32_t kReal1 = 9;   // + slot
 // 13-20 are unused (one-qubit monomials and X are written as kGen1/kReal1).
 constexpr uint32_t kGen2 = 21;   // + pair
 constexpr uint32_t kMono2 = 33;  // + pair; extra word = source rows (3 bits each)
-constexpr uint32_t kSw12 = 45;   // + pair
-constexpr uint32_t kSw13 = 57;   // + pair
-constexpr uint32_t kSw23 = 69;   // + pair
+// 45-80 are unused (exact permutations are TileMap's, not instructions).
 constexpr uint32_t kDs1R = 81;   // + slot; aux = entry classes
 // An operand position (0-31) in a header word: bits 16-19 and bit 31 (the
 // staged data offset, bits 20-30, stays below 2048 16-byte units).
@@ -182,11 +220,29 @@ constexpr uint32_t kU3Run012 = 112;
 constexpr uint32_t kSignsW = 113;
 // aux = thread bits; bits 16-31 register positions; then the phase record:
 // words 1-2 the byte offsets (16 bits each) of the four register bits' slots
-// with 16-byte slots, words 3-4 the same with 8-byte slots, words 5-28 a
-// table of 48 16-bit entries: entry 16 g + v is the tile bits that thread
-// index bits 4g..4g+3 equal to v stand for in this phase.
+// with 16-byte slots, words 3-4 the same with 8-byte slots, then a table of
+// 16-bit entries, 16 for each nibble of the thread index (two, or three with
+// 13-qubit tiles): entry 16 g + v is the tile bits that thread index bits
+// 4g..4g+3 equal to v stand for in this phase.
 constexpr uint32_t kPhase = 200;
-constexpr uint32_t kPhaseWords = 29;
+MB2_HD inline constexpr uint32_t phase_nibbles(uint32_t m) { return m > 12 ? 3u : 2u; }
+MB2_HD inline constexpr uint32_t phase_words(uint32_t m) { return 5 + 8 * phase_nibbles(m); }
+// A phase whose amplitudes lie elsewhere than at their own tile index
+// (TileMap): words 1-4 are the places' slot offsets instead, and a second
+// table follows with the slot byte offsets of the thread index's nibbles
+// (16- or 8-byte slots, as the program's precision), then for each outside
+// control (their number in aux bits 4-6) its position in bits 0-4 and in bits
+// 16-31 the offset that it adds.  kPhaseSettle in aux: the amplitudes are
+// written back to their own index.
+constexpr uint32_t kPhaseMap = 203;
+MB2_HD inline constexpr uint32_t phase_map_words(uint32_t m) { return phase_words(m) + 8 * phase_nibbles(m); }
+constexpr uint32_t kPhaseSettle = 0x80;  // in aux, beside the thread bits (0-3) and the controls
+constexpr uint32_t kMaxMapControls = 7;
+// The store record of a pass that ends with such a map, after its last
+// instruction: the canonical mapping's slot offsets of the four register bits
+// (two words) and of the thread index's nibbles (as above), the number of
+// outside controls and one word for each, as in kPhaseMap.
+constexpr uint32_t kStoreWords = 2 + 24 + 1 + kMaxMapControls;  // at most
 constexpr uint32_t kSmem = 201;  // aux = k; extra words: tile positions, gdata offset (doubles)
 // Tensor-core pass: apply the pass's composed phase matrix number aux (its
 // split-FP16 operands staged in shared memory) to the registers' amplitudes.
@@ -198,7 +254,7 @@ constexpr uint32_t kMma = 202;
 }  // namespace cop
 
 // Shared-memory budget of one pass's staged instructions + data.
-constexpr size_t kMaxStagedBytes = 32 * 1024;
+constexpr size_t kMaxStagedBytes = 32 * 1024 - cop::kStoreWords * 4;
 
 // TileInstr.data: for TOP_SMEM an offset into the program's global-only data
 // block (gdata); for every other instruction an offset into its pass's
@@ -212,7 +268,8 @@ struct TileProgram {
     uint32_t param_stride = 0;            // doubles per binding record
     std::vector<TileInstr> instrs;
     std::vector<double> data;
-    std::vector<uint32_t> words;  // compact stream of every pass (complex128 kernel)
+    std::vector<uint32_t> words;  // compact stream of every pass
+    bool c64 = false;             // for the complex64 kernels (8-byte slots)
     uint64_t fp64_per_amp = 0;    // modelled FP64 instructions per amplitude
     // Tensor-core passes: per composed phase matrix, its real 32x32 form as
     // FP16 high and low parts in the MMA's shared-memory layout (tile_tc.cpp),
@@ -240,7 +297,9 @@ void make_tensor_core_program(TileProgram& prog, const std::vector<Block>& block
 // positions): tperm[0..nthread) lists the other tile positions, the first
 // three of distinct residues mod 3 when possible (conflict-free shared-memory
 // slots under the tile kernels' XOR-fold swizzle).
-void thread_bit_order(uint32_t m, const uint32_t* reg, uint32_t nreg, uint8_t* tperm, uint8_t& nthread);
+// With a map (of a program with 16- or 8-byte slots), by the places instead.
+void thread_bit_order(uint32_t m, const uint32_t* reg, uint32_t nreg, uint8_t* tperm, uint8_t& nthread,
+                      const TileMap* map = nullptr, bool slots8 = false);
 
 // Applies a planned program's passes to a host state in FP64, instruction by
 // instruction (phase matrices exact, not split): the arithmetic the tile
@@ -265,9 +324,12 @@ constexpr uint8_t kParamM00Real = 4;   // ... entry (0,0) is real in every bindi
 // commuting: blocks on disjoint qubits may be applied in either order
 // (the complex64 path, whose result is not bitwise the reference's), and
 // the passes follow a dependency order chosen for few passes and phases.
+// split: two-qubit blocks that are a permutation and a one-qubit gate run as
+// the two (off for a program that is rewritten for the tensor cores).
 TileProgram plan_tile_program(const std::vector<Block>& blocks, uint32_t n, uint32_t m,
                               uint32_t fixed_low = kDefaultFixedLow,
-                              const std::vector<uint8_t>* parametric = nullptr, bool commuting = false);
+                              const std::vector<uint8_t>* parametric = nullptr, bool commuting = false,
+                              bool split = true);
 
 // ---- device launches (kernels_*.cu) ----------------------------------------
 struct DevCtx;  // forward (engine.cpp)
@@ -313,6 +375,7 @@ struct TileLaunch {
     uint32_t param_lo = 0;
     uint32_t param_len = 0;
     uint32_t bshift = 0;
+    uint32_t store_rec = 0;
     uint32_t stages = 2;
     int grid = 0;       // set by the instance launcher
     int sm_count = 0;
@@ -329,7 +392,7 @@ struct TileJob {
     const uint32_t* words;
     const double* sdata;
     const double* gdata;
-    uint32_t n, nwords, nsdata, cta_begin, nctas, pad;
+    uint32_t n, nwords, nsdata, cta_begin, nctas, store_rec;
 };
 // Launches pass jobs[0..njobs) (host array `jobs`, copied to dev_jobs by the
 // caller beforehand) with tile width m, the full kernel variant; smem: the

@@ -256,6 +256,7 @@ void run_small_batch(mb2_server* s, cudaStream_t stream, std::vector<Request>& b
                 J.ntiles = uint64_t{1} << (batch[i].n - tp.m);
                 J.n = batch[i].n;
                 J.nwords = tp.word_count;
+                J.store_rec = tp.store_rec;
                 J.nsdata = tp.sdata_count;
                 J.cta_begin = L.ctas;
                 J.nctas = static_cast<uint32_t>(J.ntiles);

@@ -34,7 +34,7 @@ uint32_t header(uint32_t op, uint32_t aux, uint32_t tbit, uint32_t off_doubles) 
 }
 
 bool is_param(const TileInstr& g) {
-    return g.op != TOP_PHASE && g.op != TOP_END && g.op != TOP_MMA && g.nthread != 0;
+    return g.op != TOP_PHASE && g.op != TOP_END && g.op != TOP_MMA && g.op != TOP_MOVE && g.nthread != 0;
 }
 
 // Doubles of a parametric instruction's per-binding record.
@@ -46,7 +46,7 @@ uint32_t param_doubles(const TileInstr& g) {
 // Rewrites runs of U3 words on slots 0-1-2-3, 0-1, 1-2-3 or 0-1-2 whose
 // matrices are consecutive (8 doubles apart) into one run word, in the
 // words from `begin` on.
-void fuse_u3_runs(std::vector<uint32_t>& w, size_t begin) {
+void fuse_u3_runs(std::vector<uint32_t>& w, size_t begin, uint32_t m) {
     std::vector<uint32_t> out(w.begin(), w.begin() + static_cast<long>(begin));
     size_t i = begin;
     auto is_u3 = [&](size_t k, uint32_t slot) { return k < w.size() && (w[k] & 0xffu) == cop::kU3 + slot; };
@@ -62,9 +62,10 @@ void fuse_u3_runs(std::vector<uint32_t>& w, size_t begin) {
         const uint32_t op = w[i] & 0xffu;
         // Skip over multi-word instructions unchanged.
         uint32_t len = 1;
-        if (op == cop::kPhase) len = cop::kPhaseWords;
+        if (op == cop::kPhase) len = cop::phase_words(m);
+        else if (op == cop::kPhaseMap) len = cop::phase_map_words(m) + ((w[i] >> 12) & 7u);
         else if (op == cop::kSmem) len = 3;
-        else if ((op >= cop::kMono2 && op < cop::kSw12) || op == cop::kDs2TT || op == cop::kDiagK) len = 2;
+        else if ((op >= cop::kMono2 && op < cop::kMono2 + 12) || op == cop::kDs2TT || op == cop::kDiagK) len = 2;
         else if (op == cop::kSigns) len = 1 + ((w[i] >> 8) & 0xffu);
         else if (op == cop::kSignsW) len = 1 + 2 * ((w[i] >> 8) & 0xffu);
         if (op == cop::kU3 && chain(i, 0, 4)) {
@@ -109,6 +110,31 @@ void encode_compact(TileProgram& prog) {
         };
         auto& w = prog.words;
         bool heavy = false, heavy_other = false;  // other: beyond general dense 2q
+        TileMap map;
+        // Slot byte offset of place v, in this program's slots.
+        auto slot_at = [&](uint32_t v) { return (prog.c64 ? swz8(v) << 3 : swz(v) << 4) & 0xffffu; };
+        // The places' offsets for the nibbles of a thread index whose bit t is tile bit tperm[t].
+        auto push_places = [&](const uint8_t* tperm, uint32_t nthread) {
+            uint32_t at[48] = {};
+            for (uint32_t gi = 0; gi < 3; ++gi)
+                for (uint32_t v = 0; v < 16; ++v) {
+                    uint32_t place = gi == 0 ? map.c : 0u;
+                    for (uint32_t t = 0; t < 4; ++t)
+                        if (4 * gi + t < nthread && ((v >> t) & 1u)) place ^= map.col[tperm[4 * gi + t]];
+                    at[16 * gi + v] = slot_at(place);
+                }
+            for (uint32_t k = 0; k < 8 * cop::phase_nibbles(pass.m); ++k) w.push_back(at[2 * k] | (at[2 * k + 1] << 16));
+        };
+        auto controls = [&]() {
+            uint32_t n = 0;
+            for (uint32_t v : map.out) n += v != 0 ? 1u : 0u;
+            if (n > cop::kMaxMapControls) throw std::logic_error("too many outside controls in a pass");
+            return n;
+        };
+        auto push_controls = [&]() {
+            for (uint32_t r = 0; r < kMaxGlobalQubits; ++r)
+                if (map.out[r] != 0) w.push_back((kGlobalPos0 + r) | (slot_at(map.out[r]) << 16));
+        };
         uint32_t reg[kRegQubits] = {0, 1, 2, 3};
         // A diagonal of at most two operands by entry class.
         auto emit_dsmall = [&](const TileInstr& g, uint32_t off) {
@@ -216,7 +242,9 @@ void encode_compact(TileProgram& prog) {
             }
             flush_signs();
             const uint32_t off =
-                (g.op == TOP_PHASE || g.op == TOP_END || g.op == TOP_SMEM || g.op == TOP_MMA) ? 0u : data_off(g);
+                (g.op == TOP_PHASE || g.op == TOP_END || g.op == TOP_SMEM || g.op == TOP_MMA || g.op == TOP_MOVE)
+                    ? 0u
+                    : data_off(g);
             switch (g.op) {
                 case TOP_PHASE: {
                     uint32_t packed = 0;
@@ -224,13 +252,16 @@ void encode_compact(TileProgram& prog) {
                         reg[s] = g.pos[s];
                         packed |= static_cast<uint32_t>(g.pos[s]) << (4 * s);
                     }
-                    w.push_back(cop::kPhase | (static_cast<uint32_t>(g.nthread) << 8) | (packed << 16));
+                    const bool mapped = !map.identity();
+                    const uint32_t settle = mapped && g.kind != 0 ? cop::kPhaseSettle : 0u;
+                    w.push_back((mapped ? cop::kPhaseMap : cop::kPhase) |
+                                ((static_cast<uint32_t>(g.nthread) | settle | (controls() << 4)) << 8) | (packed << 16));
                     // Slot byte offsets of the register bits (16-byte slots:
                     // tiles of at most 12 qubits; 8-byte slots: at most 13).
                     uint32_t z16[kRegQubits], z8[kRegQubits];
                     for (uint32_t s = 0; s < kRegQubits; ++s) {
-                        z16[s] = (swz(1u << g.pos[s]) << 4) & 0xffffu;
-                        z8[s] = (swz8(1u << g.pos[s]) << 3) & 0xffffu;
+                        z16[s] = (swz(map.col[g.pos[s]]) << 4) & 0xffffu;
+                        z8[s] = (swz8(map.col[g.pos[s]]) << 3) & 0xffffu;
                     }
                     w.push_back(z16[0] | (z16[1] << 16));
                     w.push_back(z16[2] | (z16[3] << 16));
@@ -244,9 +275,20 @@ void encode_compact(TileProgram& prog) {
                                 const uint32_t i = 4 * gi + t;
                                 if (i < g.nthread && ((v >> t) & 1u)) et[16 * gi + v] |= 1u << g.tperm[i];
                             }
-                    for (uint32_t k = 0; k < 24; ++k) w.push_back(et[2 * k] | (et[2 * k + 1] << 16));
+                    for (uint32_t k = 0; k < 8 * cop::phase_nibbles(pass.m); ++k) w.push_back(et[2 * k] | (et[2 * k + 1] << 16));
+                    if (mapped) {
+                        push_places(g.tperm, g.nthread);
+                        push_controls();
+                    }
+                    if (settle != 0) {
+                        heavy = heavy_other = true;
+                        map = TileMap();
+                    }
                     break;
                 }
+                case TOP_MOVE:
+                    map.move(g);
+                    break;
                 case TOP_END:
                     w.push_back(cop::kEnd);
                     break;
@@ -264,18 +306,14 @@ void encode_compact(TileProgram& prog) {
                     break;
                 }
                 case TOP_G1: {
-                    // X and monomial rows as general 2x2 products: the zero
-                    // entry's product only moves a zero's sign, so the result
-                    // is the same, and the kernel's lean variant keeps no
+                    // Monomial rows as general 2x2 products: the zero entry's
+                    // product only moves a zero's sign, so the result is the
+                    // same, and the kernel's lean variant keeps no
                     // register-moving instructions.
                     const uint32_t p = g.pos[0];
                     switch (g.kind) {
                         case TK_U3: w.push_back(header(cop::kU3 + p, 0, 0, off)); break;
                         case TK_REAL: w.push_back(header(cop::kReal1 + p, 0, 0, off)); break;
-                        case TK_X:
-                            w.push_back(header(cop::kReal1 + p, 0, 0, off));
-                            prog.fp64_per_amp += 6;
-                            break;
                         case TK_MONO:
                             w.push_back(header(cop::kGen1 + p, 0, 0, off));
                             prog.fp64_per_amp += 8;
@@ -285,13 +323,10 @@ void encode_compact(TileProgram& prog) {
                     break;
                 }
                 case TOP_G2: {
-                    heavy = true;  // permutations and monomials move registers: full variant
+                    heavy = true;  // monomials move registers: full variant
                     const uint32_t pr = pair_index(g.pos[0], g.pos[1]);
                     if (g.kind != TK_GEN) heavy_other = true;
                     switch (g.kind) {
-                        case TK_SW12: w.push_back(header(cop::kSw12 + pr, 0, 0, 0)); break;
-                        case TK_SW13: w.push_back(header(cop::kSw13 + pr, 0, 0, 0)); break;
-                        case TK_SW23: w.push_back(header(cop::kSw23 + pr, 0, 0, 0)); break;
                         case TK_MONO:
                             w.push_back(header(cop::kMono2 + pr, 0, 0, off));
                             w.push_back(g.aux);
@@ -317,9 +352,24 @@ void encode_compact(TileProgram& prog) {
             }
         }
         flush_signs();
-        fuse_u3_runs(w, pass.word_begin);
+        fuse_u3_runs(w, pass.word_begin, pass.m);
         pass.heavy = heavy;
         pass.mid = heavy && !heavy_other;
+        pass.store_rec = 0;
+        if (!map.identity()) {
+            // The canonical mapping reads the tile through the map: thread bits
+            // are tile bits 0.., the register bits the four above them.
+            w.push_back(cop::kEnd);
+            pass.store_rec = static_cast<uint32_t>(w.size()) - pass.word_begin;
+            const uint32_t tbits = pass.m - kRegQubits;
+            uint8_t own[16];
+            for (uint32_t p = 0; p < 16; ++p) own[p] = static_cast<uint8_t>(p);
+            for (uint32_t r = 0; r < kRegQubits; r += 2)
+                w.push_back(slot_at(map.col[tbits + r]) | (slot_at(map.col[tbits + r + 1]) << 16));
+            push_places(own, tbits);
+            w.push_back(controls());
+            push_controls();
+        }
         while (w.size() & 3u) w.push_back(cop::kEnd);  // 16-byte multiple: the staged data follows
         pass.word_count = static_cast<uint32_t>(w.size()) - pass.word_begin;
     }

@@ -173,28 +173,6 @@ __device__ __forceinline__ void gen2_if(double2 (&a)[kNA], const double* md) {
     if constexpr (FULL) g2<P0, P1, TK_GEN>(a, md, 0u);
 }
 
-// Exact permutations (every nonzero entry (1,0)): register moves only.
-// TK_X: 1q swap; TK_SW12 / TK_SW13 / TK_SW23: 2q, exchange local indices
-// (1,2) (SWAP), (1,3) (CX, control = operand 0), (2,3) (CX, control = operand 1).
-template <int P0, int P1, int KIND>
-__device__ __forceinline__ void perm2(double2 (&a)[kNA]) {
-    if constexpr (P0 == P1) {
-        return;
-    } else {
-        constexpr int lo = KIND == TK_SW23 ? 2 : 1;
-        constexpr int hi = KIND == TK_SW12 ? 2 : 3;
-#pragma unroll
-        for (int j = 0; j < kNA; ++j) {
-            if (j & ((1 << P0) | (1 << P1))) continue;
-            const int il = j | ((lo & 1) ? (1 << P0) : 0) | ((lo & 2) ? (1 << P1) : 0);
-            const int ih = j | ((hi & 1) ? (1 << P0) : 0) | ((hi & 2) ? (1 << P1) : 0);
-            const double2 t = a[il];
-            a[il] = a[ih];
-            a[ih] = t;
-        }
-    }
-}
-
 // cp.async of one 16-byte amplitude, global -> shared (L2 only, no L1).
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
@@ -208,13 +186,12 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // (canonical layout on entry and exit).  `sync` is the barrier of the
 // threads that share the tile; parametric data sits pshift doubles past the
 // staged data's end.  FULL = false compiles out every instruction that moves
-// amplitudes between registers or selects them at run time (permutations,
-// monomial rows) and the rare heavy ones (dense two-qubit blocks, wide
+// amplitudes between registers or selects them at run time (monomial rows) and the rare heavy ones (dense two-qubit blocks, wide
 // diagonals, shared-memory blocks): measured per U3, their presence in the
 // same switch costs ~60-85 extra register moves on every gate path (the
 // allocator's layout at the merge).  The launcher picks the lean variant for
-// passes without them (the encoder writes single-qubit X and monomial gates
-// as general 2x2 products, exact up to zero signs).
+// passes without them (the encoder writes single-qubit monomial gates as
+// general 2x2 products, exact up to zero signs).
 template <int MT, bool FULL, typename SYNC>
 __device__ __forceinline__ void compute_tile(double2* __restrict__ tile, const uint32_t* __restrict__ sw,
                                              uint32_t nwords, const double* __restrict__ sd, uint32_t nsdata,
@@ -228,22 +205,34 @@ __device__ __forceinline__ void compute_tile(double2* __restrict__ tile, const u
     while (pc < nwords) {
         const uint32_t w0 = sw[pc];
         const uint32_t op0 = w0 & 0xffu;
-        if (op0 == cop::kPhase) {
+        if (op0 == cop::kPhase || op0 == cop::kPhaseMap) {
             // The phase record (cop::kPhase): this thread's tile bits from
             // the nibble table, the register bits' slot byte offsets as words.
+            // With a map of the tile (cop::kPhaseMap) the slot comes from a
+            // table of its own: a pass's X, CX and SWAP blocks cost these
+            // lookups in the phases behind them and no move of an amplitude.
+            const bool mapped = op0 == cop::kPhaseMap;
             const uint32_t* rec = sw + pc;
-            pc += cop::kPhaseWords;
+            const uint32_t nctl = mapped ? (w0 >> 12) & 7u : 0u;
+            pc += mapped ? cop::phase_map_words(MT) + nctl : cop::phase_words(MT);
             const uint16_t* et = reinterpret_cast<const uint16_t*>(rec + 5);
             uint32_t tb = static_cast<uint32_t>(et[tid & 15u]) | static_cast<uint32_t>(et[16 + ((tid >> 4) & 15u)]);
-            if (MT == 0 || MT > 12) tb |= static_cast<uint32_t>(et[32 + ((tid >> 8) & 15u)]);
             uint32_t rb[kR];
 #pragma unroll
             for (int b = 0; b < kR; ++b) rb[b] = 1u << ((w0 >> (16 + 4 * b)) & 15u);
             // swz is linear over XOR, so slot j's byte offset is swz(tb)'s
             // XOR the register bits' of j (recomputed for the write-back
             // rather than held in 16 registers through the gates).
-            const uint32_t z0 = swz(tb) << 4, z1 = rec[1] & 0xffffu, z2 = rec[1] >> 16, z3 = rec[2] & 0xffffu,
-                           z4 = rec[2] >> 16;
+            uint32_t z0 = swz(tb) << 4;
+            if (mapped) {
+                const uint16_t* pt = et + 16 * cop::phase_nibbles(MT);
+                z0 = static_cast<uint32_t>(pt[tid & 15u]) ^ static_cast<uint32_t>(pt[16 + ((tid >> 4) & 15u)]);
+                for (uint32_t i = 0; i < nctl; ++i) {
+                    const uint32_t e = rec[cop::phase_map_words(MT) + i];
+                    z0 ^= ((gbits >> (e & 31u)) & 1u) ? e >> 16 : 0u;
+                }
+            }
+            const uint32_t z1 = rec[1] & 0xffffu, z2 = rec[1] >> 16, z3 = rec[2] & 0xffffu, z4 = rec[2] >> 16;
             // Operand bit values from here on: the tile bits, and from
             // position kGlobalPos0 the tile's bits of the qubits outside it.
             tb |= gbits;
@@ -287,9 +276,6 @@ __device__ __forceinline__ void compute_tile(double2* __restrict__ tile, const u
                     MB2_CASE4(cop::kReal1, (g1<P, TK_REAL>(a, md, 0u)))
                     MB2_CASE12(cop::kGen2, (gen2_if<P0, P1, FULL>(a, md)))
                     MB2_CASE12(cop::kMono2, if constexpr (FULL) g2<P0, P1, TK_MONO>(a, md, sw[pc++]))
-                    MB2_CASE12(cop::kSw12, if constexpr (FULL) perm2<P0, P1, TK_SW12>(a))
-                    MB2_CASE12(cop::kSw13, if constexpr (FULL) perm2<P0, P1, TK_SW13>(a))
-                    MB2_CASE12(cop::kSw23, if constexpr (FULL) perm2<P0, P1, TK_SW23>(a))
                     case cop::kU3Run0123:
                         g1<0, TK_U3>(a, md, 0u);
                         g1<1, TK_U3>(a, md + 8, 0u);
@@ -376,8 +362,18 @@ __device__ __forceinline__ void compute_tile(double2* __restrict__ tile, const u
                     } break;
                 }
             }
+            if (FULL && mapped && (w0 & (cop::kPhaseSettle << 8)) != 0) {
+                // Back to the amplitudes' own index, once every thread has read.
+                const uint32_t own = swz(tb & ((1u << kGlobalPos0) - 1u));
+                sync();
 #pragma unroll
-            for (int j = 0; j < kNA; ++j) at(j) = a[j];
+                for (int j = 0; j < kNA; ++j)
+                    tile[own ^ swz(((j & 1) ? rb[0] : 0u) | ((j & 2) ? rb[1] : 0u) | ((j & 4) ? rb[2] : 0u) |
+                                   ((j & 8) ? rb[3] : 0u))] = a[j];
+            } else {
+#pragma unroll
+                for (int j = 0; j < kNA; ++j) at(j) = a[j];
+            }
             sync();
         } else if (FULL && op0 == cop::kSmem) {
             // A dense k-qubit block (k >= 3) on the whole tile in shared memory.
@@ -435,8 +431,8 @@ __device__ __forceinline__ void tile_pass_body(double2* __restrict__ st, uint32_
                                                const double* __restrict__ sdata, uint32_t nsdata,
                                                const double* __restrict__ gdata, uint64_t ntiles,
                                                const double* __restrict__ pdata, uint32_t pstride, uint32_t param_lo,
-                                               uint32_t param_len, uint32_t bshift, uint32_t stages, uint32_t cta,
-                                               uint32_t nctas) {
+                                               uint32_t param_len, uint32_t bshift, uint32_t store_rec,
+                                               uint32_t stages, uint32_t cta, uint32_t nctas) {
     extern __shared__ double2 smem_tiles[];
     const uint32_t m = MT > 0 ? static_cast<uint32_t>(MT) : m_rt;
     const uint32_t tid = threadIdx.x;
@@ -529,10 +525,27 @@ __device__ __forceinline__ void tile_pass_body(double2* __restrict__ st, uint32_
         }
         compute_tile<MT, FULL>(tile, sw, nwords, sd, nsdata, 0u, gdata, tid, m, gbits, [] { __syncthreads(); });
 
-        // Store: canonical mapping, -0.0 normalised.
+        // Store: canonical mapping, -0.0 normalised; where the pass left the
+        // tile mapped, through the store record.
         const IDX b0 = cbase + off_lo;
+        if (store_rec != 0) {
+            const uint32_t* rec = sw + store_rec;
+            const uint16_t* pt = reinterpret_cast<const uint16_t*>(rec + 2);
+            uint32_t z0 = static_cast<uint32_t>(pt[tid & 15u]) ^ static_cast<uint32_t>(pt[16 + ((tid >> 4) & 15u)]);
+            for (uint32_t i = 0; i < rec[18]; ++i) {
+                const uint32_t e = rec[19 + i];
+                z0 ^= ((gbits >> (e & 31u)) & 1u) ? e >> 16 : 0u;
+            }
+            const uint32_t z1 = rec[0] & 0xffffu, z2 = rec[0] >> 16, z3 = rec[1] & 0xffffu, z4 = rec[1] >> 16;
+            const char* const tile_b = reinterpret_cast<const char*>(tile);
 #pragma unroll
-        for (int j = 0; j < kNA; ++j) st[b0 + reg_off(j)] = canon(tile[slot(j)]);
+            for (int j = 0; j < kNA; ++j)
+                st[b0 + reg_off(j)] = canon(*reinterpret_cast<const double2*>(
+                    tile_b + (z0 ^ ((j & 1) ? z1 : 0u) ^ ((j & 2) ? z2 : 0u) ^ ((j & 4) ? z3 : 0u) ^ ((j & 8) ? z4 : 0u))));
+        } else {
+#pragma unroll
+            for (int j = 0; j < kNA; ++j) st[b0 + reg_off(j)] = canon(tile[slot(j)]);
+        }
         cbase = advance(cbase);
         __syncthreads();  // the buffer is the target of a later prefetch
     }
@@ -543,9 +556,10 @@ __global__ void __launch_bounds__(MAXT, MINB)
     k_tile_pass(double2* __restrict__ st, uint32_t n, uint32_t m_rt, uint64_t smask, uint64_t gmask,
                 const uint32_t* __restrict__ words, uint32_t nwords, const double* __restrict__ sdata,
                 uint32_t nsdata, const double* __restrict__ gdata, uint64_t ntiles, const double* __restrict__ pdata,
-                uint32_t pstride, uint32_t param_lo, uint32_t param_len, uint32_t bshift, uint32_t stages) {
+                uint32_t pstride, uint32_t param_lo, uint32_t param_len, uint32_t bshift, uint32_t store_rec,
+                uint32_t stages) {
     tile_pass_body<MT, IDX, FULL>(st, n, m_rt, smask, gmask, words, nwords, sdata, nsdata, gdata, ntiles, pdata,
-                                  pstride, param_lo, param_len, bshift, stages, blockIdx.x, gridDim.x);
+                                  pstride, param_lo, param_len, bshift, store_rec, stages, blockIdx.x, gridDim.x);
 }
 
 // Many states' passes in one launch (small states, one tile width): CTAs
@@ -561,7 +575,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_tile_pass_jobs(const TileJob* __res
     }
     const TileJob& J = jobs[lo];
     tile_pass_body<MT, uint64_t, FULL>(static_cast<double2*>(J.st), J.n, m_rt, J.smask, J.gmask, J.words, J.nwords, J.sdata, J.nsdata,
-                                       J.gdata, J.ntiles, nullptr, 0, 0, 0, 0, 2, blockIdx.x - J.cta_begin,
+                                       J.gdata, J.ntiles, nullptr, 0, 0, 0, 0, J.store_rec, 2, blockIdx.x - J.cta_begin,
                                        J.nctas);
 }
 
@@ -585,7 +599,7 @@ int launch_instance(const TileLaunch& L) {
     if (L.smem > dyn_max) return MB2_ERR_INVALID;
     k_tile_pass<MAXT, MINB, MT, IDX, FULL><<<L.grid, L.threads, L.smem, static_cast<cudaStream_t>(L.stream)>>>(
         static_cast<double2*>(L.amps), L.n_all, L.m, L.smask, L.gmask, L.words, L.nwords, L.sdata, L.nsdata, L.gdata,
-        L.ntiles, L.pdata, L.pstride, L.param_lo, L.param_len, L.bshift, L.stages);
+        L.ntiles, L.pdata, L.pstride, L.param_lo, L.param_len, L.bshift, L.store_rec, L.stages);
     return launch_status();
 }
 

@@ -3,9 +3,9 @@
 // A pass loads every tile of 2^m amplitudes -- the amplitudes that share
 // their bits outside a set S of m qubits -- into shared memory once, applies
 // a run of blocks whose operands lie in S, and writes the tile back once.
-// A pass applies a run of consecutive blocks, in their order, and per
-// amplitude the arithmetic of every block is exactly the per-gate kernel's,
-// so the state after the sweep is bitwise the one the reference's
+// A pass applies blocks in their order (exact ones may move past blocks on
+// other qubits), and per amplitude the arithmetic of every block is exactly
+// the per-gate kernel's, so the state after the sweep is bitwise the one the reference's
 // block-by-block sweep gives
 // (src/engines/dense/fused_block.h:60-101, src/engines/dense/dense_engine.cpp:65-112).
 //
@@ -30,12 +30,21 @@ namespace {
 // more words (gate, extra word, end) and its staged entries.
 constexpr size_t kMaxBlocksPerPass = 300;
 
-size_t staged_bytes(const Block& b) {
-    const size_t dim = size_t{1} << b.k;
-    const size_t entries = b.diagonal ? dim : (b.k <= 2 ? dim * dim : 0);
-    return (cop::kPhaseWords + 3) * sizeof(uint32_t) + entries * 2 * sizeof(double);
-}
-
+// A diagonal runs in whatever phase is open; it opens one only at the pass's
+// start or behind a permutation, whose own estimate holds that.
+struct Staged {
+    uint32_t m;
+    bool mapped, c64;  // the program has permutations; it is the complex64 kernels'
+    size_t operator()(const Block& b, bool move) const {
+        const size_t dim = size_t{1} << b.k;
+        const size_t entries = move ? 0 : b.diagonal ? dim : (b.k <= 2 ? dim * dim : 0);
+        const size_t phase = b.diagonal ? 0
+                             : mapped   ? cop::phase_map_words(m) + (c64 ? 0 : cop::kMaxMapControls)
+                                        : cop::phase_words(m);
+        return (phase + (move ? 0 : 3)) * sizeof(uint32_t) + entries * 2 * sizeof(double);
+    }
+    size_t base() const { return cop::phase_map_words(m) * sizeof(uint32_t); }
+};
 
 uint32_t local_pos(uint64_t smask, uint32_t q) {
     return static_cast<uint32_t>(std::popcount(smask & ((uint64_t{1} << q) - 1)));
@@ -54,6 +63,67 @@ int mono_src(const std::vector<Cd>& m, uint32_t dim, uint32_t r) {
         }
     }
     return src;
+}
+
+// The exact permutations that a TileMap takes (X, SWAP, CX either way round),
+// or -1.
+int move_kind(const Block& b) {
+    if (b.diagonal || b.k > 2) return -1;
+    const uint32_t dim = 1u << b.k;
+    uint32_t rows = 0;
+    for (uint32_t r = 0; r < dim; ++r) {
+        const int c = mono_src(b.m, dim, r);
+        if (c < 0 || b.m[r * dim + static_cast<uint32_t>(c)] != Cd(1.0, 0.0)) return -1;
+        rows |= static_cast<uint32_t>(c) << (4 * r);
+    }
+    if (b.k == 1) return rows == 0x01u ? TK_X : -1;
+    return rows == 0x3120u ? TK_SW12 : rows == 0x1230u ? TK_SW13 : rows == 0x2310u ? TK_SW23 : -1;
+}
+
+// A two-qubit block that is an exact permutation and a one-qubit gate, in one
+// order or the other (a rotation fused with the CX before it, the commonest
+// block of an RY/RZ + CX ansatz): split into the two.  Every row of the block
+// has the gate's two entries and zeros, a zero entry's product changes at most
+// the sign of a zero, and the sum of two products does not depend on their
+// order, so the two give the block's bits -- with 12 or 14 FP64 operations per
+// amplitude instead of 30, and the permutation taken by the tile's map.
+// first, second: the parts in application order.
+bool split_block(const Block& b, Block& first, Block& second) {
+    if (b.k != 2 || b.diagonal) return false;
+    static constexpr uint32_t kPerms[4][4] = {{0, 1, 2, 3}, {0, 2, 1, 3}, {0, 3, 2, 1}, {0, 1, 3, 2}};
+    for (uint32_t r = 0; r < 4; ++r) {  // at most two entries a row
+        uint32_t entries = 0;
+        for (uint32_t c = 0; c < 4; ++c) entries += is_zero(b.m[4 * r + c]) ? 0u : 1u;
+        if (entries > 2) return false;
+    }
+    for (const auto& p : kPerms)
+        for (uint32_t t = 0; t < 2; ++t)
+            for (const bool gate_last : {true, false}) {
+                // gate_last: m[o][i] = u[o][p(i)]; else u[p(o)][i], u on operand t.
+                auto at = [&](uint32_t o, uint32_t i) { return gate_last ? b.m[4 * o + p[i]] : b.m[4 * p[o] + i]; };
+                const uint32_t bit = 1u << t;
+                const Cd u[4] = {at(0, 0), at(0, bit), at(bit, 0), at(bit, bit)};
+                bool same = true;
+                for (uint32_t o = 0; o < 4 && same; ++o)
+                    for (uint32_t i = 0; i < 4 && same; ++i)
+                        same = at(o, i) == (((o ^ i) & ~bit) ? Cd(0.0, 0.0) : u[2 * ((o >> t) & 1u) + ((i >> t) & 1u)]);
+                if (!same) continue;
+                Block perm, gate;
+                perm.k = 2;
+                perm.q[0] = b.q[0];
+                perm.q[1] = b.q[1];
+                perm.m.assign(16, Cd(0.0, 0.0));
+                for (uint32_t o = 0; o < 4; ++o) perm.m[4 * o + p[o]] = Cd(1.0, 0.0);
+                perm.diagonal = p[1] == 1 && p[2] == 2;
+                gate.k = 1;
+                gate.q[0] = b.q[t];
+                gate.m.assign(u, u + 4);
+                gate.diagonal = mb2::is_diagonal(gate.m, 2);
+                first = gate_last ? std::move(perm) : std::move(gate);
+                second = gate_last ? std::move(gate) : std::move(perm);
+                return true;
+            }
+    return false;
 }
 
 struct PassSel {
@@ -88,12 +158,36 @@ uint32_t operand_pos(uint64_t smask, uint64_t gmask, uint32_t q) {
     return kGlobalPos0 + static_cast<uint32_t>(std::popcount(gmask & ((uint64_t{1} << q) - 1)));
 }
 
-// Passes are maximal runs of CONSECUTIVE blocks whose operands fit one
-// tile -- diagonals read up to kMaxGlobalQubits qubits outside it.  Blocks
-// are never reordered, not even commuting ones: two gates on disjoint qubits
-// applied in the other order give the same state only up to rounding, and
-// the plain path is bitwise the reference's sweep, which applies the blocks
-// in plan order.
+// A block that moves amplitudes and multiplies them by 1, -1, i or -i (X, Y,
+// CX, CCX): no output is rounded.  (SWAP too, but the SWAPs that close a QFT
+// wait for the qubits that are held back: moving them saves no pass.)
+bool is_exact_move(const Block& b) {
+    if (b.diagonal || move_kind(b) == TK_SW12) return false;
+    const uint32_t dim = 1u << b.k;
+    for (uint32_t r = 0; r < dim; ++r) {
+        const int c = mono_src(b.m, dim, r);
+        if (c < 0) return false;
+        const Cd& v = b.m[r * dim + static_cast<uint32_t>(c)];
+        if (std::abs(v.real()) + std::abs(v.imag()) != 1.0 || (v.real() != 0.0 && v.imag() != 0.0)) return false;
+    }
+    return true;
+}
+
+// Passes of the plain path, bitwise the reference's sweep, which applies the
+// blocks in plan order.  Two gates on disjoint qubits applied in the other
+// order give the same state only up to rounding, so a pass takes the blocks as
+// they come until one does not fit its tile (diagonals read up to
+// kMaxGlobalQubits qubits outside it), and blocks that round never change
+// places.  An exact move is another matter.  It changes which amplitudes a
+// block on other qubits pairs with which, and their signs or parts (times
+// +-i) alike for all the amplitudes of a pair, and rounding is symmetric in
+// signs and parts: the two give the same bits in either order.  So behind the
+// block that closed the pass, exact moves still run in it when they share no
+// qubit with it nor with any block held back since.  A CX ladder then follows
+// the layer of rotations it belongs to tile by tile instead of in passes of
+// its own: the 16-qubit RY/RZ + CX ansatz of 8 layers takes 13 passes
+// instead of 28 (a CX's control, one bit for a whole tile when it lies
+// outside, need not be in it either).
 std::vector<PassSel> select_passes(const std::vector<Block>& blocks, uint32_t n, uint32_t m, uint32_t fixed_low,
                                    const std::vector<uint8_t>* parametric) {
     std::vector<PassSel> passes;
@@ -109,26 +203,56 @@ std::vector<PassSel> select_passes(const std::vector<Block>& blocks, uint32_t n,
     auto outside = [&](uint64_t s, uint64_t d) {
         return std::popcount(d & ~s) - (static_cast<int>(mt) - std::popcount(s));
     };
-    size_t i = 0;
-    while (i < blocks.size()) {
+    const uint64_t all = n >= 64 ? ~uint64_t{0} : (uint64_t{1} << n) - 1;
+    const size_t nb = blocks.size();
+    auto is_param = [&](size_t i) { return parametric != nullptr && ((*parametric)[i] & kParamBlock) != 0; };
+    std::vector<uint8_t> moves(nb), done(nb, 0);
+    std::vector<int8_t> kinds(nb, -1);
+    bool mapped = false;
+    for (size_t i = 0; i < nb; ++i) {
+        moves[i] = !is_param(i) && is_exact_move(blocks[i]);
+        if (!is_param(i)) kinds[i] = static_cast<int8_t>(move_kind(blocks[i]));
+        mapped = mapped || kinds[i] >= 0;
+    }
+    const Staged staged_of{mt, mapped, false};
+    for (size_t first = 0; first < nb;) {
         uint64_t smask = 0, dmask = 0;  // the tile's qubits so far; the diagonals' operands
         for (uint32_t q = 0; q < fixed; ++q) smask |= uint64_t{1} << q;
         PassSel sel;
-        size_t staged = 0;
-        while (i < blocks.size() && sel.gates.size() < kMaxBlocksPerPass) {
-            const bool param = parametric != nullptr && ((*parametric)[i] & kParamBlock) != 0;
+        size_t staged = staged_of.base();
+        uint64_t held = 0;  // qubits of the blocks held back, from the one that closed the pass on
+        uint64_t controls = 0;  // outside the tile
+        for (size_t i = first; i < nb && held != all && sel.gates.size() < kMaxBlocksPerPass; ++i) {
+            if (done[i]) continue;
+            const uint64_t mask = blocks[i].mask();
             uint64_t s2 = smask, d2 = dmask;
-            if (diagonal_any_operand(blocks[i], param)) d2 |= blocks[i].mask();
-            else s2 |= blocks[i].mask();
-            if (static_cast<uint32_t>(std::popcount(s2)) > mt) break;
-            if (outside(s2, d2) > static_cast<int>(kMaxGlobalQubits)) break;
-            if (staged + staged_bytes(blocks[i]) > kMaxStagedBytes && !sel.gates.empty()) break;
-            staged += staged_bytes(blocks[i]);
+            // A CX needs its target in the tile; its control may be read outside it.
+            const int kind = kinds[i];
+            const bool cx = kind == TK_SW13 || kind == TK_SW23;
+            const uint64_t control = cx ? uint64_t{1} << blocks[i].q[kind == TK_SW13 ? 0 : 1] : 0;
+            if (diagonal_any_operand(blocks[i], is_param(i))) d2 |= mask;
+            else if (cx && (s2 & control) == 0 && std::popcount(controls | control) <= static_cast<int>(cop::kMaxMapControls)) {
+                s2 |= mask & ~control;
+                d2 |= control;
+            } else s2 |= mask;
+            const bool fits = static_cast<uint32_t>(std::popcount(s2)) <= mt &&
+                              outside(s2, d2) <= static_cast<int>(kMaxGlobalQubits) &&
+                              (staged + staged_of(blocks[i], kind >= 0) <= kMaxStagedBytes || sel.gates.empty());
+            if (!fits || (held != 0 && (!moves[i] || (mask & held) != 0))) {
+                // (A move that does not fit closes the pass as any block does,
+                // and no other move passes it.)
+                if (held == 0 && moves[i]) break;
+                held |= mask;
+                continue;
+            }
+            staged += staged_of(blocks[i], kind >= 0);
             smask = s2;
             dmask = d2;
+            if (cx && (s2 & control) == 0) controls |= control;
             sel.gates.push_back(static_cast<uint32_t>(i));
-            ++i;
+            done[i] = 1;
         }
+        while (first < nb && done[first]) ++first;
         // Pad the tile to exactly mt qubits: first with the diagonals'
         // operands the global limit leaves out, then with the lowest unused
         // qubits (longer contiguous runs per tile).
@@ -159,19 +283,40 @@ uint32_t push_matrix(std::vector<double>& data, const std::vector<Cd>& m) {
 // positions): the first three thread bits get distinct residues mod 3 when
 // possible, so that the eight threads of a quarter warp hit eight distinct
 // 16-byte bank groups under the kernel's XOR-fold swizzle.
-void thread_bit_order(uint32_t m, const uint32_t* reg, uint32_t nreg, uint8_t* tperm, uint8_t& nthread) {
+void thread_bit_order(uint32_t m, const uint32_t* reg, uint32_t nreg, uint8_t* tperm, uint8_t& nthread,
+                      const TileMap* map, bool slots8) {
     std::vector<uint32_t> free_pos;
     for (uint32_t p = 0; p < m; ++p)
         if (std::find(reg, reg + nreg, p) == reg + nreg) free_pos.push_back(p);
     std::vector<uint32_t> order;
-    for (uint32_t res = 0; res < 3; ++res) {
+    const bool by_place = map != nullptr && !map->identity();
+    if (by_place) {
+        // The bank groups of a slot are its low bits (16-byte slots: three,
+        // 8-byte: four), linear in the place: bits whose places have
+        // independent ones first, by elimination.
+        const uint32_t want = slots8 ? 4 : 3, low = (1u << want) - 1;
+        uint32_t basis[4] = {0, 0, 0, 0};
+        for (uint32_t p : free_pos) {
+            if (order.size() == want) break;
+            uint32_t v = (slots8 ? swz8(map->col[p]) : swz(map->col[p])) & low;
+            for (uint32_t b = want; b-- > 0;) {
+                if (!((v >> b) & 1u)) continue;
+                if (basis[b] == 0) {
+                    basis[b] = v;
+                    order.push_back(p);
+                    break;
+                }
+                v ^= basis[b];
+            }
+        }
+    } else for (uint32_t res = 0; res < 3; ++res) {
         for (uint32_t p : free_pos)
             if (p % 3 == res && std::find(order.begin(), order.end(), p) == order.end()) {
                 order.push_back(p);
                 break;
             }
     }
-    if (order.size() < 3) order.clear();
+    if (order.size() < 3 && !by_place) order.clear();
     for (uint32_t p : free_pos)
         if (std::find(order.begin(), order.end(), p) == order.end()) order.push_back(p);
     nthread = static_cast<uint8_t>(order.size());
@@ -187,8 +332,11 @@ void thread_bit_order(uint32_t m, const uint32_t* reg, uint32_t nreg, uint8_t* t
 // the blocks are ordered phase by phase: every ready block that a register
 // set of four qubits (or no register at all: diagonals) can take, then the
 // next set from the ready dense blocks, so the kernel changes phase rarely.
+// Exact permutations need no registers either, but end the phase they come
+// in (the amplitudes' places change), so they wait until no other block of
+// the pass is ready.
 std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, uint32_t n, uint32_t m,
-                                             uint32_t fixed_low) {
+                                             uint32_t fixed_low, const std::vector<uint8_t>* parametric) {
     std::vector<PassSel> passes;
     uint32_t widest = 1;
     for (const Block& b : blocks) widest = std::max(widest, b.k);
@@ -197,6 +345,13 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
     const uint32_t fixed = std::min(fixed_low, mt - widest);
     const uint32_t nb = static_cast<uint32_t>(blocks.size());
     std::vector<std::vector<uint32_t>> lists(n);
+    std::vector<uint8_t> moves(nb, 0);
+    bool mapped = false;
+    for (uint32_t i = 0; i < nb; ++i) {
+        moves[i] = !(parametric != nullptr && ((*parametric)[i] & kParamBlock) != 0) && move_kind(blocks[i]) >= 0;
+        mapped = mapped || moves[i];
+    }
+    const Staged staged_of{mt, mapped, true};
     for (uint32_t i = 0; i < nb; ++i)
         for (uint32_t t = 0; t < blocks[i].k; ++t) lists[blocks[i].q[t]].push_back(i);
     std::vector<uint32_t> head(n, 0);
@@ -212,7 +367,7 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
     std::vector<uint32_t> work;
     auto closure = [&](uint64_t s, std::vector<uint32_t>& h, std::vector<uint32_t>* out, bool limit) {
         uint32_t count = 0;
-        size_t staged = 0;
+        size_t staged = staged_of.base();
         work.clear();
         for (uint32_t x = 0; x < n; ++x)
             if ((s >> x) & 1u) work.push_back(x);
@@ -223,9 +378,9 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
             const uint32_t i = lists[x][h[x]];
             if ((blocks[i].mask() & ~s) != 0 || !at_head(h, i)) continue;
             if (limit && (count >= kMaxBlocksPerPass ||
-                          (count > 0 && staged + staged_bytes(blocks[i]) > kMaxStagedBytes)))
+                          (count > 0 && staged + staged_of(blocks[i], moves[i] != 0) > kMaxStagedBytes)))
                 break;
-            staged += staged_bytes(blocks[i]);
+            staged += staged_of(blocks[i], moves[i] != 0);
             ++count;
             if (out) out->push_back(i);
             for (uint32_t t = 0; t < blocks[i].k; ++t) {
@@ -293,7 +448,7 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
                         if (hh[x] >= lists[x].size()) continue;
                         const uint32_t i = lists[x][hh[x]];
                         const Block& b = blocks[i];
-                        if (!in[i] || b.diagonal != diag || !at_head(hh, i) ||
+                        if (!in[i] || b.diagonal != diag || moves[i] || !at_head(hh, i) ||
                             !(b.diagonal || b.k > 2 || (b.mask() & ~regs) == 0))
                             continue;
                         in[i] = 0;
@@ -321,7 +476,32 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
             // blocks use, then the lowest).
             uint64_t cand = 0;
             for (uint32_t i : members)
-                if (in_pass[i] && !blocks[i].diagonal && blocks[i].k <= 2) cand |= blocks[i].mask();
+                if (in_pass[i] && !blocks[i].diagonal && blocks[i].k <= 2 && !moves[i]) cand |= blocks[i].mask();
+            // Nothing but permutations ready: those that are.
+            bool ready = false;
+            for (uint32_t i : members)
+                ready = ready || (in_pass[i] && !blocks[i].diagonal && blocks[i].k <= 2 && !moves[i] && at_head(ph, i));
+            if (!ready) {
+                bool any = false;
+                for (bool again = true; again;) {
+                    again = false;
+                    for (uint32_t x = 0; x < n; ++x) {
+                        if (!((s >> x) & 1u) || ph[x] >= lists[x].size()) continue;
+                        const uint32_t i = lists[x][ph[x]];
+                        if (!in_pass[i] || !moves[i] || !at_head(ph, i)) continue;
+                        in_pass[i] = 0;
+                        again = any = true;
+                        sel.gates.push_back(i);
+                        --left;
+                        for (uint32_t t = 0; t < blocks[i].k; ++t) ++ph[blocks[i].q[t]];
+                    }
+                }
+                if (any && left == 0) break;
+                if (any) {
+                    regs = 0;
+                    continue;
+                }
+            }
             regs = 0;
             for (uint32_t r = 0; r < kRegQubits && (cand & ~regs) != 0; ++r) {
                 uint64_t best_score = 0;
@@ -333,8 +513,8 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
                     const uint64_t runs = run(regs | (uint64_t{1} << x), sim, sim_in, nullptr);
                     uint32_t uses = 0;
                     for (uint32_t i : members)
-                        if (in_pass[i] && !blocks[i].diagonal && blocks[i].k <= 2 && ((blocks[i].mask() >> x) & 1u) &&
-                            at_head(ph, i))
+                        if (in_pass[i] && !blocks[i].diagonal && blocks[i].k <= 2 && !moves[i] &&
+                            ((blocks[i].mask() >> x) & 1u) && at_head(ph, i))
                             ++uses;
                     const uint64_t score = (runs << 16) | uses;
                     if (best == n || score > best_score) {
@@ -354,23 +534,90 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
     return passes;
 }
 
-TileProgram plan_tile_program(const std::vector<Block>& blocks, uint32_t n, uint32_t m, uint32_t fixed_low,
-                              const std::vector<uint8_t>* parametric, bool commuting) {
+TileProgram plan_tile_program(const std::vector<Block>& all, uint32_t n, uint32_t m, uint32_t fixed_low,
+                              const std::vector<uint8_t>* all_parametric, bool commuting, bool split) {
+    // The blocks as they are planned: origin[i] the caller's block that part i
+    // belongs to, last[i] whether it completes it.
+    std::vector<Block> parts;
+    std::vector<uint8_t> part_flags, last;
+    std::vector<uint32_t> origin;
+    for (size_t i = 0; i < all.size() && split; ++i) {
+        Block first, second;
+        const uint8_t flags = all_parametric ? (*all_parametric)[i] : uint8_t{0};
+        const bool two = !(flags & kParamBlock) && move_kind(all[i]) < 0 && split_block(all[i], first, second);
+        if (two && parts.empty()) {  // from here on the parts are a list of their own
+            parts.assign(all.begin(), all.begin() + static_cast<long>(i));
+            for (uint32_t j = 0; j < i; ++j) {
+                origin.push_back(j);
+                last.push_back(1);
+                part_flags.push_back(all_parametric ? (*all_parametric)[j] : uint8_t{0});
+            }
+            if (i == 0) parts.reserve(all.size() + 1);
+        }
+        if (two) {
+            for (Block* p : {&first, &second}) {
+                if (p->diagonal && p->k == 2) continue;  // the identity
+                parts.push_back(std::move(*p));
+                origin.push_back(static_cast<uint32_t>(i));
+                last.push_back(0);
+                part_flags.push_back(0);
+            }
+            last.back() = 1;
+        } else if (!origin.empty()) {
+            parts.push_back(all[i]);
+            origin.push_back(static_cast<uint32_t>(i));
+            last.push_back(1);
+            part_flags.push_back(flags);
+        }
+    }
+    const bool whole = origin.empty();
+    const std::vector<Block>& blocks = whole ? all : parts;
+    const std::vector<uint8_t>* parametric = whole || all_parametric == nullptr ? all_parametric : &part_flags;
+    auto origin_of = [&](uint32_t i) { return whole ? i : origin[i]; };
     if (m < kMinTileQubits || m > kMaxTileQubitsC64) throw std::invalid_argument("tile width out of range");
     TileProgram prog;
     const uint32_t mt = std::min(m, n);
     if (mt < kRegQubits) throw std::invalid_argument("state too small for the tile kernel");
     const std::vector<PassSel> sels =
-        commuting ? select_passes_commuting(blocks, n, mt, fixed_low)
+        commuting ? select_passes_commuting(blocks, n, mt, fixed_low, parametric)
                   : select_passes(blocks, n, mt, fixed_low, parametric);
-    prog.param_offsets.assign(blocks.size(), 0);
+    prog.c64 = commuting;
+    prog.param_offsets.assign(all.size(), 0);
     auto param_flags = [&](uint32_t bi) -> uint8_t { return parametric ? (*parametric)[bi] : uint8_t{0}; };
     // A parametric block's data goes to the per-binding record.
     auto push_param = [&](uint32_t bi, uint32_t doubles) {
         const uint32_t off = prog.param_stride;
-        prog.param_offsets[bi] = off;
+        prog.param_offsets[origin_of(bi)] = off;
         prog.param_stride += (doubles + 1) & ~1u;  // keep 16-byte alignment
         return off;
+    };
+    // The caller's blocks in an order of whole blocks that the parts' order
+    // amounts to: one is listed when it is complete and every earlier block on
+    // its qubits is.  Returns how many that made.
+    std::vector<std::vector<uint32_t>> waiting(n);  // per qubit, latest block first
+    for (uint32_t i = static_cast<uint32_t>(all.size()); i-- > 0;)
+        for (uint32_t t = 0; t < all[i].k; ++t) waiting[all[i].q[t]].push_back(i);
+    std::vector<uint8_t> ready(all.size(), 0);
+    std::vector<uint32_t> look;
+    auto complete = [&](uint32_t i) {
+        uint32_t listed = 0;
+        ready[i] = 1;
+        look.assign(1, i);
+        while (!look.empty()) {
+            const uint32_t b = look.back();
+            look.pop_back();
+            bool first = ready[b] != 0;
+            for (uint32_t t = 0; t < all[b].k && first; ++t)
+                first = !waiting[all[b].q[t]].empty() && waiting[all[b].q[t]].back() == b;
+            if (!first) continue;
+            prog.order.push_back(b);
+            prog.order_pass.push_back(static_cast<uint32_t>(prog.passes.size()));
+            ++listed;
+            for (uint32_t t = 0; t < all[b].k; ++t) waiting[all[b].q[t]].pop_back();
+            for (uint32_t t = 0; t < all[b].k; ++t)
+                if (!waiting[all[b].q[t]].empty()) look.push_back(waiting[all[b].q[t]].back());
+        }
+        return listed;
     };
     for (const PassSel& sel : sels) {
         TilePass pass;
@@ -379,12 +626,12 @@ TileProgram plan_tile_program(const std::vector<Block>& blocks, uint32_t n, uint
         pass.gmask = sel.gmask;
         pass.prog_begin = static_cast<uint32_t>(prog.instrs.size());
         pass.sdata_begin = static_cast<uint32_t>(prog.data.size());
-        pass.gates = static_cast<uint32_t>(sel.gates.size());
         auto push_staged = [&](const std::vector<Cd>& m) {
             return push_matrix(prog.data, m) - pass.sdata_begin;
         };
 
         bool open = false;
+        TileMap map;
         uint32_t reg[kRegQubits];
         for (uint32_t r = 0; r < kRegQubits; ++r) reg[r] = r;
         auto in_reg = [&](uint32_t p) -> int {
@@ -407,6 +654,7 @@ TileProgram plan_tile_program(const std::vector<Block>& blocks, uint32_t n, uint
             std::vector<uint32_t> r(first);
             for (size_t j = from; j < sel.gates.size() && r.size() < kRegQubits; ++j) {
                 const Block& b = blocks[sel.gates[j]];
+                if (!(param_flags(sel.gates[j]) & kParamBlock) && move_kind(b) >= 0) break;  // the phase ends there
                 if (b.diagonal || b.k > 2) continue;
                 bool fits = true;
                 uint32_t extra = 0;
@@ -425,7 +673,7 @@ TileProgram plan_tile_program(const std::vector<Block>& blocks, uint32_t n, uint
             TileInstr ph{};
             ph.op = TOP_PHASE;
             for (uint32_t s = 0; s < kRegQubits; ++s) ph.pos[s] = static_cast<uint8_t>(reg[s]);
-            thread_bit_order(mt, reg, kRegQubits, ph.tperm, ph.nthread);
+            thread_bit_order(mt, reg, kRegQubits, ph.tperm, ph.nthread, &map, commuting);
             prog.instrs.push_back(ph);
             open = true;
         };
@@ -441,10 +689,20 @@ TileProgram plan_tile_program(const std::vector<Block>& blocks, uint32_t n, uint
         for (size_t j = 0; j < sel.gates.size(); ++j) {
             const Block& b = blocks[sel.gates[j]];
             const uint32_t dim = 1u << b.k;
-            prog.order.push_back(sel.gates[j]);
-            prog.order_pass.push_back(static_cast<uint32_t>(prog.passes.size()));
+            if (whole || last[sel.gates[j]]) pass.gates += complete(origin_of(sel.gates[j]));
             TileInstr g{};
             g.k = static_cast<uint8_t>(b.k);
+            const int move = param_flags(sel.gates[j]) & kParamBlock ? -1 : move_kind(b);
+            if (move >= 0) {
+                close_phase();
+                g.op = TOP_MOVE;
+                g.kind = static_cast<uint8_t>(move);
+                for (uint32_t t = 0; t < b.k; ++t)
+                    g.pos[t] = static_cast<uint8_t>(operand_pos(sel.smask, sel.gmask, b.q[t]));
+                map.move(g);
+                prog.instrs.push_back(g);
+                continue;
+            }
             if (b.diagonal) {
                 if (!open) open_phase({}, j + 1);
                 g.op = TOP_DIAG;
@@ -517,24 +775,7 @@ TileProgram plan_tile_program(const std::vector<Block>& blocks, uint32_t n, uint
                 if (mono) {
                     g.kind = TK_MONO;
                     g.aux = aux;
-                    // Exact permutations run as register moves.
-                    bool ones = true;
-                    for (uint32_t r = 0; r < dim; ++r) {
-                        const uint32_t src = (aux >> (3 * r)) & 7u;
-                        if (src == 7u || b.m[r * dim + src] != Cd(1.0, 0.0) || std::signbit(b.m[r * dim + src].imag()))
-                            ones = false;
-                    }
-                    auto is_perm = [&](std::initializer_list<uint32_t> srcs) {
-                        uint32_t r = 0;
-                        for (uint32_t v : srcs)
-                            if (((aux >> (3 * r++)) & 7u) != v) return false;
-                        return true;
-                    };
-                    if (ones && b.k == 1 && is_perm({1, 0})) g.kind = TK_X;
-                    else if (ones && b.k == 2 && is_perm({0, 2, 1, 3})) g.kind = TK_SW12;
-                    else if (ones && b.k == 2 && is_perm({0, 3, 2, 1})) g.kind = TK_SW13;
-                    else if (ones && b.k == 2 && is_perm({0, 1, 3, 2})) g.kind = TK_SW23;
-                    prog.fp64_per_amp += (g.kind == TK_MONO) ? 6 : 0;
+                    prog.fp64_per_amp += 6;
                 } else if (b.k == 1) {
                     bool all_real = is_real(b.m[0]) && is_real(b.m[1]) && is_real(b.m[2]) && is_real(b.m[3]);
                     bool m00_real = is_real(b.m[0]);
@@ -565,8 +806,15 @@ TileProgram plan_tile_program(const std::vector<Block>& blocks, uint32_t n, uint
                 prog.instrs.push_back(g);
                 continue;
             }
-            // Wider dense block: from shared memory, as a phase of its own.
+            // Wider dense block: from shared memory, as a phase of its own, with
+            // the amplitudes at their own index.
             close_phase();
+            if (!map.identity()) {
+                open_phase({}, sel.gates.size());
+                prog.instrs.back().kind = 1;  // settle
+                close_phase();
+                map = TileMap();
+            }
             g.op = TOP_SMEM;
             for (uint32_t t = 0; t < b.k; ++t) g.pos[t] = static_cast<uint8_t>(local_pos(sel.smask, b.q[t]));
             if (param_flags(sel.gates[j]) & kParamBlock)

@@ -455,6 +455,20 @@ void run_program_on_host(const TileProgram& prog, uint32_t n, Cd* state) {
                     break;
                 case TOP_END:
                     break;
+                case TOP_MOVE: {
+                    const uint32_t dim = 1u << g.k;
+                    std::vector<Cd> m(size_t{dim} * dim, Cd(0.0, 0.0));
+                    for (uint32_t r = 0; r < dim; ++r) {
+                        const uint32_t from = g.kind == TK_X ? r ^ 1u
+                                              : g.kind == TK_SW12 ? ((r >> 1) | ((r & 1u) << 1))
+                                              : g.kind == TK_SW13 ? r ^ ((r & 1u) << 1)
+                                                                  : r ^ (r >> 1);
+                        m[r * dim + from] = Cd(1.0, 0.0);
+                    }
+                    for (uint32_t t = 0; t < g.k; ++t) ops[t] = qubit_at(g.pos[t]);
+                    host_apply_generic(state, amps, m.data(), ops, g.k);
+                    break;
+                }
                 case TOP_MMA: {
                     for (uint32_t s = 0; s < kRegQubits; ++s) ops[s] = qubit[reg[s]];
                     const Cd* u = prog.tcmatrices.data() + size_t{pass.tc_begin / kTcOperandWords + g.aux} * kDim * kDim;
