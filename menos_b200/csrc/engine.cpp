@@ -225,6 +225,8 @@ struct ExpectPlan {
         const auto *dx = reinterpret_cast<const uint64_t*>(base), *dz = reinterpret_cast<const uint64_t*>(base + off_z);
         auto* partials = reinterpret_cast<double*>(base + off_p);
         int rc = MB2_OK;
+        // The groups' CTAs write fewer partials than a streaming term's.
+        MB2_CUDA(ctx, cudaMemsetAsync(partials, 0, size_t{num_terms} * mb2::kExpBlocks * 16, s));
         for (const mb2::PauliGroupPlan& g : plan.groups) {
             if (g.nterms == 1 || g.c + g.d < mb2::kPauliMinTileQubits) {
                 // Nothing to share (or a state too small for the grouped tiles):
@@ -238,7 +240,7 @@ struct ExpectPlan {
                 rc = mb2::launch_pauli_group(amps, n, g.c, g.d,
                                              reinterpret_cast<const uint64_t*>(base + off_s) + g.span_off, g.free_mask,
                                              base + off_t + size_t{g.term_off} * sizeof(mb2::PauliGroupTerm), g.nterms,
-                                             partials, mb2::kExpBlocks, s, precision);
+                                             partials, mb2::kPauliGroupBlocks, mb2::kExpBlocks, s, precision);
             }
             if (rc != MB2_OK) break;
         }

@@ -160,15 +160,16 @@ __global__ void __launch_bounds__(kFinishThreads)
 // same pair gives the same s(m) Re t (or s(m) Im t), so a pair may equally be
 // visited once with weight 2 or from both members with weight 1.
 //
-// Thread r of the CTA owns tile amplitudes L = r | i << 8 (i < 2^(c+d-8),
-// four or eight), read into registers once per tile; per term it visits its
+// Thread r of the CTA owns tile amplitudes L = r | i << 9 (i < 2^(c+d-9),
+// two or four), read into registers once per tile; per term it visits its
 // own amplitudes and reads only the partners from shared memory.  When dl
-// has a bit b >= 8 the visiting member is the one with bit b clear (half of
+// has a bit b >= 9 (the plan's coordinates give most terms the highest bit of
+// the tile index) the visiting member is the one with bit b clear (half of
 // every thread's amplitudes, weight 2); otherwise every member visits
 // (weight 1).  s(m) is linear over XOR in the tile index apart from the
-// coset representative: s = parity(z_hi & rep) ^ sigma(r) ^ sigma(i << 8),
+// coset representative: s = parity(z_hi & rep) ^ sigma(r) ^ sigma(i << 9),
 // with sigma(L) = parity(z_lo & L) ^ parity(z_hi & span[L >> c]); the
-// thread's sigma(r) of every term is a register bit mask, sigma(i << 8) a
+// thread's sigma(r) of every term is a register bit mask, sigma(i << 9) a
 // per-term byte.  Each term runs a body compiled for its (own count,
 // visiting bit, mode): its products are independent and summed as a
 // balanced tree before one add into the thread's accumulator of the term
@@ -177,9 +178,9 @@ __global__ void __launch_bounds__(kFinishThreads)
 // the finish kernel.
 using GroupTerm = PauliGroupTerm;
 constexpr uint32_t kChunkWords = (1u << kPauliMaxSpan) / 32;
-constexpr uint32_t kOwnShift = 8;  // log2(kThreads): tile bits of the thread index
+constexpr uint32_t kOwnShift = 9;  // log2(kGroupThreads): tile bits of the thread index
+constexpr int kGroupThreads = 1 << kOwnShift;
 constexpr uint32_t kMaxOwn = 1u << (kPauliTileQubits - kOwnShift);
-static_assert(kThreads == (1 << kOwnShift), "one thread per low tile index");
 static_assert(kPauliMinTileQubits >= kOwnShift + 1, "every thread owns at least two amplitudes");
 
 // cp.async of one amplitude (16 or 8 bytes), global -> shared.
@@ -200,12 +201,23 @@ struct GroupShared {
     uint32_t cpar[kMaxGroupTerms][kChunkWords];  // parity of z_hi & span[k], bit k
     uint32_t tdl[kMaxGroupTerms], tzl[kMaxGroupTerms], tmode[kMaxGroupTerms];
     uint32_t tcode[kMaxGroupTerms];  // the term's body (term_body)
-    uint32_t tsigi[kMaxGroupTerms];  // bit i: sigma(i << 8)
+    // The terms in the order they are reduced, the regular ones (below) first:
+    // per place the term, what its body needs in one word -- dl, its code from
+    // bit 16 (a regular term: its mode), and from bit 24 sigma(i << kOwnShift)
+    // per own amplitude i; one more to read ahead -- and its high z bits.
+    uint32_t place[kMaxGroupTerms], regular;
+    uint32_t tword[kMaxGroupTerms + 1];
+    uint64_t pzh[32];  // zero past the terms
     uint32_t tweight[kMaxGroupTerms];  // 2: each pair visited once; 1: from both members
     uint64_t tzh[kMaxGroupTerms];
-    double acc[kMaxGroupTerms][kThreads];
-    double red[kThreads / 32];
+    double red[kGroupThreads / 32];
 };
+// Every thread's accumulator of every term follows the tile buffers in
+// dynamic shared memory: acc[t * kGroupThreads + thread].  Regular terms --
+// those whose pairs differ in the tile index's highest bit, in tiles of four
+// own amplitudes: nearly all, by the plan's choice of coordinates -- have
+// theirs in registers while the tiles are read, up to kRegularTerms of them.
+constexpr uint32_t kRegularTerms = 8;
 
 // sigma(L): the sign parity of tile index L without the coset's part.
 __device__ __forceinline__ uint32_t group_sigma(const GroupShared& g, uint32_t t, uint32_t L, uint32_t c) {
@@ -214,22 +226,24 @@ __device__ __forceinline__ uint32_t group_sigma(const GroupShared& g, uint32_t t
 }
 
 // Term bodies: (own amplitudes, selector bit, mode).  Code = base of the
-// own count (0 for four, 7 for eight) + 0 for a Z string, else
+// own count (0 for two, 5 for four) + 0 for a Z string, else
 // 1 + 2 * (selector bit + 1) + (mode - 1), the selector bit -1 meaning every
 // member visits.
 __host__ __device__ constexpr uint32_t body_code(uint32_t own, int selb, uint32_t mode) {
-    return (own == 8 ? 7u : 0u) + (mode == 0 ? 0u : 1u + 2u * static_cast<uint32_t>(selb + 1) + (mode - 1));
+    return (own == 4 ? 5u : 0u) + (mode == 0 ? 0u : 1u + 2u * static_cast<uint32_t>(selb + 1) + (mode - 1));
 }
 
 // Fills the tables and clears the accumulators; returns this thread's
-// sigma(r) of every term (bit t).
-__device__ __forceinline__ uint32_t group_setup(GroupShared& g, uint32_t c, uint32_t d,
+// sigma(r) of every term (bit p: the term at place p).
+__device__ __forceinline__ uint32_t group_setup(GroupShared& g, double* acc, uint32_t c, uint32_t d,
                                                 const uint64_t* __restrict__ span,
                                                 const GroupTerm* __restrict__ terms, uint32_t nterms) {
     const uint32_t nchunks = 1u << d;
     const uint32_t own = 1u << (c + d - kOwnShift);
-    for (uint32_t i = threadIdx.x; i < nchunks; i += kThreads) g.sspan[i] = span[i];
-    for (uint32_t t = threadIdx.x; t < nterms; t += kThreads) {
+    for (uint32_t i = threadIdx.x; i < nchunks; i += kGroupThreads) g.sspan[i] = span[i];
+    if (threadIdx.x < 32) g.pzh[threadIdx.x] = 0;
+    __syncthreads();
+    for (uint32_t t = threadIdx.x; t < nterms; t += kGroupThreads) {
         const GroupTerm T = terms[t];
         const uint32_t dl = (T.kx << c) | T.xl;
         g.tdl[t] = dl;
@@ -245,9 +259,9 @@ __device__ __forceinline__ uint32_t group_setup(GroupShared& g, uint32_t c, uint
         g.tcode[t] = body_code(own, mode == 0 ? -1 : selb, mode);
         g.tweight[t] = (mode != 0 && selb >= 0) ? 2u : 1u;
     }
-    for (uint32_t i = threadIdx.x; i < kMaxGroupTerms * kThreads; i += kThreads) (&g.acc[0][0])[i] = 0.0;
+    for (uint32_t i = threadIdx.x; i < nterms * kGroupThreads; i += kGroupThreads) acc[i] = 0.0;
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < kMaxGroupTerms * kChunkWords; i += kThreads) {
+    for (uint32_t i = threadIdx.x; i < kMaxGroupTerms * kChunkWords; i += kGroupThreads) {
         const uint32_t t = i / kChunkWords, w = i % kChunkWords;
         uint32_t bits = 0;
         if (t < nterms)
@@ -256,13 +270,29 @@ __device__ __forceinline__ uint32_t group_setup(GroupShared& g, uint32_t c, uint
         g.cpar[t][w] = bits;
     }
     __syncthreads();
-    for (uint32_t t = threadIdx.x; t < nterms; t += kThreads) {
+    auto is_regular = [&](uint32_t t) { return own == 4 && g.tmode[t] != 0 && (g.tdl[t] >> (kOwnShift + 1)) != 0; };
+    if (threadIdx.x == 0) {
+        uint32_t n = 0;
+        for (uint32_t t = 0; t < nterms && n < kRegularTerms; ++t)
+            if (is_regular(t)) g.place[n++] = t;
+        g.regular = n;
+        uint32_t left = 0;  // regular terms past the registers' go with the others
+        for (uint32_t t = 0; t < nterms; ++t) {
+            if (is_regular(t) && left++ < kRegularTerms) continue;
+            g.place[n++] = t;
+        }
+        g.tword[nterms] = 0;
+    }
+    __syncthreads();
+    for (uint32_t p = threadIdx.x; p < nterms; p += kGroupThreads) {
+        const uint32_t t = g.place[p];
         uint32_t bits = 0;
         for (uint32_t i = 0; i < own; ++i) bits |= group_sigma(g, t, i << kOwnShift, c) << i;
-        g.tsigi[t] = bits;
+        g.tword[p] = g.tdl[t] | ((p < g.regular ? g.tmode[t] : g.tcode[t]) << 16) | (bits << 24);
+        g.pzh[p] = g.tzh[t];
     }
     uint32_t sig = 0;
-    for (uint32_t t = 0; t < nterms; ++t) sig |= group_sigma(g, t, threadIdx.x, c) << t;
+    for (uint32_t p = 0; p < nterms; ++p) sig |= group_sigma(g, g.place[p], threadIdx.x, c) << p;
     __syncthreads();
     return sig;
 }
@@ -273,7 +303,8 @@ __device__ __forceinline__ double flip_if(double v, uint32_t f) {
 }
 
 // One term's share of this thread's own amplitudes in one tile, as a
-// balanced sum in a fixed order: OWN own amplitudes, SELB the register bit
+// balanced sum in a fixed order, the second product of each pair added
+// without a rounding of its own (FMA): OWN own amplitudes, SELB the register bit
 // that marks the non-visiting member (-1: all visit), MODE 0 (|a|^2),
 // 1 (Re conj(a) b) or 2 (Im conj(a) b); sg bit i: the sign of own
 // amplitude i.  Every branch is resolved at compile time.
@@ -289,11 +320,11 @@ __device__ __forceinline__ double term_body(const double2 (&a)[kMaxOwn], const A
         const int i = SELB < 0 ? k : (((k >> SB) << (SB + 1)) | (k & ((1 << SB) - 1)));
         double x;
         if constexpr (MODE == 0) {
-            x = __dadd_rn(__dmul_rn(a[i].x, a[i].x), __dmul_rn(a[i].y, a[i].y));
+            x = __fma_rn(a[i].x, a[i].x, __dmul_rn(a[i].y, a[i].y));
         } else {
             const double2 b = as_d2(cur[(r | (static_cast<uint32_t>(i) << kOwnShift)) ^ dl]);
-            x = MODE == 1 ? __dadd_rn(__dmul_rn(a[i].x, b.x), __dmul_rn(a[i].y, b.y))
-                          : __dsub_rn(__dmul_rn(a[i].x, b.y), __dmul_rn(a[i].y, b.x));
+            x = MODE == 1 ? __fma_rn(a[i].x, b.x, __dmul_rn(a[i].y, b.y))
+                          : __fma_rn(a[i].x, b.y, -__dmul_rn(a[i].y, b.x));
         }
         v[k] = flip_if(x, (sg >> i) & 1u);
     }
@@ -306,8 +337,20 @@ __device__ __forceinline__ double term_body(const double2 (&a)[kMaxOwn], const A
 
 // Adds one gathered coset tile (representative rep) to every term's
 // accumulator.  sig: this thread's sigma(r) bits (group_setup).
+//
+// Bound by shared memory and issue slots: a term is its partner loads, a
+// handful of FP64 operations, and what steers them.  So the cosets' signs of
+// all terms come from one ballot per tile, a term's tables are one word, 512
+// threads own four amplitudes each (32 warps per SM hide what 16 did not), and
+// a regular term is two partner loads and eight FP64 operations without a
+// branch: the mode picks the parts that multiply the partner's by selects,
+// the signs ride on them, the sum stays in a register.  64 strings at 27
+// qubits: 7.06 ms with 256 threads, eight own amplitudes and a branch and a
+// shared-memory sum per term; 6.31 with one word per term and 512 threads;
+// 5.5 now.
 template <typename A>
-__device__ __forceinline__ void group_tile(GroupShared& g, const A* __restrict__ cur, uint64_t rep,
+__device__ __forceinline__ void group_tile(GroupShared& g, double (&reg)[kRegularTerms], double* __restrict__ acc,
+                                           const A* __restrict__ cur, uint64_t rep,
                                            uint32_t tile_amps, uint32_t nterms, uint32_t sig) {
     const uint32_t r = threadIdx.x;
     const uint32_t own = tile_amps >> kOwnShift;
@@ -315,13 +358,41 @@ __device__ __forceinline__ void group_tile(GroupShared& g, const A* __restrict__
 #pragma unroll
     for (uint32_t i = 0; i < kMaxOwn; ++i)
         a[i] = i < own ? as_d2(cur[r | (i << kOwnShift)]) : make_double2(0.0, 0.0);
-    for (uint32_t t = 0; t < nterms; ++t) {
+    // Bit p: the sign of the term at place p at this thread's first amplitude.
+    const uint32_t signs = sig ^ __ballot_sync(0xffffffffu, __popcll(g.pzh[r & 31u] & rep) & 1);
+    const uint32_t regular = g.regular;
+#pragma unroll
+    for (uint32_t p = 0; p < kRegularTerms; ++p) {
+        if (p >= regular) break;  // (uniform over the CTA)
+        const uint32_t word = g.tword[p], s0 = signs >> p;
+        const bool imag = (word >> 17) & 1u;  // mode 2
+        const uint32_t at = r ^ (word & 0xffffu);
+        double v[2];
+#pragma unroll
+        for (uint32_t i = 0; i < 2; ++i) {  // the own amplitudes whose highest bit is clear
+            const double2 b = as_d2(cur[at ^ (i << kOwnShift)]);
+            const uint32_t flip = s0 ^ (word >> (24 + i));
+            // Re: a.x b.x + a.y b.y; Im: -a.y b.x + a.x b.y.
+            const double px = flip_if(imag ? a[i].y : a[i].x, (flip ^ (imag ? 1u : 0u)) & 1u);
+            const double py = flip_if(imag ? a[i].x : a[i].y, flip & 1u);
+            v[i] = __fma_rn(px, b.x, __dmul_rn(py, b.y));
+        }
+        reg[p] = __dadd_rn(reg[p], __dadd_rn(v[0], v[1]));
+    }
+    uint32_t next = g.tword[regular];
+    for (uint32_t t = regular; t < nterms; ++t) {
+        const uint32_t word = next;
+        next = g.tword[t + 1];
         // Bit i: the sign of own amplitude i.
-        const uint32_t s0 = (static_cast<uint32_t>(__popcll(g.tzh[t] & rep)) ^ (sig >> t)) & 1u;
-        const uint32_t sg = g.tsigi[t] ^ (0u - s0);
-        const uint32_t dl = g.tdl[t];
+        const uint32_t sg = (word >> 24) ^ (0u - ((signs >> t) & 1u));
+        const uint32_t dl = word & 0xffffu;
         double v = 0.0;
-        switch (g.tcode[t]) {
+        switch ((word >> 16) & 0xffu) {
+            case body_code(2, -1, 0): v = term_body<2, -1, 0>(a, cur, r, dl, sg); break;
+            case body_code(2, -1, 1): v = term_body<2, -1, 1>(a, cur, r, dl, sg); break;
+            case body_code(2, -1, 2): v = term_body<2, -1, 2>(a, cur, r, dl, sg); break;
+            case body_code(2, 0, 1): v = term_body<2, 0, 1>(a, cur, r, dl, sg); break;
+            case body_code(2, 0, 2): v = term_body<2, 0, 2>(a, cur, r, dl, sg); break;
             case body_code(4, -1, 0): v = term_body<4, -1, 0>(a, cur, r, dl, sg); break;
             case body_code(4, -1, 1): v = term_body<4, -1, 1>(a, cur, r, dl, sg); break;
             case body_code(4, -1, 2): v = term_body<4, -1, 2>(a, cur, r, dl, sg); break;
@@ -329,18 +400,9 @@ __device__ __forceinline__ void group_tile(GroupShared& g, const A* __restrict__
             case body_code(4, 0, 2): v = term_body<4, 0, 2>(a, cur, r, dl, sg); break;
             case body_code(4, 1, 1): v = term_body<4, 1, 1>(a, cur, r, dl, sg); break;
             case body_code(4, 1, 2): v = term_body<4, 1, 2>(a, cur, r, dl, sg); break;
-            case body_code(8, -1, 0): v = term_body<8, -1, 0>(a, cur, r, dl, sg); break;
-            case body_code(8, -1, 1): v = term_body<8, -1, 1>(a, cur, r, dl, sg); break;
-            case body_code(8, -1, 2): v = term_body<8, -1, 2>(a, cur, r, dl, sg); break;
-            case body_code(8, 0, 1): v = term_body<8, 0, 1>(a, cur, r, dl, sg); break;
-            case body_code(8, 0, 2): v = term_body<8, 0, 2>(a, cur, r, dl, sg); break;
-            case body_code(8, 1, 1): v = term_body<8, 1, 1>(a, cur, r, dl, sg); break;
-            case body_code(8, 1, 2): v = term_body<8, 1, 2>(a, cur, r, dl, sg); break;
-            case body_code(8, 2, 1): v = term_body<8, 2, 1>(a, cur, r, dl, sg); break;
-            case body_code(8, 2, 2): v = term_body<8, 2, 2>(a, cur, r, dl, sg); break;
             default: break;
         }
-        g.acc[t][r] = __dadd_rn(g.acc[t][r], v);
+        acc[t * kGroupThreads + r] = __dadd_rn(acc[t * kGroupThreads + r], v);
     }
 }
 
@@ -348,18 +410,24 @@ __device__ __forceinline__ void group_tile(GroupShared& g, const A* __restrict__
 // slot_of(t) as (re, im) of the pair sum before the i^popcount(x & z)
 // factor, with the term's visit weight; the accumulators are cleared.
 template <typename SLOT>
-__device__ __forceinline__ void group_write(GroupShared& g, const GroupTerm* __restrict__ terms, uint32_t nterms,
-                                            SLOT slot_of) {
-    for (uint32_t t = 0; t < nterms; ++t) {
-        double r = g.acc[t][threadIdx.x];
-        g.acc[t][threadIdx.x] = 0.0;
+__device__ __forceinline__ void group_write(GroupShared& g, double (&reg)[kRegularTerms], double* __restrict__ acc,
+                                            const GroupTerm* __restrict__ terms, uint32_t nterms, SLOT slot_of) {
+#pragma unroll
+    for (uint32_t p = 0; p < kRegularTerms; ++p) {
+        if (p < g.regular) acc[p * kGroupThreads + threadIdx.x] = reg[p];
+        reg[p] = 0.0;
+    }
+    for (uint32_t p = 0; p < nterms; ++p) {
+        const uint32_t t = g.place[p];
+        double r = acc[p * kGroupThreads + threadIdx.x];
+        acc[p * kGroupThreads + threadIdx.x] = 0.0;
         for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
         __syncthreads();
         if ((threadIdx.x & 31) == 0) g.red[threadIdx.x >> 5] = r;
         __syncthreads();
         if (threadIdx.x == 0) {
             double sum = 0.0;
-            for (int w = 0; w < kThreads / 32; ++w) sum += g.red[w];
+            for (int w = 0; w < kGroupThreads / 32; ++w) sum += g.red[w];
             double* p = slot_of(terms[t].out);
             const uint32_t mode = g.tmode[t];
             const double w = static_cast<double>(g.tweight[t]);
@@ -386,7 +454,7 @@ template <typename A>
 __device__ __forceinline__ void group_gather(const A* __restrict__ st, uint64_t rep, A* buf, const GroupShared& g,
                                              uint32_t c, uint32_t tile_amps) {
     const uint32_t lowmask = (1u << c) - 1;
-    for (uint32_t L = threadIdx.x; L < tile_amps; L += kThreads) {
+    for (uint32_t L = threadIdx.x; L < tile_amps; L += kGroupThreads) {
         const uint64_t m = ((rep ^ g.sspan[L >> c]) << c) | (L & lowmask);
         cp_async_amp(buf + L, st + m);
     }
@@ -396,16 +464,18 @@ __device__ __forceinline__ void group_gather(const A* __restrict__ st, uint64_t 
 // Cosets are processed with two shared-memory buffers: the next coset's
 // amplitudes are gathered with cp.async while this one is reduced.
 template <typename A>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kGroupThreads, 2)
     k_pauli_group(const A* __restrict__ st, uint32_t c, uint32_t d, const uint64_t* __restrict__ span,
                   uint64_t free_mask, const GroupTerm* __restrict__ terms, uint32_t nterms, uint64_t ncosets,
-                  double* __restrict__ partials) {
+                  uint32_t pitch, double* __restrict__ partials) {
     extern __shared__ __align__(16) unsigned char gsm[];
     __shared__ GroupShared g;
     const uint32_t tile_amps = 1u << (c + d);
     A* buf0 = reinterpret_cast<A*>(gsm);
     A* buf1 = buf0 + tile_amps;
-    const uint32_t sig = group_setup(g, c, d, span, terms, nterms);
+    double* acc = reinterpret_cast<double*>(buf1 + tile_amps);
+    const uint32_t sig = group_setup(g, acc, c, d, span, terms, nterms);
+    double reg[kRegularTerms] = {};
     // Moving gridDim.x cosets on is a masked add on the free bits.
     const uint64_t rstep = deposit_bits(gridDim.x, free_mask);
     auto advance = [&](uint64_t r) { return ((r | ~free_mask) + rstep) & free_mask; };
@@ -419,7 +489,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         else asm volatile("cp.async.commit_group;\n" ::: "memory");
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         __syncthreads();
-        group_tile(g, cur, rep, tile_amps, nterms, sig);
+        group_tile(g, reg, acc, cur, rep, tile_amps, nterms, sig);
         __syncthreads();  // this buffer is the target of the gather after next
         rep = rep_next;
         A* tmp = cur;
@@ -427,8 +497,8 @@ __global__ void __launch_bounds__(kThreads, 2)
         nxt = tmp;
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    group_write(g, terms, nterms, [&](uint32_t out) {
-        return partials + 2 * (static_cast<uint64_t>(out) * gridDim.x + blockIdx.x);
+    group_write(g, reg, acc, terms, nterms, [&](uint32_t out) {
+        return partials + 2 * (static_cast<uint64_t>(out) * pitch + blockIdx.x);
     });
 }
 
@@ -439,7 +509,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 // partials[2 * ((term * bindings + b) * per + s)], so a binding's value
 // depends only on its own state and on `per`.
 template <typename A>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kGroupThreads, 2)
     k_pauli_group_batch(const A* __restrict__ st, uint32_t n, uint32_t c, uint32_t d,
                         const uint64_t* __restrict__ span, uint64_t free_mask, const GroupTerm* __restrict__ terms,
                         uint32_t nterms, uint64_t bindings, uint32_t per, double* __restrict__ partials) {
@@ -448,7 +518,9 @@ __global__ void __launch_bounds__(kThreads, 2)
     const uint32_t tile_amps = 1u << (c + d);
     A* buf0 = reinterpret_cast<A*>(gsm);
     A* buf1 = buf0 + tile_amps;
-    const uint32_t sig = group_setup(g, c, d, span, terms, nterms);
+    double* acc = reinterpret_cast<double*>(buf1 + tile_amps);
+    const uint32_t sig = group_setup(g, acc, c, d, span, terms, nterms);
+    double reg[kRegularTerms] = {};
     const uint64_t ncosets = uint64_t{1} << (n - c - d);
     const uint32_t slot = blockIdx.x % per;
     const uint64_t b0 = blockIdx.x / per, bstep = gridDim.x / per;
@@ -458,7 +530,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     const uint64_t mine = ncosets > slot ? (ncosets - slot + per - 1) / per : 0;
     const uint64_t nb = (bindings - b0 + bstep - 1) / bstep;
     auto write = [&](uint64_t b) {
-        group_write(g, terms, nterms, [&](uint32_t out) {
+        group_write(g, reg, acc, terms, nterms, [&](uint32_t out) {
             return partials + 2 * ((static_cast<uint64_t>(out) * bindings + b) * per + slot);
         });
     };
@@ -486,7 +558,7 @@ __global__ void __launch_bounds__(kThreads, 2)
         }
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         __syncthreads();
-        group_tile(g, cur, rep, tile_amps, nterms, sig);
+        group_tile(g, reg, acc, cur, rep, tile_amps, nterms, sig);
         __syncthreads();  // this buffer is the target of the gather after next
         if ((f + 1) % mine == 0) write(b);
         b = bn;
@@ -522,17 +594,22 @@ __global__ void k_batch_group_finish(const double* __restrict__ partials, uint64
 
 }  // namespace
 
+// Dynamic shared memory of a group: two tile buffers and the accumulators.
+static size_t group_smem(uint32_t tile_qubits, uint32_t nterms, int precision) {
+    return 2 * (size_t{1} << tile_qubits) * (precision == MB2_C64 ? sizeof(float2) : sizeof(double2)) +
+           size_t{nterms} * kGroupThreads * sizeof(double);
+}
+
 int launch_pauli_group(const void* amps, uint32_t n, uint32_t c, uint32_t d, const uint64_t* dev_span,
                        uint64_t free_mask, const void* dev_terms, uint32_t nterms, double* dev_partials,
-                       uint32_t grid, void* stream, int precision) {
+                       uint32_t grid, uint32_t pitch, void* stream, int precision) {
     if (nterms == 0) return MB2_OK;
     if (nterms > kMaxGroupTerms || c + d > kPauliTileQubits || d > kPauliMaxSpan) return MB2_ERR_INVALID;
     const auto s = static_cast<cudaStream_t>(stream);
     const uint64_t ncosets = uint64_t{1} << (n - c - d);
-    // Two buffers of 2^(c+d) amplitudes; each thread takes two amplitudes (or
-    // two pairs) per step, so a tile holds at least 4 * kThreads of them.
-    if (c + d < kPauliMinTileQubits) return MB2_ERR_INVALID;
-    const size_t smem = 2 * (size_t{1} << (c + d)) * (precision == MB2_C64 ? sizeof(float2) : sizeof(double2));
+    // Two buffers of 2^(c+d) amplitudes, of which each thread owns two or four.
+    if (c + d < kPauliMinTileQubits || grid > pitch) return MB2_ERR_INVALID;
+    const size_t smem = group_smem(c + d, nterms, precision);
     static const bool attr = [] {  // once, thread-safe (concurrent callers wait for it)
         return cudaFuncSetAttribute(k_pauli_group<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     128 * 1024) == cudaSuccess &&
@@ -542,11 +619,11 @@ int launch_pauli_group(const void* amps, uint32_t n, uint32_t c, uint32_t d, con
     if (!attr) return launch_status();
     const auto* terms = static_cast<const GroupTerm*>(dev_terms);
     if (precision == MB2_C64)
-        k_pauli_group<float2><<<grid, kThreads, smem, s>>>(static_cast<const float2*>(amps), c, d, dev_span,
-                                                           free_mask, terms, nterms, ncosets, dev_partials);
+        k_pauli_group<float2><<<grid, kGroupThreads, smem, s>>>(static_cast<const float2*>(amps), c, d, dev_span,
+                                                           free_mask, terms, nterms, ncosets, pitch, dev_partials);
     else
-        k_pauli_group<double2><<<grid, kThreads, smem, s>>>(static_cast<const double2*>(amps), c, d, dev_span,
-                                                            free_mask, terms, nterms, ncosets, dev_partials);
+        k_pauli_group<double2><<<grid, kGroupThreads, smem, s>>>(static_cast<const double2*>(amps), c, d, dev_span,
+                                                            free_mask, terms, nterms, ncosets, pitch, dev_partials);
     note_launches(1);
     return launch_status();
 }
@@ -558,7 +635,7 @@ int launch_pauli_group_batch(const void* amps, uint32_t n, uint32_t c, uint32_t 
     if (nterms > kMaxGroupTerms || c + d > kPauliTileQubits || d > kPauliMaxSpan || c + d > n || per == 0 ||
         c + d < kPauliMinTileQubits)
         return MB2_ERR_INVALID;
-    const size_t smem = 2 * (size_t{1} << (c + d)) * (precision == MB2_C64 ? sizeof(float2) : sizeof(double2));
+    const size_t smem = group_smem(c + d, nterms, precision);
     static const bool attr = [] {  // once, thread-safe
         return cudaFuncSetAttribute(k_pauli_group_batch<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     128 * 1024) == cudaSuccess &&
@@ -573,10 +650,10 @@ int launch_pauli_group_batch(const void* amps, uint32_t n, uint32_t c, uint32_t 
     const auto s = static_cast<cudaStream_t>(stream);
     const auto* terms = static_cast<const GroupTerm*>(dev_terms);
     if (precision == MB2_C64)
-        k_pauli_group_batch<float2><<<grid, kThreads, smem, s>>>(static_cast<const float2*>(amps), n, c, d, dev_span,
+        k_pauli_group_batch<float2><<<grid, kGroupThreads, smem, s>>>(static_cast<const float2*>(amps), n, c, d, dev_span,
                                                                  free_mask, terms, nterms, bindings, per, dev_partials);
     else
-        k_pauli_group_batch<double2><<<grid, kThreads, smem, s>>>(static_cast<const double2*>(amps), n, c, d,
+        k_pauli_group_batch<double2><<<grid, kGroupThreads, smem, s>>>(static_cast<const double2*>(amps), n, c, d,
                                                                   dev_span, free_mask, terms, nterms, bindings, per,
                                                                   dev_partials);
     note_launches(1);

@@ -535,7 +535,9 @@ int probe_rates(int sm_count, double* fp64_per_s, double* copy_gbs);
 // Grouped Pauli terms (pauli_groups.cpp plans, kernels_reduce.cu reduces):
 // terms whose X masks above the low c bits span a subspace of dimension d
 // share one read of the state, in tiles of 2^(c+d) <= 2^12 amplitudes.
-// Partials are written at (term.out * grid + CTA).
+// Partials are written at (term.out * pitch + CTA).  kPauliGroupBlocks CTAs,
+// two for each of 148 SMs (512 left the second wave a quarter empty).
+constexpr uint32_t kPauliGroupBlocks = 296;
 constexpr uint32_t kMaxGroupTerms = 16;
 constexpr uint32_t kPauliTileQubits = 11;
 constexpr uint32_t kPauliMinTileQubits = 10;  // smaller states: one streaming pass per term
@@ -560,7 +562,7 @@ struct PauliPlan {
 PauliPlan plan_pauli_groups(const uint64_t* x, const uint64_t* z, uint32_t num_terms, uint32_t n);
 int launch_pauli_group(const void* amps, uint32_t n, uint32_t c, uint32_t d, const uint64_t* dev_span,
                        uint64_t free_mask, const void* dev_terms, uint32_t nterms, double* dev_partials,
-                       uint32_t grid, void* stream, int precision);
+                       uint32_t grid, uint32_t pitch, void* stream, int precision);
 // One streaming pass per term (partials only), for terms that share no read.
 int launch_expectation_partials(const void* amps, uint32_t n, const uint64_t* dev_x, const uint64_t* dev_z,
                                 uint32_t num_terms, double* dev_partials, void* stream, int precision);

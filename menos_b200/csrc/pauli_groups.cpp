@@ -19,8 +19,7 @@ namespace mb2 {
 namespace {
 
 // GF(2) basis in reduced echelon form: vec[i] has bit piv[i] set and no other
-// basis vector has that bit, so a vector of the span has coordinate i equal
-// to its bit piv[i].
+// basis vector has that bit.
 struct Gf2Basis {
     std::vector<uint64_t> vec;
     std::vector<uint32_t> piv;
@@ -39,11 +38,34 @@ struct Gf2Basis {
         piv.push_back(p);
         return true;
     }
-    uint32_t coords(uint64_t v) const {
+};
+
+// A basis of the span that takes each vector that enlarges it as it is, and
+// a vector's coordinates in it: echelon rows with the combination of basis
+// vectors that each one is.
+struct RawBasis {
+    std::vector<uint64_t> vec, row;
+    std::vector<uint32_t> combo, piv;
+    // Reduces v; the coordinates of what was taken away.
+    uint32_t reduce(uint64_t& v) const {
         uint32_t k = 0;
-        for (size_t i = 0; i < vec.size(); ++i) k |= static_cast<uint32_t>((v >> piv[i]) & 1u) << i;
+        for (size_t i = 0; i < row.size(); ++i)
+            if ((v >> piv[i]) & 1u) {
+                v ^= row[i];
+                k ^= combo[i];
+            }
         return k;
     }
+    void add(uint64_t v) {
+        uint64_t r = v;
+        const uint32_t k = reduce(r);
+        if (r == 0) return;
+        piv.push_back(63u - static_cast<uint32_t>(__builtin_clzll(r)));
+        row.push_back(r);
+        combo.push_back(k ^ (1u << vec.size()));
+        vec.push_back(v);
+    }
+    uint32_t coords(uint64_t v) const { return reduce(v); }
 };
 
 uint32_t rank_above(const std::vector<uint64_t>& xs, uint32_t c) {
@@ -101,11 +123,26 @@ PauliPlan plan_pauli_groups(const uint64_t* x, const uint64_t* z, uint32_t num_t
         const uint64_t high = (n - c >= 64) ? ~uint64_t{0} : ((uint64_t{1} << (n - c)) - 1);
         gp.free_mask = high & ~pivots;
         gp.span_off = static_cast<uint32_t>(plan.spans.size());
-        for (uint32_t k = 0; k < (1u << gp.d); ++k) {
+        // The tile's chunk coordinates: those of the members' own X masks as a
+        // basis, the highest replaced by the sum of all.  Every member that
+        // enlarged the span then has the highest bit set, and so has any sum of
+        // an odd number of them: the pairs of such a term differ in the
+        // highest bit of the tile index, which the kernel keeps in a thread's
+        // registers, so each thread visits its amplitudes with that bit clear.
+        RawBasis raw;
+        for (uint64_t v : xs) raw.add(v >> c);
+        const uint32_t top = gp.d == 0 ? 0u : 1u << (gp.d - 1);
+        auto chunk_coords = [&](uint64_t v) {
+            const uint32_t k = raw.coords(v);
+            return (k & ~top) | ((__builtin_popcount(k) & 1) ? top : 0u);
+        };
+        const size_t s0 = plan.spans.size();
+        plan.spans.resize(s0 + (size_t{1} << gp.d), 0);
+        for (uint32_t k = 0; k < (1u << gp.d); ++k) {  // raw coordinates
             uint64_t v = 0;
             for (uint32_t i = 0; i < gp.d; ++i)
-                if ((k >> i) & 1u) v ^= b.vec[i];
-            plan.spans.push_back(v);
+                if ((k >> i) & 1u) v ^= raw.vec[i];
+            plan.spans[s0 + ((k & ~top) | ((__builtin_popcount(k) & 1) ? top : 0u))] = v;
         }
         gp.term_off = static_cast<uint32_t>(plan.terms.size());
         gp.nterms = static_cast<uint32_t>(g.members.size());
@@ -113,7 +150,7 @@ PauliPlan plan_pauli_groups(const uint64_t* x, const uint64_t* z, uint32_t num_t
             PauliGroupTerm pt{};
             pt.x = x[t];
             pt.z = z[t];
-            pt.kx = b.coords(x[t] >> c);
+            pt.kx = chunk_coords(x[t] >> c);
             pt.xl = static_cast<uint32_t>(x[t] & ((uint64_t{1} << c) - 1));
             pt.out = t;
             plan.terms.push_back(pt);
