@@ -97,7 +97,10 @@ enum TileKind : uint8_t {
     TK_X = 5,      // 1q exact swap of the pair (X)
     TK_SW12 = 6,   // 2q exact exchange of local indices 1 and 2 (SWAP)
     TK_SW13 = 7,   // 2q exact exchange of local indices 1 and 3 (CX, control = operand 0)
-    TK_SW23 = 8    // 2q exact exchange of local indices 2 and 3 (CX, control = operand 1)
+    TK_SW23 = 8,   // 2q exact exchange of local indices 2 and 3 (CX, control = operand 1)
+    // 2q, real, pairing local indices (0,3) and (1,2) only: data is m00 m03 m30
+    // m33 m11 m12 m21 m22, slots pos[0] < pos[1]
+    TK_CROSS = 9
 };
 struct TileInstr {
     uint8_t op;
@@ -196,7 +199,8 @@ constexpr uint32_t kReal1 = 9;   // + slot
 // 13-20 are unused (one-qubit monomials and X are written as kGen1/kReal1).
 constexpr uint32_t kGen2 = 21;   // + pair
 constexpr uint32_t kMono2 = 33;  // + pair; extra word = source rows (3 bits each)
-// 45-80 are unused (exact permutations are TileMap's, not instructions).
+constexpr uint32_t kCross = 45;  // + unordered pair (0,1) (0,2) (0,3) (1,2) (1,3) (2,3)
+// 51-80 are unused (exact permutations are TileMap's, not instructions).
 constexpr uint32_t kDs1R = 81;   // + slot; aux = entry classes
 // An operand position (0-31) in a header word: bits 16-19 and bit 31 (the
 // staged data offset, bits 20-30, stays below 2048 16-byte units).

@@ -323,6 +323,11 @@ void encode_compact(TileProgram& prog) {
                     break;
                 }
                 case TOP_G2: {
+                    if (g.kind == TK_CROSS) {
+                        static constexpr uint32_t kPair[4][4] = {{9, 0, 1, 2}, {9, 9, 3, 4}, {9, 9, 9, 5}, {9, 9, 9, 9}};
+                        w.push_back(header(cop::kCross + kPair[g.pos[0]][g.pos[1]], 0, 0, off));
+                        break;
+                    }
                     heavy = true;  // monomials move registers: full variant
                     const uint32_t pr = pair_index(g.pos[0], g.pos[1]);
                     if (g.kind != TK_GEN) heavy_other = true;

@@ -126,6 +126,20 @@ bool split_block(const Block& b, Block& first, Block& second) {
     return false;
 }
 
+// A real two-qubit block whose entries lie on the two diagonals: it pairs
+// local index 0 with 3 and 1 with 2.  The superoperators of the common
+// channels (depolarizing, damping, flips) on a qubit's row and column bits
+// are such blocks.
+bool is_cross(const Block& b) {
+    if (b.k != 2) return false;
+    for (uint32_t r = 0; r < 4; ++r)
+        for (uint32_t c = 0; c < 4; ++c) {
+            const Cd& v = b.m[4 * r + c];
+            if (!is_real(v) || (!is_zero(v) && c != r && c != 3 - r)) return false;
+        }
+    return true;
+}
+
 struct PassSel {
     uint64_t smask;
     uint64_t gmask = 0;           // qubits outside the tile that diagonals of the pass read
@@ -793,6 +807,18 @@ TileProgram plan_tile_program(const std::vector<Block>& all, uint32_t n, uint32_
                         g.kind = TK_GEN;
                         prog.fp64_per_amp += 14;
                     }
+                } else if (!commuting && (pf & kParamBlock) == 0 && is_cross(b)) {
+                    // 6 FP64 operations per amplitude instead of 30.  Slots in
+                    // ascending order: swapped operands exchange indices 1 and 2.
+                    g.kind = TK_CROSS;
+                    const uint32_t one = g.pos[0] < g.pos[1] ? 1 : 2, two = 3 - one;
+                    if (g.pos[0] > g.pos[1]) std::swap(g.pos[0], g.pos[1]);
+                    auto e = [&](uint32_t r, uint32_t c) { return b.m[4 * r + c].real(); };
+                    g.data = push_staged({Cd(e(0, 0), e(0, 3)), Cd(e(3, 0), e(3, 3)), Cd(e(one, one), e(one, two)),
+                                          Cd(e(two, one), e(two, two))});
+                    prog.fp64_per_amp += 6;
+                    prog.instrs.push_back(g);
+                    continue;
                 } else {
                     g.kind = TK_GEN;
                     prog.fp64_per_amp += 30;

@@ -478,7 +478,15 @@ void run_program_on_host(const TileProgram& prog, uint32_t n, Cd* state) {
                 case TOP_G1:
                 case TOP_G2: {
                     for (uint32_t t = 0; t < g.k; ++t) ops[t] = qubit[reg[g.pos[t]]];
-                    host_apply_generic(state, amps, reinterpret_cast<const Cd*>(sdata + g.data), ops, g.k);
+                    const double* const e = sdata + g.data;
+                    if (g.op == TOP_G2 && g.kind == TK_CROSS) {
+                        std::vector<Cd> m(16, Cd(0.0, 0.0));
+                        m[0] = e[0], m[3] = e[1], m[12] = e[2], m[15] = e[3];
+                        m[5] = e[4], m[6] = e[5], m[9] = e[6], m[10] = e[7];
+                        host_apply_generic(state, amps, m.data(), ops, g.k);
+                        break;
+                    }
+                    host_apply_generic(state, amps, reinterpret_cast<const Cd*>(e), ops, g.k);
                     break;
                 }
                 case TOP_DIAG: {

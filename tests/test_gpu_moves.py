@@ -101,3 +101,29 @@ def test_batched_bindings(ctx, oracle, n):
             b.ops[i] = (oc, qs, tuple(float(v) for v in row[k:k + s]) if s else ps, m, *rest)
             k += s
         assert bits_equal(got, oracle.run(b, fuse_gates=False))
+
+
+@pytest.mark.parametrize("n,tile", [(4, 4), (9, 6), (12, 12), (13, 11)])
+def test_real_blocks_on_the_two_diagonals(ctx, oracle, n, tile):
+    # Channel superoperators' shape on every ordered operand pair, zeros and signs among the entries.
+    rng = np.random.default_rng(n)
+    a, b = Circuit(n), pyoracle.Circuit(n)
+    for q in range(n):
+        for c in (a, b):
+            c.gate("u", [q], [0.3 + q, 1.1, 0.2])
+    for q in range(n):
+        for r in range(n):
+            if q == r:
+                continue
+            m = np.zeros((4, 4))
+            v = rng.normal(size=(4, 2)) * 0.7
+            for i in range(4):
+                m[i, i], m[i, 3 - i] = v[i]
+            if (q + r) % 3 == 0:
+                m[1, 2] = m[2, 1] = 0.0
+            for c in (a, b):
+                c.unitary([q, r], m)
+    st = DeviceState(ctx, n)
+    st.init(0.0)
+    st.apply_program(a, fuse_gates=False, tile_qubits=tile)
+    assert bits_equal(st.copy_out(), oracle.run(b, fuse_gates=False))
