@@ -14,6 +14,7 @@
 
 #include "c64_ops.cuh"
 #include "device_math.cuh"
+#include "launch_next.cuh"
 #include "mb2_internal.h"
 
 namespace mb2 {
@@ -86,6 +87,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
                     const double* __restrict__ pdata, uint32_t pstride, uint32_t param_lo, uint32_t param_len,
                     uint32_t bshift, uint32_t store_rec, uint32_t stages) {
     extern __shared__ float2 smem_f[];
+    allow_next();
     const uint32_t m = MT > 0 ? static_cast<uint32_t>(MT) : m_rt;
     const uint32_t tid = threadIdx.x;
     const uint32_t tbits = m - kRegQubits;
@@ -130,6 +132,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
         for (int j = 0; j < kNA; ++j) cp_async8(buf + slot(j), st + (b0 + reg_off(j)));
         cp_async_commit();
     };
+    await_previous();
     uint64_t tp = blockIdx.x;
     IDX pbase = static_cast<IDX>(pdep64(blockIdx.x, nmask64));
     IDX cbase = pbase;
@@ -376,7 +379,8 @@ int launch_c64_instance(const TileLaunch& L) {
     }();
     if (dyn_max == 0) return launch_status();
     if (L.smem > dyn_max) return MB2_ERR_INVALID;
-    k_tile_pass_c64<MAXT, MINB, MT, IDX, V><<<L.grid, L.threads, L.smem, static_cast<cudaStream_t>(L.stream)>>>(
+    launch_behind(
+        k_tile_pass_c64<MAXT, MINB, MT, IDX, V>, L.grid, L.threads, L.smem, static_cast<cudaStream_t>(L.stream),
         static_cast<float2*>(L.amps), L.n_all, L.m, L.smask, L.words, L.nwords, L.sdata, L.nsdata, L.gdata, L.ntiles,
         L.pdata, L.pstride, L.param_lo, L.param_len, L.bshift, L.store_rec, L.stages);
     return launch_status();

@@ -12,6 +12,7 @@
 #include <cstdint>
 
 #include "device_math.cuh"
+#include "launch_next.cuh"
 #include "mb2_internal.h"
 
 namespace mb2 {
@@ -461,6 +462,7 @@ __device__ __forceinline__ void tile_pass_body(double2* __restrict__ st, uint32_
                                                uint32_t param_len, uint32_t bshift, uint32_t store_rec,
                                                uint32_t stages, uint32_t cta, uint32_t nctas) {
     extern __shared__ double2 smem_tiles[];
+    allow_next();
     const uint32_t m = MT > 0 ? static_cast<uint32_t>(MT) : m_rt;
     const uint32_t tid = threadIdx.x;
     const uint32_t tbits = m - kRegQubits;
@@ -512,6 +514,7 @@ __device__ __forceinline__ void tile_pass_body(double2* __restrict__ st, uint32_
         cp_async_commit();
     };
 
+    await_previous();
     // `stages` tile buffers: the tiles `stages - 1` ahead are in flight
     // while this one is computed (one commit group per tile, empty groups
     // past the end keep the count uniform).
@@ -624,7 +627,8 @@ int launch_instance(const TileLaunch& L) {
     }();
     if (dyn_max == 0) return launch_status();
     if (L.smem > dyn_max) return MB2_ERR_INVALID;
-    k_tile_pass<MAXT, MINB, MT, IDX, FULL><<<L.grid, L.threads, L.smem, static_cast<cudaStream_t>(L.stream)>>>(
+    launch_behind(
+        k_tile_pass<MAXT, MINB, MT, IDX, FULL>, L.grid, L.threads, L.smem, static_cast<cudaStream_t>(L.stream),
         static_cast<double2*>(L.amps), L.n_all, L.m, L.smask, L.gmask, L.words, L.nwords, L.sdata, L.nsdata, L.gdata,
         L.ntiles, L.pdata, L.pstride, L.param_lo, L.param_len, L.bshift, L.store_rec, L.stages);
     return launch_status();
