@@ -173,6 +173,10 @@ def dist_barrier(dist):
 # ----------------------------------------------------------------------------
 # CPU leg: the reference's own CPU kernels (oracle/_ref), bounded sample.
 # ----------------------------------------------------------------------------
+def reference_built():
+    return os.path.exists(os.path.join(ROOT, "oracle", "_ref", "libmenos_ref.so"))
+
+
 def cpu_reference_sample(n, circ, paulis, shots, seed):
     """Times the reference CPU engine's kernels on the job at n qubits over a
     bounded sample -- the first brick layer's gates (each gate of the job is
@@ -362,7 +366,7 @@ def main():
         "gpu_launches": launches,
         "clocks": clk,
     }
-    if rank == 0 and world == 1 and not args.no_cpu_baseline:
+    if rank == 0 and world == 1 and not args.no_cpu_baseline and reference_built():
         v, detail, cores, sampled = cpu_reference_sample(n, circ, paulis, args.shots, 1234)
         line["cpu_baseline"] = {"value": round(v, 6), "unit": UNIT, "cores": cores, "kind": "reference",
                                 "sample": f"reference CPU kernels (oracle/_ref) at {n} qubits: {sampled} gates "
