@@ -138,24 +138,20 @@ __device__ __forceinline__ PMap shfl_up(const PMap& m, uint32_t o) {
 // (Two FP64 adds and integer work: ldexp, floor and a conversion for each
 // element were what bounded steps C and E.)
 constexpr double kTwo52 = 4503599627370496.0;
-__device__ __forceinline__ long long element_inc(double p, double scale, double& d) {
+__device__ __forceinline__ PMap element_map(double p, double scale) {
     double q = __dmul_rn(p, scale);
     q = q < kTwo52 ? q : kTwo52;
     const double t = __dadd_rn(q, kTwo52);
-    d = __dsub_rn(q, __dsub_rn(t, kTwo52));  // +-0.5: a tie
-    return __double_as_longlong(t) - __double_as_longlong(kTwo52);
-}
-__device__ __forceinline__ PMap element_map(double p, double scale) {
-    double d;
-    const long long r = element_inc(p, scale, d);
+    const double d = __dsub_rn(q, __dsub_rn(t, kTwo52));
+    const long long r = __double_as_longlong(t) - __double_as_longlong(kTwo52);
     return PMap{r, fabs(d) == 0.5 ? (d > 0.0 ? r + 1 : r - 1) : r};
 }
 
-// The binade of a normal c, and 2^e for a normal power.
 __device__ __forceinline__ int binade_of(double c) {
-    return static_cast<int>((__double_as_longlong(c) >> 52) & 0x7ff) - 1023;
+    int e;
+    frexp(c, &e);  // c = f * 2^e, f in [0.5, 1): binade 2^(e-1)
+    return e - 1;
 }
-__device__ __forceinline__ double pow2(int e) { return __longlong_as_double(static_cast<long long>(e + 1023) << 52); }
 
 // Binades the maps are used in: u and 1 / u are normal numbers there.
 constexpr int kMinBinade = -900, kMaxBinade = 900;
@@ -220,37 +216,16 @@ __global__ void __launch_bounds__(kThreads) k_chunk_maps(const A* __restrict__ s
     // the approximate scan's error.
     const double slack = (static_cast<double>(base + chunk) + 1.0e6) * 2.3e-16;
     const int e = a > 0.0 ? binade_of(a) : -2000;
-    const bool ok = a > 0.0 && e > kMinBinade && e < kMaxBinade && a * (1.0 - slack) > pow2(e) &&
-                    hi * (1.0 + slack) < pow2(e + 1);
+    const double lo_edge = ldexp(1.0, e), hi_edge = ldexp(1.0, e + 1);
+    const bool ok = a > 0.0 && e > kMinBinade && e < kMaxBinade && a * (1.0 - slack) > lo_edge &&
+                    hi * (1.0 + slack) < hi_edge;
     if (!ok) {  // (uniform over the CTA)
         if (threadIdx.x == 0) maps[j] = ChunkMap{0, 0, e, 0};
         return;
     }
     stage_chunk(st, base, chunk, sh);
     // Each thread composes its contiguous run of 16 elements in order.
-    // Ties are rare: without one in the chunk its map adds the same to an even
-    // and an odd M, and the increments add up in any order.
-    const double scale = pow2(52 - e);
-    long long sum = 0;
-    bool tie = false;
-#pragma unroll
-    for (int i = 0; i < kPerThread; ++i) {
-        double d;
-        sum += element_inc(sh[pad(threadIdx.x * kPerThread + i)], scale, d);
-        tie = tie || fabs(d) == 0.5;
-    }
-    __shared__ PMap wm[kThreads / 32];
-    if (!__syncthreads_or(tie)) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
-        if (lane == 0) wm[warp].inc0 = sum;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int w = 1; w < kThreads / 32; ++w) sum += wm[w].inc0;
-            maps[j] = ChunkMap{sum, sum, e, 1};
-        }
-        return;
-    }
+    const double scale = ldexp(1.0, 52 - e);
     PMap acc{0, 0};
 #pragma unroll
     for (int i = 0; i < kPerThread; ++i) acc = compose(acc, element_map(sh[pad(threadIdx.x * kPerThread + i)], scale));
@@ -260,6 +235,7 @@ __global__ void __launch_bounds__(kThreads) k_chunk_maps(const A* __restrict__ s
         const PMap other{__shfl_down_sync(0xffffffffu, acc.inc0, o), __shfl_down_sync(0xffffffffu, acc.inc1, o)};
         if ((lane & (2 * o - 1)) == 0) acc = compose(acc, other);
     }
+    __shared__ PMap wm[kThreads / 32];
     if (lane == 0) wm[warp] = acc;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -339,61 +315,34 @@ __device__ double chain_chunk(double* sh, double c) {
             if (walked == kThreads) return c;
         } else {
             const int e = binade_of(c);
-            const double u = pow2(e - 52), scale = pow2(52 - e);
+            const double u = ldexp(1.0, e - 52), scale = ldexp(1.0, 52 - e);
             const long long m0 = static_cast<long long>(__dmul_rn(c, scale));  // exact: c is on the grid
-            long long m, m_end;  // M before and after this thread's run
-            long long sum = 0;
-            bool tie = false;
+            PMap inc{0, 0};
             if (tid >= pos) {
 #pragma unroll
-                for (int i = 0; i < kPerThread; ++i) {
-                    double d;
-                    sum += element_inc(sh[pad(tid * kPerThread + i)], scale, d);
-                    tie = tie || fabs(d) == 0.5;
-                }
+                for (int i = 0; i < kPerThread; ++i)
+                    inc = compose(inc, element_map(sh[pad(tid * kPerThread + i)], scale));
             }
-            if (!__syncthreads_or(tie)) {
-                // No tie: one increment per run, whatever M's parity.
-                const long long own = sum;
 #pragma unroll
-                for (uint32_t o = 1; o < 32; o <<= 1) {
-                    const long long prev = __shfl_up_sync(0xffffffffu, sum, o);
-                    if (lane >= o) sum += prev;
-                }
-                if (lane == 31) warp_map[warp].inc0 = min(sum, kSaturated);
-                __syncthreads();
-                long long before = m0;
-#pragma unroll
-                for (uint32_t w = 0; w < kThreads / 32; ++w) before += w < warp ? warp_map[w].inc0 : 0;
-                m_end = before + min(sum, kSaturated);
-                m = before + (sum - own);
-            } else {
-                PMap inc{0, 0};
-                if (tid >= pos) {
-#pragma unroll
-                    for (int i = 0; i < kPerThread; ++i)
-                        inc = compose(inc, element_map(sh[pad(tid * kPerThread + i)], scale));
-                }
-#pragma unroll
-                for (uint32_t o = 1; o < 32; o <<= 1) {
-                    const PMap prev = shfl_up(inc, o);
-                    if (lane >= o) inc = compose(prev, inc);
-                }
-                inc.inc0 = min(inc.inc0, kSaturated);
-                inc.inc1 = min(inc.inc1, kSaturated);
-                if (lane == 31) warp_map[warp] = inc;
-                __syncthreads();
-                PMap before{0, 0};
-                for (uint32_t w = 0; w < warp; ++w) before = compose(before, warp_map[w]);
-                PMap ex = shfl_up(inc, 1);
-                if (lane == 0) ex = PMap{0, 0};
-                ex = compose(before, ex);
-                inc = compose(before, inc);
-                m_end = m0 + ((m0 & 1) ? inc.inc1 : inc.inc0);
-                m = m0 + ((m0 & 1) ? ex.inc1 : ex.inc0);
+            for (uint32_t o = 1; o < 32; o <<= 1) {
+                const PMap prev = shfl_up(inc, o);
+                if (lane >= o) inc = compose(prev, inc);
             }
+            inc.inc0 = min(inc.inc0, kSaturated);
+            inc.inc1 = min(inc.inc1, kSaturated);
+            if (lane == 31) warp_map[warp] = inc;
+            __syncthreads();
+            PMap before{0, 0};
+            for (uint32_t w = 0; w < warp; ++w) before = compose(before, warp_map[w]);
+            PMap ex = shfl_up(inc, 1);
+            if (lane == 0) ex = PMap{0, 0};
+            ex = compose(before, ex);
+            inc = compose(before, inc);
+            const bool odd = m0 & 1;
+            const long long m_end = m0 + (odd ? inc.inc1 : inc.inc0);
             // The sums never fall, so the runs past the binade's end are the last ones.
             walked = kThreads - __syncthreads_count(tid >= pos && m_end >= (1LL << 53));
+            long long m = m0 + (odd ? ex.inc1 : ex.inc0);
             if (tid == walked) c_run = static_cast<double>(m) * u;  // exact: m < 2^53
             if (STORE && tid >= pos && tid < walked) {
 #pragma unroll
@@ -524,8 +473,8 @@ __global__ void __launch_bounds__(kSegThreads) k_seg_scan(const ChunkMap* __rest
 }
 
 __device__ __forceinline__ bool advance_exact(double& c, int e, const PMap& m) {
-    if (!(c > 0.0) || binade_of(c) != e) return false;  // (e is a normal number's)
-    const double u = pow2(e - 52);
+    if (!(c > 0.0) || binade_of(c) != e) return false;
+    const double u = ldexp(1.0, e - 52);
     const long long M = static_cast<long long>(c / u);  // exact: c is on the grid
     const long long M2 = M + ((M & 1) ? m.inc1 : m.inc0);
     if (M2 >= (1LL << 53)) return false;
@@ -614,7 +563,7 @@ __global__ void __launch_bounds__(kThreads) k_shot_bounds(uint64_t nchunks, cons
     } else {
         const SMap x = excl[j];
         const double c0 = seg_c[j - x.count];
-        const double g = pow2(maps[j].e - 52);
+        const double g = ldexp(1.0, maps[j].e - 52);
         const long long M = static_cast<long long>(c0 / g);
         c = static_cast<double>(M + ((M & 1) ? x.map.inc1 : x.map.inc0)) * g;
         cstart[j] = c;
