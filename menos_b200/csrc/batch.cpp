@@ -14,6 +14,8 @@
 
 #include <algorithm>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <stdexcept>
 #include <string>
 #include <thread>
@@ -60,10 +62,24 @@ struct Runner {
     cudaStream_t stream = nullptr;
     void* state = nullptr;
     void* work = nullptr;
+    // Memory from the device's stream-ordered pool, as the states' (a
+    // cudaMalloc and cudaFree of a batch's states cost milliseconds a call).
+    // Up to kMostPooled apiece: the pool keeps what it is given back.
+    static constexpr size_t kMostPooled = size_t{1} << 30;
+    bool state_pooled = false, work_pooled = false;
+    cudaError_t take(void** p, size_t bytes, bool& pooled) {
+        pooled = bytes <= kMostPooled;
+        return pooled ? cudaMallocAsync(p, bytes, stream) : cudaMalloc(p, bytes);
+    }
+    void give(void* p, bool pooled) {
+        if (p && pooled) cudaFreeAsync(p, stream);
+        else if (p) cudaFree(p);
+    }
     ~Runner() {
         if (stream) cudaStreamSynchronize(stream);
-        if (state) cudaFree(state);
-        if (work) cudaFree(work);
+        give(state, state_pooled);
+        give(work, work_pooled);
+        if (stream) cudaStreamSynchronize(stream);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -121,6 +137,13 @@ extern "C" int mb2_sweep_batch(mb2_context* ctx, const mb2_op* ops, uint32_t num
     // Unfused: block i is gate op i; only gates with parameters can differ,
     // and their matrices are built per binding from the gate table.
     std::vector<uint32_t> gate_op, gate_pofs;
+    // Their matrices, kept from the look at what differs for the records:
+    // block i's of binding b at b * matrices_per + matrix_at[i].
+    // (Not a vector: megabytes that the workers write before anyone reads them,
+    // zeroed by nobody.)
+    std::unique_ptr<double[]> matrices;
+    std::vector<size_t> matrix_at;
+    size_t matrices_per = 0;
     try {
         shape = binding_blocks(ops, num_ops, params, fuse);
     } catch (const std::exception&) {
@@ -137,6 +160,13 @@ extern "C" int mb2_sweep_batch(mb2_context* ctx, const mb2_op* ops, uint32_t num
             if (ops[i].opcode != MB2_UNITARY) k += static_cast<uint32_t>(mb2::gate_num_params(ops[i].opcode));
         }
         if (gate_op.size() != nb) return MB2_ERR_INVALID;
+        for (size_t i = 0; i < nb; ++i) {
+            const mb2_op& o = ops[gate_op[i]];
+            matrix_at.push_back(matrices_per);
+            if (o.opcode != MB2_UNITARY && mb2::gate_num_params(o.opcode) != 0) matrices_per += shape[i].m.size();
+        }
+        matrices.reset(new (std::nothrow) double[2 * matrices_per * num_bindings]);
+        if (!matrices) return MB2_ERR_RESOURCE;
         // Per worker: differs / all_real / m00_real / all_diag per block.
         std::vector<std::vector<uint8_t>> acc(nt, std::vector<uint8_t>(4 * nb, 0));
         const bool ok = parallel([&](unsigned w) {
@@ -152,6 +182,7 @@ extern "C" int mb2_sweep_batch(mb2_context* ctx, const mb2_op* ops, uint32_t num
                     if (mb2::gate_matrix(o.opcode, pb + gate_pofs[i], m) == 0)
                         throw std::invalid_argument("gate matrix");
                     const uint32_t dim = 1u << shape[i].k;
+                    std::memcpy(matrices.get() + 2 * (b * matrices_per + matrix_at[i]), m.data(), m.size() * sizeof(mb2::Cd));
                     if (std::memcmp(m.data(), shape[i].m.data(), m.size() * sizeof(mb2::Cd)) != 0) f[4 * i] = 1;
                     for (const mb2::Cd& c : m) f[4 * i + 1] &= c.imag() == 0.0 ? 1 : 0;
                     f[4 * i + 2] &= m[0].imag() == 0.0 ? 1 : 0;
@@ -222,32 +253,28 @@ extern "C" int mb2_sweep_batch(mb2_context* ctx, const mb2_op* ops, uint32_t num
     }
     // Per-binding records of the parametric blocks, in the kernel's layout.
     const size_t stride = prog.param_stride;
-    std::vector<double> pdata(std::max<size_t>(1, stride * num_bindings), 0.0);
-    auto write_record = [&](uint32_t b, size_t i, const std::vector<mb2::Cd>& m, uint32_t k) {
+    const size_t records = std::max<size_t>(1, stride * num_bindings);
+    const std::unique_ptr<double[]> pdata(new (std::nothrow) double[records]);
+    if (!pdata) return MB2_ERR_RESOURCE;
+    if (stride == 0) pdata[0] = 0.0;
+    auto write_record = [&](uint32_t b, size_t i, const mb2::Cd* m, uint32_t k) {
         const uint32_t dim = 1u << k;
-        double* dst = pdata.data() + size_t{b} * stride + prog.param_offsets[i];
+        double* dst = pdata.get() + size_t{b} * stride + prog.param_offsets[i];
         if (shape[i].diagonal) {
             for (uint32_t e = 0; e < dim; ++e) {
                 dst[2 * e] = m[size_t{e} * dim + e].real();
                 dst[2 * e + 1] = m[size_t{e} * dim + e].imag();
             }
         } else {
-            std::memcpy(dst, m.data(), size_t{dim} * dim * sizeof(mb2::Cd));
+            std::memcpy(dst, m, size_t{dim} * dim * sizeof(mb2::Cd));
         }
     };
     const bool filled = parallel([&](unsigned w) {
-        std::vector<mb2::Cd> m;
         for (uint32_t b = w; b < num_bindings; b += nt)
             for (size_t i = 0; i < nb; ++i) {
                 if (!(flags[i] & mb2::kParamBlock)) continue;
-                if (fuse) {
-                    write_record(b, i, per[b][i].m, per[b][i].k);
-                } else {
-                    const mb2_op& o = ops[gate_op[i]];
-                    if (mb2::gate_matrix(o.opcode, params + size_t{b} * params_per_binding + gate_pofs[i], m) == 0)
-                        throw std::invalid_argument("gate matrix");
-                    write_record(b, i, m, shape[i].k);
-                }
+                if (fuse) write_record(b, i, per[b][i].m.data(), per[b][i].k);
+                else write_record(b, i, reinterpret_cast<const mb2::Cd*>(matrices.get()) + b * matrices_per + matrix_at[i], shape[i].k);
             }
     });
     if (!filled) return MB2_ERR_INVALID;
@@ -262,7 +289,7 @@ extern "C" int mb2_sweep_batch(mb2_context* ctx, const mb2_op* ops, uint32_t num
     const size_t state_bytes = (size_t{num_bindings} << num_qubits) * (c64 ? 8 : sizeof(mb2::Cd));
     auto al = [](size_t v) { return (v + 255) & ~size_t{255}; };
     const size_t ib = prog.words.size() * sizeof(uint32_t), sb = prog.data.size() * 8,
-                 gb = prog.gdata.size() * 8, pb = pdata.size() * 8, tb = size_t{num_terms} * 8;
+                 gb = prog.gdata.size() * 8, pb = records * 8, tb = size_t{num_terms} * 8;
     // <H> per binding: with at least kPauliTileQubits qubits, the grouped
     // reduction (terms sharing a GF(2) span read each state once, `per`
     // CTAs per binding); smaller states: one 8-CTA cluster per binding.
@@ -280,7 +307,8 @@ extern "C" int mb2_sweep_batch(mb2_context* ctx, const mb2_op* ops, uint32_t num
     const size_t o_s = al(ib), o_g = o_s + al(sb), o_p = o_g + al(gb), o_x = o_p + al(pb), o_z = o_x + al(tb),
                  o_c = o_z + al(tb), o_sp = o_c + al(tb), o_tr = o_sp + al(spb), o_o = o_tr + al(trb),
                  o_pr = o_o + al(size_t{num_bindings} * 8), total = o_pr + al(prb);
-    if (cudaMalloc(&r.state, state_bytes) != cudaSuccess || cudaMalloc(&r.work, total) != cudaSuccess) {
+    if (r.take(&r.state, state_bytes, r.state_pooled) != cudaSuccess ||
+        r.take(&r.work, total, r.work_pooled) != cudaSuccess) {
         cudaGetLastError();
         return MB2_ERR_RESOURCE;
     }
@@ -289,7 +317,6 @@ extern "C" int mb2_sweep_batch(mb2_context* ctx, const mb2_op* ops, uint32_t num
     std::memcpy(host.data(), prog.words.data(), ib);
     if (sb) std::memcpy(host.data() + o_s, prog.data.data(), sb);
     if (gb) std::memcpy(host.data() + o_g, prog.gdata.data(), gb);
-    std::memcpy(host.data() + o_p, pdata.data(), pb);
     if (tb) {
         std::memcpy(host.data() + o_x, x_masks, tb);
         std::memcpy(host.data() + o_z, z_masks, tb);
@@ -297,7 +324,11 @@ extern "C" int mb2_sweep_batch(mb2_context* ctx, const mb2_op* ops, uint32_t num
     }
     if (spb) std::memcpy(host.data() + o_sp, pplan.spans.data(), spb);
     if (trb) std::memcpy(host.data() + o_tr, pplan.terms.data(), trb);
-    if (cudaMemcpyAsync(w, host.data(), host.size(), cudaMemcpyHostToDevice, r.stream) != cudaSuccess)
+    // The bindings' records, most of the bytes, go from where they were made.
+    if (cudaMemcpyAsync(w, host.data(), o_p, cudaMemcpyHostToDevice, r.stream) != cudaSuccess ||
+        cudaMemcpyAsync(w + o_p, pdata.get(), pb, cudaMemcpyHostToDevice, r.stream) != cudaSuccess ||
+        (o_o > o_x &&
+         cudaMemcpyAsync(w + o_x, host.data() + o_x, o_o - o_x, cudaMemcpyHostToDevice, r.stream) != cudaSuccess))
         return MB2_ERR_CUDA;
     const mb2::Cd ph = mb2::initial_phase(0.0);
     if (mb2::launch_batch_init(r.state, num_qubits, num_bindings, ph.real(), ph.imag(), r.stream, o.precision) !=

@@ -15,6 +15,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <random>
 #include <stdexcept>
@@ -24,8 +25,43 @@
 
 #include "mb2_internal.h"
 
+// Streams of freed states, kept for the next ones (creating and destroying
+// one costs more than a small state's sweep).  At most kMost idle ones;
+// shared with the states, which may outlive their context.
+struct StreamPool {
+    static constexpr size_t kMost = 16;
+    std::mutex mu;
+    std::vector<cudaStream_t> idle;
+    cudaError_t take(cudaStream_t* out) {
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (!idle.empty()) {
+                *out = idle.back();
+                idle.pop_back();
+                return cudaSuccess;
+            }
+        }
+        return cudaStreamCreateWithFlags(out, cudaStreamNonBlocking);
+    }
+    // A stream with nothing queued on it.
+    void give(cudaStream_t s) {
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (idle.size() < kMost) {
+                idle.push_back(s);
+                return;
+            }
+        }
+        cudaStreamDestroy(s);
+    }
+    ~StreamPool() {
+        for (cudaStream_t s : idle) cudaStreamDestroy(s);
+    }
+};
+
 struct mb2_context {
     int device = 0;
+    std::shared_ptr<StreamPool> streams = std::make_shared<StreamPool>();
     int sm_count = 0;
     std::mutex mu;
     std::string last_error;
@@ -41,7 +77,8 @@ struct mb2_state {
     int precision = MB2_C128;
     void* amps = nullptr;
     cudaStream_t stream = nullptr;
-    bool owns_stream = true;
+    bool owns_stream = true;  // else the caller's
+    std::shared_ptr<StreamPool> streams;  // where an owned stream goes back to
     void* scratch = nullptr;  // staging: program, matrices, masks, partials
     size_t scratch_bytes = 0;
     // A host-resident state (mb2_state_alloc_host): the pinned, mapped host
@@ -399,14 +436,15 @@ int mb2_state_alloc(mb2_context* ctx, uint32_t num_qubits, int precision, uint64
     s->ctx = ctx;
     s->n = num_qubits;
     s->precision = precision;
-    cudaError_t e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
+    s->streams = ctx->streams;
+    cudaError_t e = s->streams->take(&s->stream);
     if (e != cudaSuccess) {
         delete s;
         return cuda_fail(ctx, e, "cudaStreamCreate");
     }
     e = cudaMallocAsync(&s->amps, bytes, s->stream);
     if (e != cudaSuccess) {
-        cudaStreamDestroy(s->stream);
+        s->streams->give(s->stream);
         delete s;
         return cuda_fail(ctx, e, "cudaMallocAsync(state)");
     }
@@ -439,7 +477,8 @@ int mb2_state_alloc_host(mb2_context* ctx, uint32_t num_qubits, uint64_t budget_
     s->ctx = ctx;
     s->n = num_qubits;
     s->precision = MB2_C128;
-    e = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
+    s->streams = ctx->streams;
+    e = s->streams->take(&s->stream);
     if (e != cudaSuccess) {
         cudaFreeHost(host);
         delete s;
@@ -461,9 +500,10 @@ int mb2_state_free(mb2_state* s) {
     if (s == nullptr) return MB2_OK;
     if (s->scratch) cudaFreeAsync(s->scratch, s->stream);
     if (s->host_amps == nullptr) cudaFreeAsync(s->amps, s->stream);
-    cudaStreamSynchronize(s->stream);
+    const cudaError_t done = cudaStreamSynchronize(s->stream);
     if (s->host_amps != nullptr) cudaFreeHost(s->host_amps);
-    if (s->owns_stream) cudaStreamDestroy(s->stream);
+    if (s->owns_stream && done == cudaSuccess) s->streams->give(s->stream);
+    else if (s->owns_stream) cudaStreamDestroy(s->stream);
     delete s;
     return MB2_OK;
 }

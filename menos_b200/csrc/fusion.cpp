@@ -41,8 +41,14 @@ void host_apply_generic(Cd* state, uint64_t n_amps, const Cd* matrix, const uint
     uint64_t mask = 0;
     for (uint32_t j = 0; j < k; ++j) mask |= uint64_t{1} << operands[j];
     const uint64_t n_outer = n_amps >> k;
-    std::vector<uint64_t> idx(dim);
-    std::vector<Cd> g(dim);
+    // (A fused block's matrix is built from one call per member: no
+    // allocation for the operand counts it has.)
+    uint64_t idx_few[1u << MB2_MAX_OP_QUBITS];
+    Cd g_few[1u << MB2_MAX_OP_QUBITS];
+    std::vector<uint64_t> idx_many(k > MB2_MAX_OP_QUBITS ? dim : 0);
+    std::vector<Cd> g_many(k > MB2_MAX_OP_QUBITS ? dim : 0);
+    uint64_t* const idx = k > MB2_MAX_OP_QUBITS ? idx_many.data() : idx_few;
+    Cd* const g = k > MB2_MAX_OP_QUBITS ? g_many.data() : g_few;
     for (uint64_t compact = 0; compact < n_outer; ++compact) {
         uint64_t base = 0;
         int src = 0;

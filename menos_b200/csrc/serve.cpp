@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <condition_variable>
 #include <cstring>
@@ -201,7 +202,11 @@ void run_small_batch(mb2_server* s, cudaStream_t stream, std::vector<Request>& b
     std::vector<mb2::TileProgram> progs(B);
     std::vector<uint32_t> tile(B, 0);
     std::vector<bool> ok(B, true);
-    for (size_t i = 0; i < B; ++i) {
+    // Plans and draws: host work of half a millisecond a request, spread over a
+    // few threads (vectors of bool share bytes, hence the plain flags).
+    std::vector<uint8_t> planned(B, 0);
+    std::vector<std::vector<double>> uniforms(B);
+    auto prepare = [&](size_t i) {
         const Request& r = batch[i];
         try {
             const std::vector<mb2::Block> blocks =
@@ -210,13 +215,33 @@ void run_small_batch(mb2_server* s, cudaStream_t stream, std::vector<Request>& b
             for (const mb2::Block& b : blocks) m = std::max(m, b.k);
             if (m > r.n) throw std::invalid_argument("a block wider than the state");
             progs[i] = mb2::plan_tile_program(blocks, r.n, m, mb2::kDefaultFixedLow, nullptr, false);
-            mb2::encode_compact(progs[i]);
             tile[i] = std::min(m, r.n);
+            if (r.output == MB2_OUT_COUNTS && r.shots > 0)
+                uniforms[i] = mb2::sorted_reference_uniforms(r.shots, r.seed);
+            planned[i] = 1;
         } catch (const std::exception&) {
+        }
+    };
+    {
+        const size_t threads = std::min<size_t>({8, std::max(1u, std::thread::hardware_concurrency()), (B + 3) / 4});
+        std::atomic<size_t> next{0};
+        auto work = [&]() {
+            for (size_t i = next++; i < B; i = next++) prepare(i);
+        };
+        std::vector<std::thread> helpers;
+        try {
+            helpers.reserve(threads);
+            for (size_t t = 1; t < threads; ++t) helpers.emplace_back(work);
+        } catch (const std::exception&) {  // fewer helpers
+        }
+        work();
+        for (std::thread& t : helpers) t.join();
+    }
+    for (size_t i = 0; i < B; ++i)
+        if (!planned[i]) {
             ok[i] = false;
             dones[i].c.status = MB2_ERR_INVALID;
         }
-    }
     // Device layout: [uploaded: programs, job tables, init table, uniforms]
     // [states] [written: terms, basis].
     auto up = [](size_t v) { return (v + 255) & ~size_t{255}; };
@@ -281,7 +306,6 @@ void run_small_batch(mb2_server* s, cudaStream_t stream, std::vector<Request>& b
     std::vector<mb2::ExpectJob> ejobs;
     std::vector<size_t> e_first(B, 0);
     std::vector<mb2::WalkJob> wjobs;
-    std::vector<std::vector<double>> uniforms(B);
     for (size_t i = 0; i < B; ++i) {
         if (!ok[i]) continue;
         const Request& r = batch[i];
@@ -289,7 +313,6 @@ void run_small_batch(mb2_server* s, cudaStream_t stream, std::vector<Request>& b
             e_first[i] = ejobs.size();
             for (size_t t = 0; t < r.xs.size(); ++t) ejobs.push_back(mb2::ExpectJob{nullptr, r.xs[t], r.zs[t], r.n, 0});
         } else if (r.shots > 0) {
-            uniforms[i] = mb2::sorted_reference_uniforms(r.shots, r.seed);
             u_off[i] = off;
             off = up(off + r.shots * 8);
         }

@@ -377,14 +377,18 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
         return true;
     };
     // Blocks that can run inside tile s from heads h, in a dependency order
-    // (h advances past them); stops at the pass limits when `limit`.
+    // (h advances past them); stops at the pass limits when `limit`.  Only
+    // the heads of the qubits in `from` are looked at first: where h is already
+    // past everything that runs in s without qubit x, x alone is enough, which
+    // is how a candidate is tried below (a whole closure for each was most of
+    // the time a plan took).
     std::vector<uint32_t> work;
-    auto closure = [&](uint64_t s, std::vector<uint32_t>& h, std::vector<uint32_t>* out, bool limit) {
+    auto closure = [&](uint64_t s, std::vector<uint32_t>& h, std::vector<uint32_t>* out, bool limit, uint64_t from) {
         uint32_t count = 0;
         size_t staged = staged_of.base();
         work.clear();
         for (uint32_t x = 0; x < n; ++x)
-            if ((s >> x) & 1u) work.push_back(x);
+            if ((from >> x) & 1u) work.push_back(x);
         while (!work.empty()) {
             const uint32_t x = work.back();
             work.pop_back();
@@ -406,18 +410,20 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
     };
     uint32_t applied = 0, first = 0;
     std::vector<uint8_t> done(nb, 0);
-    std::vector<uint32_t> h;
+    std::vector<uint32_t> h, base;
     while (applied < nb) {
         while (done[first]) ++first;
         uint64_t s = blocks[first].mask();
         for (uint32_t q = 0; q < fixed; ++q) s |= uint64_t{1} << q;
+        base = head;
+        uint64_t base_runs = closure(s, base, nullptr, false, s);
         while (static_cast<uint32_t>(std::popcount(s)) < mt) {
             uint64_t best_score = 0;
             uint32_t best = n;
             for (uint32_t x = 0; x < n; ++x) {
                 if ((s >> x) & 1u) continue;
-                h = head;
-                const uint64_t runs = closure(s | (uint64_t{1} << x), h, nullptr, false);
+                h = base;
+                const uint64_t runs = base_runs + closure(s | (uint64_t{1} << x), h, nullptr, false, uint64_t{1} << x);
                 // Blocked blocks at the tile's heads that wait for x.
                 uint32_t waits = 0;
                 for (uint32_t y = 0; y < n; ++y)
@@ -431,18 +437,19 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
                 }
             }
             s |= uint64_t{1} << best;
+            base_runs += closure(s, base, nullptr, false, uint64_t{1} << best);
         }
         std::vector<uint32_t> members;
         h = head;
-        closure(s, h, &members, true);
+        closure(s, h, &members, true, s);
         if (members.empty()) throw std::logic_error("tile selection made no progress");
         // Phase-by-phase order of the members.
         PassSel sel;
         sel.smask = s;
         std::vector<uint8_t> in_pass(nb, 0);
         for (uint32_t i : members) in_pass[i] = 1;
-        std::vector<uint32_t> ph = head, sim;
-        std::vector<uint8_t> sim_in;
+        std::vector<uint32_t> ph = head, sim, grown;
+        std::vector<uint8_t> sim_in, grown_in;
         // Runs every member that register set `regs` can take (diagonals and
         // wide blocks need none), from heads hh, in waves: the ready dense
         // blocks, then the ready diagonals (so that the diagonals of one
@@ -474,6 +481,27 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
                             work.push_back(b.q[t]);
                         }
                     }
+                }
+            }
+            return dense;
+        };
+        // The dense blocks that `regs` lets run from heads hh (which advance, as
+        // `in` does), starting at qubit x: the same set as run's, in any order.
+        auto count_from = [&](uint64_t regs, uint32_t x, std::vector<uint32_t>& hh, std::vector<uint8_t>& in) {
+            uint32_t dense = 0;
+            work.assign(1, x);
+            while (!work.empty()) {
+                const uint32_t y = work.back();
+                work.pop_back();
+                if (hh[y] >= lists[y].size()) continue;
+                const uint32_t i = lists[y][hh[y]];
+                const Block& b = blocks[i];
+                if (!in[i] || moves[i] || !at_head(hh, i) || !(b.diagonal || b.k > 2 || (b.mask() & ~regs) == 0)) continue;
+                in[i] = 0;
+                if (!b.diagonal && b.k <= 2) ++dense;
+                for (uint32_t t = 0; t < b.k; ++t) {
+                    ++hh[b.q[t]];
+                    work.push_back(b.q[t]);
                 }
             }
             return dense;
@@ -517,14 +545,17 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
                 }
             }
             regs = 0;
+            grown = ph;  // the heads after what the registers chosen so far let run
+            grown_in = in_pass;
+            uint64_t grown_runs = 0;
             for (uint32_t r = 0; r < kRegQubits && (cand & ~regs) != 0; ++r) {
                 uint64_t best_score = 0;
                 uint32_t best = n;
                 for (uint32_t x = 0; x < n; ++x) {
                     if (!((cand >> x) & 1u) || ((regs >> x) & 1u)) continue;
-                    sim = ph;
-                    sim_in = in_pass;
-                    const uint64_t runs = run(regs | (uint64_t{1} << x), sim, sim_in, nullptr);
+                    sim = grown;
+                    sim_in = grown_in;
+                    const uint64_t runs = grown_runs + count_from(regs | (uint64_t{1} << x), x, sim, sim_in);
                     uint32_t uses = 0;
                     for (uint32_t i : members)
                         if (in_pass[i] && !blocks[i].diagonal && blocks[i].k <= 2 && !moves[i] &&
@@ -537,6 +568,7 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
                     }
                 }
                 regs |= uint64_t{1} << best;
+                grown_runs += count_from(regs, best, grown, grown_in);
             }
             if (regs == 0) throw std::logic_error("phase ordering made no progress");
         }
