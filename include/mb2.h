@@ -556,6 +556,13 @@ int mb2_debug_schedule(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_opti
 int mb2_debug_run_plan(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_options* opts, uint32_t num_qubits,
                        int32_t precision, double* state, uint64_t* stats);
 
+/* The most bytes of instructions and data that a pass of that program (a pass
+ * in tensor-core form aside) stages in shared memory beside its tile buffers,
+ * data counted in FP64, and the limit that a plan keeps to (a single block
+ * may exceed it).  num_qubits 4..40.  Has no counterpart in the reference. */
+int mb2_debug_staged_bytes(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_options* opts, uint32_t num_qubits,
+                           int32_t precision, uint64_t* most, uint64_t* limit);
+
 /* The complex64 tensor-core step alone, on the context's device: 256 rows of
  * 16 complex64 amplitudes (rows: 256 * 32 floats, interleaved) times the
  * 16x16 complex matrix (row-major, interleaved doubles) as the tile pass

@@ -2010,6 +2010,29 @@ int mb2_synchronize(mb2_state* s) {
     return MB2_OK;
 }
 
+namespace {
+
+// The tiled program mb2_apply_program would plan for a num_qubits state, of
+// the operations' blocks; m and tc: its tile width and form.
+mb2::TileProgram debug_plan(const std::vector<mb2::Block>& blocks, const mb2_sweep_options& o, uint32_t num_qubits,
+                            bool c64, uint32_t& m, bool& tc) {
+    m = tile_width(o.tile_qubits > 0 ? static_cast<uint32_t>(o.tile_qubits) : 0, num_qubits, blocks);
+    tc = false;
+    if (c64) {
+        const C64Choice ch = c64_choice(o, num_qubits, mb2::kDefaultTileQubitsC64, blocks);
+        m = ch.m;
+        tc = ch.tc;
+    }
+    m = std::min(std::max(m, mb2::kMinTileQubits), num_qubits);
+    const uint32_t low = o.low_qubits < 0 ? 0u : (o.low_qubits == 0 ? mb2::kDefaultFixedLow
+                                                                     : static_cast<uint32_t>(o.low_qubits));
+    mb2::TileProgram prog = mb2::plan_tile_program(blocks, num_qubits, m, low, nullptr, c64, !tc);
+    if (tc) mb2::make_tensor_core_program(prog, blocks, mb2::tc_max_phases(m));
+    return prog;
+}
+
+}  // namespace
+
 int mb2_debug_run_plan(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_options* opts, uint32_t num_qubits,
                        int32_t precision, double* state, uint64_t* stats) {
     if ((ops == nullptr && num_ops != 0) || num_qubits < 1 || num_qubits > 40 || (state != nullptr && num_qubits > 28) ||
@@ -2021,19 +2044,10 @@ int mb2_debug_run_plan(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_opti
         const std::vector<mb2::Block> blocks = mb2::build_blocks(ops, num_ops, o.fuse_gates != 0, static_cast<uint32_t>(o.fusion_width));
         if (blocks.empty()) return MB2_OK;
         const bool c64 = precision == MB2_C64;
-        uint32_t m = tile_width(o.tile_qubits > 0 ? static_cast<uint32_t>(o.tile_qubits) : 0, num_qubits, blocks);
+        if (c64 && num_qubits < mb2::kMinTileQubits) return MB2_ERR_UNSUPPORTED;
+        uint32_t m = 0;
         bool tc = false;
-        if (c64) {
-            if (num_qubits < mb2::kMinTileQubits) return MB2_ERR_UNSUPPORTED;
-            const C64Choice ch = c64_choice(o, num_qubits, mb2::kDefaultTileQubitsC64, blocks);
-            m = ch.m;
-            tc = ch.tc;
-        }
-        m = std::min(std::max(m, mb2::kMinTileQubits), num_qubits);
-        const uint32_t low = o.low_qubits < 0 ? 0u : (o.low_qubits == 0 ? mb2::kDefaultFixedLow
-                                                                         : static_cast<uint32_t>(o.low_qubits));
-        mb2::TileProgram prog = mb2::plan_tile_program(blocks, num_qubits, m, low, nullptr, c64, !tc);
-        if (tc) mb2::make_tensor_core_program(prog, blocks, mb2::tc_max_phases(m));
+        const mb2::TileProgram prog = debug_plan(blocks, o, num_qubits, c64, m, tc);
         if (state != nullptr) mb2::run_program_on_host(prog, num_qubits, reinterpret_cast<mb2::Cd*>(state));
         if (stats != nullptr) {
             uint64_t tcp = 0, smem = 0, layouts = 0;
@@ -2051,6 +2065,30 @@ int mb2_debug_run_plan(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_opti
             stats[4] = smem;
             stats[5] = layouts;
         }
+    } catch (const std::exception&) {
+        return MB2_ERR_INVALID;
+    }
+    return MB2_OK;
+}
+
+int mb2_debug_staged_bytes(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_options* opts, uint32_t num_qubits,
+                           int32_t precision, uint64_t* most, uint64_t* limit) {
+    if ((ops == nullptr && num_ops != 0) || most == nullptr || limit == nullptr || num_qubits < mb2::kMinTileQubits ||
+        num_qubits > 40 || (precision != MB2_C128 && precision != MB2_C64))
+        return MB2_ERR_INVALID;
+    mb2_sweep_options o{1, 0, 0, 0, 0, 0};
+    if (opts != nullptr) o = *opts;
+    *most = 0;
+    *limit = mb2::kStagedLimit;
+    try {
+        const std::vector<mb2::Block> blocks = mb2::build_blocks(ops, num_ops, o.fuse_gates != 0, static_cast<uint32_t>(o.fusion_width));
+        if (blocks.empty()) return MB2_OK;
+        uint32_t m = 0;
+        bool tc = false;
+        const mb2::TileProgram prog = debug_plan(blocks, o, num_qubits, precision == MB2_C64, m, tc);
+        for (const mb2::TilePass& p : prog.passes)
+            if (!p.tc)
+                *most = std::max(*most, uint64_t{p.word_count} * 4 + (uint64_t{p.sdata_count} + p.param_len) * sizeof(double));
     } catch (const std::exception&) {
         return MB2_ERR_INVALID;
     }

@@ -257,8 +257,11 @@ constexpr uint32_t kMma = 202;
 // threads whose tile bits cover bits 16-31 change sign.
 }  // namespace cop
 
-// Shared-memory budget of one pass's staged instructions + data.
-constexpr size_t kMaxStagedBytes = 32 * 1024 - cop::kStoreWords * 4;
+// Shared-memory budget of one pass's staged instructions + data, and what of
+// it the blocks may take: the rest is the store record's, the instruction
+// before it and the padding to 16 bytes.
+constexpr size_t kStagedLimit = 32 * 1024;
+constexpr size_t kMaxStagedBytes = kStagedLimit - (cop::kStoreWords + 4) * 4;
 
 // TileInstr.data: for TOP_SMEM an offset into the program's global-only data
 // block (gdata); for every other instruction an offset into its pass's

@@ -25,23 +25,32 @@
 namespace mb2 {
 namespace {
 
-// A pass's instruction words and small-matrix data are staged in shared
-// memory (kMaxStagedBytes); a block costs at most a phase record, three
-// more words (gate, extra word, end) and its staged entries.
 constexpr size_t kMaxBlocksPerPass = 300;
 
-// A diagonal runs in whatever phase is open; it opens one only at the pass's
-// start or behind a permutation, whose own estimate holds that.
+// A pass's instruction words and small-matrix data are staged in shared memory
+// (kMaxStagedBytes): a bound on what each block adds, whatever order the
+// pass's blocks come in.
+//
+// Phase records: a dense block of one or two qubits opens at most one.  A
+// diagonal runs in whatever phase is open, so it opens one only at the pass's
+// start (base), behind a permutation or behind a wide block (k >= 3), and is
+// held by those: a permutation counts one record, a wide block one, and in a
+// program with permutations one more, for the phase that brings moved
+// amplitudes back before it.  Every record is counted as large as a program
+// with permutations may need it.
+// Words beside them: a gate's, at most one extra and its phase's end for a
+// dense block or a diagonal, a wide block's three and the end of the phase
+// that brings amplitudes back.
 struct Staged {
     uint32_t m;
     bool mapped, c64;  // the program has permutations; it is the complex64 kernels'
     size_t operator()(const Block& b, bool move) const {
         const size_t dim = size_t{1} << b.k;
-        const size_t entries = move ? 0 : b.diagonal ? dim : (b.k <= 2 ? dim * dim : 0);
-        const size_t phase = b.diagonal ? 0
-                             : mapped   ? cop::phase_map_words(m) + (c64 ? 0 : cop::kMaxMapControls)
-                                        : cop::phase_words(m);
-        return (phase + (move ? 0 : 3)) * sizeof(uint32_t) + entries * 2 * sizeof(double);
+        const bool wide = !b.diagonal && b.k > 2;
+        const size_t entries = move || wide ? 0 : b.diagonal ? dim : dim * dim;
+        const size_t record = mapped ? cop::phase_map_words(m) + (c64 ? 0 : cop::kMaxMapControls) : cop::phase_words(m);
+        const size_t records = b.diagonal ? 0 : wide && mapped ? 2 : 1;
+        return (records * record + (move ? 0 : wide ? 4 : 3)) * sizeof(uint32_t) + entries * 2 * sizeof(double);
     }
     size_t base() const { return cop::phase_map_words(m) * sizeof(uint32_t); }
 };
