@@ -272,9 +272,15 @@ class DeviceState:
         return out
 
     def copy_out(self, out: Optional[np.ndarray] = None) -> np.ndarray:
-        """The amplitudes; out: a host_array to put them into."""
+        """The amplitudes; out: a host_array, or an array like one, to put
+        them into (ValueError where it is not one the library can fill)."""
         if out is None:
             out = self.host_array()
+        else:
+            dt = np.complex128 if self.precision == C128 else np.complex64
+            if not (isinstance(out, np.ndarray) and out.dtype == dt and out.size == 1 << self.n
+                    and out.flags.c_contiguous and out.flags.aligned and out.flags.writeable):
+                raise ValueError(f"out must be a contiguous, writeable {np.dtype(dt)} array of {1 << self.n} amplitudes")
         self._chk(lib().mb2_copy_out(self.h, out.ctypes.data, out.size), "mb2_copy_out")
         return out
 
