@@ -563,6 +563,12 @@ int mb2_debug_run_plan(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_opti
 int mb2_debug_staged_bytes(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_options* opts, uint32_t num_qubits,
                            int32_t precision, uint64_t* most, uint64_t* limit);
 
+/* From now on this context's scratch, and what mb2_trajectories takes beside
+ * its one state, is refused above `bytes` a piece, as by a device that has no
+ * more left (0: no limit).  Lets tests take the paths for a full device.  Has
+ * no counterpart in the reference. */
+int mb2_debug_room(mb2_context* ctx, uint64_t bytes);
+
 /* The complex64 tensor-core step alone, on the context's device: 256 rows of
  * 16 complex64 amplitudes (rows: 256 * 32 floats, interleaved) times the
  * 16x16 complex matrix (row-major, interleaved doubles) as the tile pass

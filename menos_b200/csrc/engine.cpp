@@ -63,6 +63,7 @@ struct mb2_context {
     int device = 0;
     std::shared_ptr<StreamPool> streams = std::make_shared<StreamPool>();
     int sm_count = 0;
+    std::atomic<uint64_t> debug_room{0};  // mb2_debug_room
     std::mutex mu;
     std::string last_error;
     // Tile widths and time-model costs (mb2_autotune; built-in defaults
@@ -114,6 +115,14 @@ int cuda_fail(mb2_context* ctx, cudaError_t e, const char* what) {
 
 size_t amp_bytes(int precision) { return precision == MB2_C64 ? 8 : 16; }
 
+// Stream-ordered device memory.  A context's debug_room stands in for a device
+// that has no more than that many bytes left in one piece.
+cudaError_t take_device(mb2_context* ctx, void** p, size_t bytes, cudaStream_t stream) {
+    const uint64_t room = ctx->debug_room.load();
+    if (room != 0 && bytes > room) return cudaErrorMemoryAllocation;
+    return cudaMallocAsync(p, bytes, stream);
+}
+
 // Grow-only device staging buffer of the state.  Allocations are
 // stream-ordered (cudaMallocAsync / cudaFreeAsync on the state's stream):
 // work queued before a free finishes before the memory is reused, and no
@@ -126,7 +135,7 @@ int ensure_scratch(mb2_state* s, size_t bytes) {
     s->scratch_bytes = 0;
     size_t want = 1 << 20;
     while (want < bytes) want <<= 1;
-    MB2_CUDA(s->ctx, cudaMallocAsync(&s->scratch, want, s->stream));
+    MB2_CUDA(s->ctx, take_device(s->ctx, &s->scratch, want, s->stream));
     s->scratch_bytes = want;
     return MB2_OK;
 }
@@ -1032,6 +1041,12 @@ int mb2_estimate_sweep(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_opti
     return MB2_OK;
 }
 
+int mb2_debug_room(mb2_context* ctx, uint64_t bytes) {
+    if (ctx == nullptr) return MB2_ERR_INVALID;
+    ctx->debug_room.store(bytes);
+    return MB2_OK;
+}
+
 int mb2_last_sweep_stats(mb2_state* s, mb2_sweep_stats* out) {
     if (s == nullptr || out == nullptr) return MB2_ERR_INVALID;
     *out = s->stats;
@@ -1563,6 +1578,30 @@ struct TrajChannel {
 // together (a larger state runs alone).
 constexpr uint64_t kTrajBatch = 64;
 constexpr uint64_t kTrajBatchBytes = uint64_t{256} << 20;
+uint64_t trajectory_batch(uint32_t n, uint64_t trajectories, bool monitored) {
+    if (monitored) return 1;
+    return std::max<uint64_t>(1, std::min({kTrajBatch, trajectories, kTrajBatchBytes / (uint64_t{16} << n)}));
+}
+
+// What a batch takes on the device beside its states: byte offsets of the
+// uploaded program and channels, the draws, the outputs and the kernels'
+// scratch.
+struct TrajLayout {
+    size_t u, shot, err, basis, vals, chan, norms, terms, bytes;
+    TrajLayout(uint32_t n, uint64_t batch, uint64_t channels, uint64_t num_terms, size_t upload, size_t term_bytes) {
+        auto up = [](size_t v) { return (v + 255) & ~size_t{255}; };
+        const auto b = static_cast<uint32_t>(batch);
+        u = up(upload);
+        shot = u + up(batch * channels * 8);
+        err = shot + up(batch * 8);
+        basis = err + up(batch * 4);
+        vals = basis + up(batch * 8);
+        chan = vals + up(batch * num_terms * 16);
+        norms = chan + up(mb2::traj_scratch_bytes(n, b));
+        terms = norms + up(mb2::norms_scratch_bytes(n, b));
+        bytes = terms + term_bytes;
+    }
+};
 
 // K^dagger K (kraus_products, trajectory_engine.cpp:50-69).
 std::vector<mb2::Cd> kraus_product(const std::vector<mb2::Cd>& k, size_t dim) {
@@ -1700,8 +1739,7 @@ int mb2_trajectories_monitored(mb2_context* ctx, uint32_t n, const mb2_op* ops, 
     // Trajectories run in batches, their states back to back, every launch for
     // the whole batch; a monitored run one at a time.
     const uint64_t state_amps = uint64_t{1} << n;
-    uint64_t batch = std::clamp<uint64_t>(kTrajBatchBytes / (16 * state_amps), 1, std::min(kTrajBatch, trajectories));
-    if (boundary != nullptr) batch = 1;
+    uint64_t batch = trajectory_batch(n, trajectories, boundary != nullptr);
     struct Work {  // the batch's states, as a state whose first 2^n amplitudes are trajectory 0's
         mb2_state* s = nullptr;
         void* extra = nullptr;
@@ -1714,31 +1752,34 @@ int mb2_trajectories_monitored(mb2_context* ctx, uint32_t n, const mb2_op* ops, 
     if (int e = mb2_state_alloc(ctx, n, MB2_C128, ~uint64_t{0}, &work.s); e != MB2_OK) return e;
     mb2_state* const st = work.s;
     const cudaStream_t stream = st->stream;
+    const ExpectPlan terms(n, x_masks, z_masks, num_terms);
+    const uint32_t C = static_cast<uint32_t>(channels.size());
+    const size_t term_bytes = want_exp ? terms.bytes() : 0;
+    TrajLayout at(n, batch, C, num_terms, upload.size(), term_bytes);
     if (batch > 1) {
-        MB2_CUDA(ctx, cudaFreeAsync(st->amps, stream));
-        if (cudaMallocAsync(&st->amps, batch * 16 * state_amps, stream) != cudaSuccess) {
+        // Where the device refuses the batch's states, or what goes with them,
+        // there is still the one state.
+        void* states = nullptr;
+        if (take_device(ctx, &states, batch * 16 * state_amps, stream) != cudaSuccess) states = nullptr;
+        if (states != nullptr && take_device(ctx, &work.extra, at.bytes, stream) != cudaSuccess) work.extra = nullptr;
+        if (work.extra != nullptr) {
+            MB2_CUDA(ctx, cudaFreeAsync(st->amps, stream));
+            st->amps = states;
+        } else {
             cudaGetLastError();
+            if (states != nullptr) cudaFreeAsync(states, stream);
             batch = 1;
-            st->amps = nullptr;
-            MB2_CUDA(ctx, cudaMallocAsync(&st->amps, 16 * state_amps, stream));
+            at = TrajLayout(n, batch, C, num_terms, upload.size(), term_bytes);
         }
     }
-    const uint32_t B = static_cast<uint32_t>(batch), C = static_cast<uint32_t>(channels.size());
-    auto up = [](size_t v) { return (v + 255) & ~size_t{255}; };
-    const ExpectPlan terms(n, x_masks, z_masks, num_terms);
-    const size_t off_u = up(upload.size()), off_shot = off_u + up(size_t{B} * C * 8), off_err = off_shot + up(B * 8),
-                 off_basis = off_err + up(B * 4), off_vals = off_basis + up(B * 8),
-                 off_chan = off_vals + up(size_t{B} * num_terms * 16),
-                 off_norms = off_chan + up(mb2::traj_scratch_bytes(n, B)),
-                 off_terms = off_norms + up(mb2::norms_scratch_bytes(n, B)),
-                 bytes = off_terms + (want_exp ? terms.bytes() : 0);
-    MB2_CUDA(ctx, cudaMallocAsync(&work.extra, bytes, stream));
+    if (work.extra == nullptr) MB2_CUDA(ctx, take_device(ctx, &work.extra, at.bytes, stream));
+    const uint32_t B = static_cast<uint32_t>(batch);
     auto* const dev = static_cast<unsigned char*>(work.extra);
     if (!upload.empty()) MB2_CUDA(ctx, cudaMemcpyAsync(dev, upload.data(), upload.size(), cudaMemcpyHostToDevice, stream));
     if (want_exp)
-        if (int e = terms.upload(ctx, dev + off_terms, stream); e != MB2_OK) return e;
-    auto* const dev_err = reinterpret_cast<int*>(dev + off_err);
-    auto* const dev_vals = reinterpret_cast<double*>(dev + off_vals);
+        if (int e = terms.upload(ctx, dev + at.terms, stream); e != MB2_OK) return e;
+    auto* const dev_err = reinterpret_cast<int*>(dev + at.err);
+    auto* const dev_vals = reinterpret_cast<double*>(dev + at.vals);
     std::vector<mb2::Cd> term_sums(num_terms, mb2::Cd{0.0, 0.0});
     std::vector<double> vals(size_t{2} * B * std::max<uint32_t>(num_terms, 1)), draws(size_t{B} * std::max<uint32_t>(C, 1)),
         shot_draws(B);
@@ -1781,7 +1822,7 @@ int mb2_trajectories_monitored(mb2_context* ctx, uint32_t n, const mb2_op* ops, 
             if (want_counts && t0 + t < shots) shot_draws[t] = word_to_uniform(rngs[t]());
         }
         if (C != 0)
-            MB2_CUDA(ctx, cudaMemcpyAsync(dev + off_u, draws.data(), size_t{nt} * C * 8, cudaMemcpyHostToDevice, stream));
+            MB2_CUDA(ctx, cudaMemcpyAsync(dev + at.u, draws.data(), size_t{nt} * C * 8, cudaMemcpyHostToDevice, stream));
         MB2_CUDA(ctx, cudaMemsetAsync(dev_err, 0, B * sizeof(int), stream));
         // |0..0>, no global phase.
         if (int e = launched(mb2::launch_batch_init(st->amps, n, nt, 1.0, 0.0, stream, MB2_C128)); e != MB2_OK) return e;
@@ -1823,13 +1864,13 @@ int mb2_trajectories_monitored(mb2_context* ctx, uint32_t n, const mb2_op* ops, 
             } else {
                 const TrajChannel& ch = channels[idx];
                 const mb2::TrajChannelData data{dev + ch.products, dev + ch.kraus, ch.branches,
-                                                reinterpret_cast<const double*>(dev + off_u) + idx, C};
+                                                reinterpret_cast<const double*>(dev + at.u) + idx, C};
                 if (int e = launched(mb2::launch_traj_channel(st->amps, n, nt, ch.qubits.data(),
                                                               static_cast<uint32_t>(ch.qubits.size()), pending, data,
-                                                              dev + off_chan, dev_err, stream));
+                                                              dev + at.chan, dev_err, stream));
                     e != MB2_OK)
                     return e;
-                if (int e = launched(mb2::launch_norms(st->amps, n, nt, dev + off_norms, &pending.norms, &pending.pitch,
+                if (int e = launched(mb2::launch_norms(st->amps, n, nt, dev + at.norms, &pending.norms, &pending.pitch,
                                                        stream));
                     e != MB2_OK)
                     return e;
@@ -1843,20 +1884,20 @@ int mb2_trajectories_monitored(mb2_context* ctx, uint32_t n, const mb2_op* ops, 
         const uint32_t ns = want_counts && t0 < shots ? static_cast<uint32_t>(std::min<uint64_t>(nt, shots - t0)) : 0;
         if (want_exp)
             for (uint32_t t = 0; t < nt; ++t)
-                if (int e = terms.launch(ctx, static_cast<mb2::Cd*>(st->amps) + t * state_amps, MB2_C128, dev + off_terms,
+                if (int e = terms.launch(ctx, static_cast<mb2::Cd*>(st->amps) + t * state_amps, MB2_C128, dev + at.terms,
                                          dev_vals + size_t{2} * t * num_terms, stream);
                     e != MB2_OK)
                     return e;
         if (ns != 0) {
-            MB2_CUDA(ctx, cudaMemcpyAsync(dev + off_shot, shot_draws.data(), ns * 8, cudaMemcpyHostToDevice, stream));
+            MB2_CUDA(ctx, cudaMemcpyAsync(dev + at.shot, shot_draws.data(), ns * 8, cudaMemcpyHostToDevice, stream));
             for (uint32_t t = 0; t < ns; ++t)
                 if (int e = launched(mb2::launch_sample(static_cast<mb2::Cd*>(st->amps) + t * state_amps, n,
-                                                        reinterpret_cast<double*>(dev + off_shot) + t, 1, nullptr, nullptr,
-                                                        dev + off_norms, reinterpret_cast<uint64_t*>(dev + off_basis) + t,
+                                                        reinterpret_cast<double*>(dev + at.shot) + t, 1, nullptr, nullptr,
+                                                        dev + at.norms, reinterpret_cast<uint64_t*>(dev + at.basis) + t,
                                                         stream));
                     e != MB2_OK)
                     return e;
-            MB2_CUDA(ctx, cudaMemcpyAsync(basis.data(), dev + off_basis, ns * 8, cudaMemcpyDeviceToHost, stream));
+            MB2_CUDA(ctx, cudaMemcpyAsync(basis.data(), dev + at.basis, ns * 8, cudaMemcpyDeviceToHost, stream));
         }
         if (want_exp)
             MB2_CUDA(ctx, cudaMemcpyAsync(vals.data(), dev_vals, size_t{nt} * num_terms * 16, cudaMemcpyDeviceToHost, stream));
