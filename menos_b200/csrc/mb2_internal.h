@@ -277,6 +277,7 @@ struct TileProgram {
     std::vector<double> data;
     std::vector<uint32_t> words;  // compact stream of every pass
     bool c64 = false;             // for the complex64 kernels (8-byte slots)
+    std::vector<uint8_t> tc_blocks;  // per block, tc_convertible (a program to be rewritten for the tensor cores)
     uint64_t fp64_per_amp = 0;    // modelled FP64 instructions per amplitude
     // Tensor-core passes: per composed phase matrix, its real 32x32 form as
     // FP16 high and low parts in the MMA's shared-memory layout (tile_tc.cpp),
@@ -299,6 +300,7 @@ void encode_compact(TileProgram& prog);
 // 0-31) over FP16 low parts (rows 32-63), 4096 bytes.
 constexpr uint32_t kTcOperandWords = 1024;
 constexpr double kTcOperandScale = 4096.0;  // U's operand is 2^12 U
+bool tc_convertible(const Block& b);
 void make_tensor_core_program(TileProgram& prog, const std::vector<Block>& blocks, uint32_t max_phases);
 // Thread-bit order of a phase whose register bits are reg[0..nreg) (tile
 // positions): tperm[0..nthread) lists the other tile positions, the first
@@ -332,7 +334,8 @@ constexpr uint8_t kParamM00Real = 4;   // ... entry (0,0) is real in every bindi
 // (the complex64 path, whose result is not bitwise the reference's), and
 // the passes follow a dependency order chosen for few passes and phases.
 // split: two-qubit blocks that are a permutation and a one-qubit gate run as
-// the two (off for a program that is rewritten for the tensor cores).
+// the two (off for a commuting program that make_tensor_core_program rewrites,
+// which takes permutations as it takes other blocks).
 TileProgram plan_tile_program(const std::vector<Block>& blocks, uint32_t n, uint32_t m,
                               uint32_t fixed_low = kDefaultFixedLow,
                               const std::vector<uint8_t>* parametric = nullptr, bool commuting = false,

@@ -53,15 +53,21 @@ constexpr size_t kMaxAhead = 512;
 struct Staged {
     uint32_t m;
     bool mapped, c64;  // the program has permutations; it is the complex64 kernels'
+    bool tc = false;   // every pass is rewritten for the tensor cores
     size_t operator()(const Block& b, bool move) const {
         const size_t dim = size_t{1} << b.k;
+        // Nothing of this is staged then; 128 bytes a block and its entries
+        // make passes whose phase matrices fill the room they have (longer ones
+        // are split and leave short ends: 17 passes instead of 14 for the
+        // unfused 30-qubit ansatz of 10 layers).
+        if (tc) return 128 + (b.diagonal ? dim : dim * dim) * 2 * sizeof(double);
         const bool wide = !b.diagonal && b.k > 2;
         const size_t entries = move || wide ? 0 : b.diagonal ? dim : dim * dim;
         const size_t record = mapped ? cop::phase_map_words(m) + (c64 ? 0 : cop::kMaxMapControls) : cop::phase_words(m);
         const size_t records = b.diagonal ? 0 : wide && mapped ? 2 : 1;
         return (records * record + (move ? 0 : wide ? 4 : 3)) * sizeof(uint32_t) + entries * 2 * sizeof(double);
     }
-    size_t base() const { return cop::phase_map_words(m) * sizeof(uint32_t); }
+    size_t base() const { return tc ? 0 : cop::phase_map_words(m) * sizeof(uint32_t); }
 };
 
 uint32_t local_pos(uint64_t smask, uint32_t q) {
@@ -369,9 +375,13 @@ void thread_bit_order(uint32_t m, const uint32_t* reg, uint32_t nreg, uint8_t* t
 // next set from the ready dense blocks, so the kernel changes phase rarely.
 // Exact permutations need no registers either, but end the phase they come
 // in (the amplitudes' places change), so they wait until no other block of
-// the pass is ready.
+// the pass is ready.  Not in a program that is rewritten for the tensor cores
+// (tc_blocks: which blocks can be): there they are part of a phase's matrix
+// like any other block, and waiting would spread them over more phases
+// (81 layouts instead of 75 for a 26-qubit RY/RZ + CX ansatz, unfused).
 std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, uint32_t n, uint32_t m,
-                                             uint32_t fixed_low, const std::vector<uint8_t>* parametric) {
+                                             uint32_t fixed_low, const std::vector<uint8_t>* parametric,
+                                             const std::vector<uint8_t>* tc_blocks) {
     std::vector<PassSel> passes;
     uint32_t widest = 1;
     for (const Block& b : blocks) widest = std::max(widest, b.k);
@@ -383,10 +393,12 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
     std::vector<uint8_t> moves(nb, 0);
     bool mapped = false;
     for (uint32_t i = 0; i < nb; ++i) {
-        moves[i] = !(parametric != nullptr && ((*parametric)[i] & kParamBlock) != 0) && move_kind(blocks[i]) >= 0;
-        mapped = mapped || moves[i];
+        const bool move = !(parametric != nullptr && ((*parametric)[i] & kParamBlock) != 0) && move_kind(blocks[i]) >= 0;
+        moves[i] = move && tc_blocks == nullptr;
+        mapped = mapped || move;
     }
-    const Staged staged_of{mt, mapped, true};
+    const bool tc = tc_blocks != nullptr && std::find(tc_blocks->begin(), tc_blocks->end(), 0) == tc_blocks->end();
+    const Staged staged_of{mt, mapped, true, tc};
     for (uint32_t i = 0; i < nb; ++i)
         for (uint32_t t = 0; t < blocks[i].k; ++t) lists[blocks[i].q[t]].push_back(i);
     std::vector<uint32_t> head(n, 0);
@@ -645,8 +657,10 @@ TileProgram plan_tile_program(const std::vector<Block>& all, uint32_t n, uint32_
     TileProgram prog;
     const uint32_t mt = std::min(m, n);
     if (mt < kRegQubits) throw std::invalid_argument("state too small for the tile kernel");
+    if (commuting && !split)
+        for (const Block& b : all) prog.tc_blocks.push_back(tc_convertible(b));
     const std::vector<PassSel> sels =
-        commuting ? select_passes_commuting(blocks, n, mt, fixed_low, parametric)
+        commuting ? select_passes_commuting(blocks, n, mt, fixed_low, parametric, split ? nullptr : &prog.tc_blocks)
                   : select_passes(blocks, n, mt, fixed_low, parametric);
     prog.c64 = commuting;
     prog.param_offsets.assign(all.size(), 0);

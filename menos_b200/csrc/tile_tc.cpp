@@ -123,6 +123,10 @@ bool is_unitary(const Block& b) {
 
 }  // namespace
 
+// No wide dense block, and unitary (to 1e-10): a pass of such blocks preserves
+// each tile's norm, which the kernel's FP16 scaling relies on.
+bool tc_convertible(const Block& b) { return (b.diagonal || b.k <= 2) && is_unitary(b); }
+
 void tc_operands(const Cd* u, uint32_t* out) {
     auto* h = reinterpret_cast<uint16_t*>(out);  // little-endian: element k even in a word's low half
     for (uint32_t n = 0; n < 32; ++n) {
@@ -279,15 +283,9 @@ void make_tensor_core_program(TileProgram& prog, const std::vector<Block>& block
     for (size_t pi = 0; pi < prog.passes.size(); ++pi) {
         const TilePass& src = prog.passes[pi];
         const std::vector<uint32_t>& mem = members[pi];
-        // Convertible: no wide dense or parametric blocks, and every block
-        // unitary (to 1e-10): the pass then preserves each tile's norm, which
-        // the kernel's FP16 scaling relies on.
+        // Convertible: no parametric blocks, and every block a convertible one.
         bool convertible = src.param_len == 0 && !mem.empty();
-        for (uint32_t i : mem) {
-            const Block& b = blocks[i];
-            if (!b.diagonal && b.k > 2) convertible = false;
-            if (convertible && !is_unitary(b)) convertible = false;
-        }
+        for (uint32_t i : mem) convertible = convertible && prog.tc_blocks[i];
         if (!convertible) {  // kept as it is, for the FP32 SIMT kernel
             const TileInstr* ins = prog.instrs.data() + src.prog_begin;
             const double* sdata = prog.data.data() + src.sdata_begin;
