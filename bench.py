@@ -173,6 +173,9 @@ def dist_barrier(dist):
 # ----------------------------------------------------------------------------
 # CPU leg: the reference's own CPU kernels (oracle/_ref), bounded sample.
 # ----------------------------------------------------------------------------
+NO_REFERENCE = "oracle/_ref/libmenos_ref.so is not built (the reference's sources were not at hand)"
+
+
 def reference_built():
     return os.path.exists(os.path.join(ROOT, "oracle", "_ref", "libmenos_ref.so"))
 
@@ -366,7 +369,9 @@ def main():
         "gpu_launches": launches,
         "clocks": clk,
     }
-    if rank == 0 and world == 1 and not args.no_cpu_baseline and reference_built():
+    if rank == 0 and world == 1 and not args.no_cpu_baseline and not reference_built():
+        line["cpu_baseline"] = {"unavailable": NO_REFERENCE}
+    elif rank == 0 and world == 1 and not args.no_cpu_baseline:
         v, detail, cores, sampled = cpu_reference_sample(n, circ, paulis, args.shots, 1234)
         line["cpu_baseline"] = {"value": round(v, 6), "unit": UNIT, "cores": cores, "kind": "reference",
                                 "sample": f"reference CPU kernels (oracle/_ref) at {n} qubits: {sampled} gates "
@@ -813,6 +818,9 @@ def reference_gpu_job(n, circ, paulis, shots):
 
 def main_reference(args, rank, world):
     if rank != 0:
+        return
+    if not reference_built():
+        print(json.dumps({"impl": "reference", "unavailable": NO_REFERENCE}), flush=True)
         return
     if args.validate_cpu:
         return validate_cpu_baseline(args)
