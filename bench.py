@@ -308,24 +308,25 @@ def main():
                                  shots=args.shots, seed=1234, measure_targets=targets, bitstring_width=n,
                                  observable=[PauliTerm(0, 0)] + [PauliTerm(x, z) for x, z in paulis])
     st.free()
-    eng.execute(req)
+    drawn = eng.execute(req).counts
     dist_barrier(dist)
     t0 = time.perf_counter()
     for _ in range(args.steps):
         eng.execute(req)
     e2e_s = dist_max(dist, time.perf_counter() - t0)
     # The copies one execute() makes (the circuit is planned on the host and
-    # only its encoded program crosses): the tiled program, the Pauli terms'
-    # X and Z masks and the sampler's sorted uniforms in; the terms' values
-    # and each shot's basis index out.  The expectation's group tables (a
-    # few KB) are not counted.
+    # only its encoded program crosses; the shots are drawn and counted on the
+    # device): the tiled program and the Pauli terms' X and Z masks in; the
+    # terms' values and the distinct outcomes with their counts, and how many
+    # there are, out.  The expectation's group tables (a few KB) are not
+    # counted.
     arr, _keep = to_mb2_ops(circ)
     est = SweepEstimate()
     rc_est = lib().mb2_estimate_sweep(arr, len(circ.ops), C.byref(SweepOptions(1, 0, args.tile, 0, 0, args.fusion)),
                                       n, C.byref(est))
     n_terms = len(paulis) + 1
-    h2d = int(est.h2d_bytes) + 16 * n_terms + 8 * args.shots if rc_est == 0 else None
-    d2h = 16 * n_terms + 8 * args.shots
+    h2d = int(est.h2d_bytes) + 16 * n_terms if rc_est == 0 else None
+    d2h = 16 * n_terms + 16 * len(drawn) + 8
 
     passes = int(stats.passes)
     sweep_avg = statistics.median(sweep_ms)
