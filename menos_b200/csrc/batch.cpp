@@ -28,7 +28,7 @@ int launch_batch_expect(const void* amps, uint32_t n, uint64_t bindings, const u
                         const uint64_t* dev_z, const double* dev_coefs, uint32_t num_terms, double* dev_out,
                         void* stream, int precision);
 int launch_pauli_group_batch(const void* amps, uint32_t n, uint32_t c, uint32_t d, const uint64_t* dev_span,
-                             uint64_t free_mask, const void* dev_terms, uint32_t nterms, uint64_t bindings,
+                             uint64_t free_mask, const void* dev_terms, uint32_t nterms, uint32_t held, uint64_t bindings,
                              uint32_t per, double* dev_partials, int sm_count, void* stream, int precision);
 int launch_batch_group_finish(const double* dev_partials, uint64_t bindings, uint32_t per, const uint64_t* dev_x,
                               const uint64_t* dev_z, const double* dev_coefs, uint32_t num_terms, double* dev_out,
@@ -358,7 +358,7 @@ extern "C" int mb2_sweep_batch(mb2_context* ctx, const mb2_op* ops, uint32_t num
             for (const mb2::PauliGroupPlan& g : pplan.groups)
                 if (mb2::launch_pauli_group_batch(
                         r.state, num_qubits, g.c, g.d, reinterpret_cast<const uint64_t*>(w + o_sp) + g.span_off,
-                        g.free_mask, w + o_tr + size_t{g.term_off} * sizeof(mb2::PauliGroupTerm), g.nterms,
+                        g.free_mask, w + o_tr + size_t{g.term_off} * sizeof(mb2::PauliGroupTerm), g.nterms, g.held,
                         num_bindings, gper, parts, sm, r.stream, o.precision) != MB2_OK)
                     return MB2_ERR_CUDA;
             if (mb2::launch_batch_group_finish(parts, num_bindings, gper, dx, dz, dc, num_terms, dout, r.stream) !=

@@ -285,7 +285,7 @@ struct ExpectPlan {
             } else {
                 rc = mb2::launch_pauli_group(amps, n, g.c, g.d,
                                              reinterpret_cast<const uint64_t*>(base + off_s) + g.span_off, g.free_mask,
-                                             base + off_t + size_t{g.term_off} * sizeof(mb2::PauliGroupTerm), g.nterms,
+                                             base + off_t + size_t{g.term_off} * sizeof(mb2::PauliGroupTerm), g.nterms, g.held,
                                              partials, mb2::kPauliGroupBlocks, mb2::kExpBlocks, s, precision);
             }
             if (rc != MB2_OK) break;

@@ -172,8 +172,7 @@ __global__ void __launch_bounds__(kFinishThreads)
 // thread's sigma(r) of every term is a register bit mask, sigma(i << 9) a
 // per-term byte.  Each term runs a body compiled for its (own count,
 // visiting bit, mode): its products are independent and summed as a
-// balanced tree before one add into the thread's accumulator of the term
-// (in shared memory, so the term loop needs no unrolling).
+// balanced tree before one add into the thread's sum of the term.
 // Partial sums go to fixed slots (term, CTA) and are added in CTA order by
 // the finish kernel.
 using GroupTerm = PauliGroupTerm;
@@ -194,30 +193,33 @@ __device__ __forceinline__ void cp_async_amp(float2* smem, const float2* gmem) {
 }
 
 // Per-group tables in shared memory: the span, the parity of z_hi & span[k]
-// per chunk k, per term its partner offset, body, sigma(i << 8) bits and
-// high z bits, and every thread's accumulator of every term.
+// per chunk k, per term its partner offset, body, sigma(i << 9) bits and
+// high z bits.
 struct GroupShared {
     uint64_t sspan[1u << kPauliMaxSpan];
+    uint64_t off[kMaxOwn];  // state index of own amplitude i, XOR that of own amplitude 0
     uint32_t cpar[kMaxGroupTerms][kChunkWords];  // parity of z_hi & span[k], bit k
     uint32_t tdl[kMaxGroupTerms], tzl[kMaxGroupTerms], tmode[kMaxGroupTerms];
     uint32_t tcode[kMaxGroupTerms];  // the term's body (term_body)
-    // The terms in the order they are reduced, the regular ones (below) first:
-    // per place the term, what its body needs in one word -- dl, its code from
-    // bit 16 (a regular term: its mode), and from bit 24 sigma(i << kOwnShift)
+    // The terms in the order they are reduced (the places): regular pairs, Z
+    // strings with a sum in a register, other Z strings, other pairs (below).
+    // Per place the term, what its body needs in one word -- dl, its code from
+    // bit 16 (a regular pair: its mode), and from bit 24 sigma(i << kOwnShift)
     // per own amplitude i; one more to read ahead -- and its high z bits.
-    uint32_t place[kMaxGroupTerms], regular;
+    uint32_t place[kMaxGroupTerms], regular, held, zs;  // the first three kinds end there
     uint32_t tword[kMaxGroupTerms + 1];
     uint64_t pzh[32];  // zero past the terms
     uint32_t tweight[kMaxGroupTerms];  // 2: each pair visited once; 1: from both members
     uint64_t tzh[kMaxGroupTerms];
     double red[kGroupThreads / 32];
 };
-// Every thread's accumulator of every term follows the tile buffers in
-// dynamic shared memory: acc[t * kGroupThreads + thread].  Regular terms --
-// those whose pairs differ in the tile index's highest bit, in tiles of four
-// own amplitudes: nearly all, by the plan's choice of coordinates -- have
-// theirs in registers while the tiles are read, up to kRegularTerms of them.
-constexpr uint32_t kRegularTerms = 8;
+// Sums in registers while the tiles are read: up to kPauliHeldTerms terms,
+// first the regular pairs -- those whose members differ in the tile index's
+// highest bit, in tiles of four own amplitudes: nearly all, by the plan's
+// choice of coordinates -- then Z strings (pauli_can_hold).  The other terms'
+// sums, one per thread or one per pair of neighbouring threads (paired, 0 or
+// 1), follow the tile buffers in dynamic shared memory: that of the term at
+// place p at acc[((p - held) * kGroupThreads + thread) >> paired].
 
 // sigma(L): the sign parity of tile index L without the coset's part.
 __device__ __forceinline__ uint32_t group_sigma(const GroupShared& g, uint32_t t, uint32_t L, uint32_t c) {
@@ -226,16 +228,15 @@ __device__ __forceinline__ uint32_t group_sigma(const GroupShared& g, uint32_t t
 }
 
 // Term bodies: (own amplitudes, selector bit, mode).  Code = base of the
-// own count (0 for two, 5 for four) + 0 for a Z string, else
-// 1 + 2 * (selector bit + 1) + (mode - 1), the selector bit -1 meaning every
-// member visits.
+// own count (0 for two, 4 for four) + 2 * (selector bit + 1) + (mode - 1),
+// the selector bit -1 meaning every member visits; Z strings have none.
 __host__ __device__ constexpr uint32_t body_code(uint32_t own, int selb, uint32_t mode) {
-    return (own == 4 ? 5u : 0u) + (mode == 0 ? 0u : 1u + 2u * static_cast<uint32_t>(selb + 1) + (mode - 1));
+    return (own == 4 ? 4u : 0u) + 2u * static_cast<uint32_t>(selb + 1) + (mode - 1);
 }
 
 // Fills the tables and clears the accumulators; returns this thread's
 // sigma(r) of every term (bit p: the term at place p).
-__device__ __forceinline__ uint32_t group_setup(GroupShared& g, double* acc, uint32_t c, uint32_t d,
+__device__ __forceinline__ uint32_t group_setup(GroupShared& g, double* acc, uint32_t held, uint32_t paired, uint32_t c, uint32_t d,
                                                 const uint64_t* __restrict__ span,
                                                 const GroupTerm* __restrict__ terms, uint32_t nterms) {
     const uint32_t nchunks = 1u << d;
@@ -243,6 +244,10 @@ __device__ __forceinline__ uint32_t group_setup(GroupShared& g, double* acc, uin
     for (uint32_t i = threadIdx.x; i < nchunks; i += kGroupThreads) g.sspan[i] = span[i];
     if (threadIdx.x < 32) g.pzh[threadIdx.x] = 0;
     __syncthreads();
+    if (threadIdx.x < own) {
+        const uint32_t L = threadIdx.x << kOwnShift;
+        g.off[threadIdx.x] = (g.sspan[L >> c] << c) | (L & ((1u << c) - 1));
+    }
     for (uint32_t t = threadIdx.x; t < nterms; t += kGroupThreads) {
         const GroupTerm T = terms[t];
         const uint32_t dl = (T.kx << c) | T.xl;
@@ -256,10 +261,9 @@ __device__ __forceinline__ uint32_t group_setup(GroupShared& g, double* acc, uin
         // among the register index bits is clear; none there: both visit.
         const uint32_t hi = dl >> kOwnShift;
         const int selb = hi == 0 ? -1 : 31 - __clz(hi);
-        g.tcode[t] = body_code(own, mode == 0 ? -1 : selb, mode);
+        g.tcode[t] = mode == 0 ? 0u : body_code(own, selb, mode);
         g.tweight[t] = (mode != 0 && selb >= 0) ? 2u : 1u;
     }
-    for (uint32_t i = threadIdx.x; i < nterms * kGroupThreads; i += kGroupThreads) acc[i] = 0.0;
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < kMaxGroupTerms * kChunkWords; i += kGroupThreads) {
         const uint32_t t = i / kChunkWords, w = i % kChunkWords;
@@ -270,20 +274,26 @@ __device__ __forceinline__ uint32_t group_setup(GroupShared& g, double* acc, uin
         g.cpar[t][w] = bits;
     }
     __syncthreads();
-    auto is_regular = [&](uint32_t t) { return own == 4 && g.tmode[t] != 0 && (g.tdl[t] >> (kOwnShift + 1)) != 0; };
     if (threadIdx.x == 0) {
+        // Kinds: 0 regular pairs, 1 Z strings, 2 other pairs.
+        auto kind = [&](uint32_t t) {
+            return g.tmode[t] == 0 ? 1u : pauli_can_hold(false, g.tdl[t], c + d) ? 0u : 2u;
+        };
         uint32_t n = 0;
-        for (uint32_t t = 0; t < nterms && n < kRegularTerms; ++t)
-            if (is_regular(t)) g.place[n++] = t;
+        for (uint32_t t = 0; t < nterms && n < kPauliHeldTerms; ++t)
+            if (kind(t) == 0) g.place[n++] = t;
         g.regular = n;
-        uint32_t left = 0;  // regular terms past the registers' go with the others
-        for (uint32_t t = 0; t < nterms; ++t) {
-            if (is_regular(t) && left++ < kRegularTerms) continue;
-            g.place[n++] = t;
-        }
+        for (uint32_t t = 0; t < nterms; ++t)
+            if (kind(t) == 1) g.place[n++] = t;
+        g.zs = n;
+        g.held = held;
+        uint32_t past = 0;  // regular pairs past the registers' go with the others
+        for (uint32_t t = 0; t < nterms; ++t)
+            if (kind(t) == 2 || (kind(t) == 0 && past++ >= g.regular)) g.place[n++] = t;
         g.tword[nterms] = 0;
     }
     __syncthreads();
+    for (uint32_t i = threadIdx.x; i < ((nterms - held) * kGroupThreads) >> paired; i += kGroupThreads) acc[i] = 0.0;
     for (uint32_t p = threadIdx.x; p < nterms; p += kGroupThreads) {
         const uint32_t t = g.place[p];
         uint32_t bits = 0;
@@ -305,9 +315,9 @@ __device__ __forceinline__ double flip_if(double v, uint32_t f) {
 // One term's share of this thread's own amplitudes in one tile, as a
 // balanced sum in a fixed order, the second product of each pair added
 // without a rounding of its own (FMA): OWN own amplitudes, SELB the register bit
-// that marks the non-visiting member (-1: all visit), MODE 0 (|a|^2),
-// 1 (Re conj(a) b) or 2 (Im conj(a) b); sg bit i: the sign of own
-// amplitude i.  Every branch is resolved at compile time.
+// that marks the non-visiting member (-1: all visit), MODE 1 (Re conj(a) b)
+// or 2 (Im conj(a) b); sg bit i: the sign of own amplitude i.  Every branch
+// is resolved at compile time.
 template <int OWN, int SELB, int MODE, typename A>
 __device__ __forceinline__ double term_body(const double2 (&a)[kMaxOwn], const A* __restrict__ cur, uint32_t r,
                                             uint32_t dl, uint32_t sg) {
@@ -318,14 +328,9 @@ __device__ __forceinline__ double term_body(const double2 (&a)[kMaxOwn], const A
     for (int k = 0; k < NV; ++k) {
         // The k-th visiting own amplitude: k with a zero inserted at SELB.
         const int i = SELB < 0 ? k : (((k >> SB) << (SB + 1)) | (k & ((1 << SB) - 1)));
-        double x;
-        if constexpr (MODE == 0) {
-            x = __fma_rn(a[i].x, a[i].x, __dmul_rn(a[i].y, a[i].y));
-        } else {
-            const double2 b = as_d2(cur[(r | (static_cast<uint32_t>(i) << kOwnShift)) ^ dl]);
-            x = MODE == 1 ? __fma_rn(a[i].x, b.x, __dmul_rn(a[i].y, b.y))
-                          : __fma_rn(a[i].x, b.y, -__dmul_rn(a[i].y, b.x));
-        }
+        const double2 b = as_d2(cur[(r | (static_cast<uint32_t>(i) << kOwnShift)) ^ dl]);
+        const double x = MODE == 1 ? __fma_rn(a[i].x, b.x, __dmul_rn(a[i].y, b.y))
+                                   : __fma_rn(a[i].x, b.y, -__dmul_rn(a[i].y, b.x));
         v[k] = flip_if(x, (sg >> i) & 1u);
     }
 #pragma unroll
@@ -341,17 +346,26 @@ __device__ __forceinline__ double term_body(const double2 (&a)[kMaxOwn], const A
 // Bound by shared memory and issue slots: a term is its partner loads, a
 // handful of FP64 operations, and what steers them.  So the cosets' signs of
 // all terms come from one ballot per tile, a term's tables are one word, 512
-// threads own four amplitudes each (32 warps per SM hide what 16 did not), and
-// a regular term is two partner loads and eight FP64 operations without a
-// branch: the mode picks the parts that multiply the partner's by selects,
-// the signs ride on them, the sum stays in a register.  64 strings at 27
-// qubits: 7.06 ms with 256 threads, eight own amplitudes and a branch and a
-// shared-memory sum per term; 6.31 with one word per term and 512 threads;
-// 5.5 now.
+// threads own four amplitudes each (two CTAs, 32 warps, per SM hide what 16
+// did not), and a regular pair is two partner loads and eight FP64 operations
+// without a branch: the mode picks the parts that multiply the partner's by
+// selects, the signs ride on them, the sum stays in a register.
+// A Z string's signs over a thread's four amplitudes are linear in the two
+// index bits, so its sum is, up to one sign, one of four that all of them
+// share: one add a term.
+// Only the sums that no register holds take shared memory (4 KiB each): with
+// all of a 16-term group's there, one CTA fitted an SM.
+// 27 qubits, with 256 threads, eight own amplitudes, a branch and a
+// shared-memory sum per term; with 512 threads, regular pairs in registers and
+// every term's sum in shared memory; now: 64 random strings 7.06, 5.50,
+// 5.39 ms; 60 Z strings of a chain 4.13, 5.07, 2.46; 16 strings on the low
+// eight qubits, all irregular, 2.04, 2.28, 1.93.  2 random strings at 28
+// qubits, bound by the read: 0.89, 0.96, 0.90 (a third buffer in flight and
+// one barrier a tile; three instructions to an address instead of a dozen).
 template <typename A>
-__device__ __forceinline__ void group_tile(GroupShared& g, double (&reg)[kRegularTerms], double* __restrict__ acc,
+__device__ __forceinline__ void group_tile(GroupShared& g, double (&reg)[kPauliHeldTerms], double* __restrict__ acc,
                                            const A* __restrict__ cur, uint64_t rep,
-                                           uint32_t tile_amps, uint32_t nterms, uint32_t sig) {
+                                           uint32_t tile_amps, uint32_t nterms, uint32_t paired, uint32_t sig) {
     const uint32_t r = threadIdx.x;
     const uint32_t own = tile_amps >> kOwnShift;
     double2 a[kMaxOwn];
@@ -360,9 +374,9 @@ __device__ __forceinline__ void group_tile(GroupShared& g, double (&reg)[kRegula
         a[i] = i < own ? as_d2(cur[r | (i << kOwnShift)]) : make_double2(0.0, 0.0);
     // Bit p: the sign of the term at place p at this thread's first amplitude.
     const uint32_t signs = sig ^ __ballot_sync(0xffffffffu, __popcll(g.pzh[r & 31u] & rep) & 1);
-    const uint32_t regular = g.regular;
+    const uint32_t regular = g.regular, held = g.held, zs = g.zs;
 #pragma unroll
-    for (uint32_t p = 0; p < kRegularTerms; ++p) {
+    for (uint32_t p = 0; p < kPauliHeldTerms; ++p) {
         if (p >= regular) break;  // (uniform over the CTA)
         const uint32_t word = g.tword[p], s0 = signs >> p;
         const bool imag = (word >> 17) & 1u;  // mode 2
@@ -379,21 +393,25 @@ __device__ __forceinline__ void group_tile(GroupShared& g, double (&reg)[kRegula
         }
         reg[p] = __dadd_rn(reg[p], __dadd_rn(v[0], v[1]));
     }
-    uint32_t next = g.tword[regular];
-    for (uint32_t t = regular; t < nterms; ++t) {
+    // A term's sum in shared memory; paired: the two threads' shares first.
+    auto add = [&](uint32_t p, double v) {
+        if (paired) v = __dadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
+        double& sum = acc[((p - held) * kGroupThreads + r) >> paired];
+        if ((r & paired) == 0) sum = __dadd_rn(sum, v);
+    };
+    uint32_t next = g.tword[zs];
+    for (uint32_t p = zs; p < nterms; ++p) {
         const uint32_t word = next;
-        next = g.tword[t + 1];
+        next = g.tword[p + 1];
         // Bit i: the sign of own amplitude i.
-        const uint32_t sg = (word >> 24) ^ (0u - ((signs >> t) & 1u));
+        const uint32_t sg = (word >> 24) ^ (0u - ((signs >> p) & 1u));
         const uint32_t dl = word & 0xffffu;
         double v = 0.0;
         switch ((word >> 16) & 0xffu) {
-            case body_code(2, -1, 0): v = term_body<2, -1, 0>(a, cur, r, dl, sg); break;
             case body_code(2, -1, 1): v = term_body<2, -1, 1>(a, cur, r, dl, sg); break;
             case body_code(2, -1, 2): v = term_body<2, -1, 2>(a, cur, r, dl, sg); break;
             case body_code(2, 0, 1): v = term_body<2, 0, 1>(a, cur, r, dl, sg); break;
             case body_code(2, 0, 2): v = term_body<2, 0, 2>(a, cur, r, dl, sg); break;
-            case body_code(4, -1, 0): v = term_body<4, -1, 0>(a, cur, r, dl, sg); break;
             case body_code(4, -1, 1): v = term_body<4, -1, 1>(a, cur, r, dl, sg); break;
             case body_code(4, -1, 2): v = term_body<4, -1, 2>(a, cur, r, dl, sg); break;
             case body_code(4, 0, 1): v = term_body<4, 0, 1>(a, cur, r, dl, sg); break;
@@ -402,25 +420,49 @@ __device__ __forceinline__ void group_tile(GroupShared& g, double (&reg)[kRegula
             case body_code(4, 1, 2): v = term_body<4, 1, 2>(a, cur, r, dl, sg); break;
             default: break;
         }
-        acc[t * kGroupThreads + r] = __dadd_rn(acc[t * kGroupThreads + r], v);
+        add(p, v);
     }
+    if (regular == zs) return;
+    // |a|^2 of the own amplitudes, and their four sums: bit 0 of the number is
+    // the sign of amplitude 1, bit 1 that of amplitude 2, amplitude 3's follows.
+    double q[kMaxOwn];
+#pragma unroll
+    for (uint32_t i = 0; i < kMaxOwn; ++i) q[i] = __fma_rn(a[i].x, a[i].x, __dmul_rn(a[i].y, a[i].y));
+    const double e0 = __dadd_rn(q[0], q[1]), e1 = __dadd_rn(q[2], q[3]), o0 = __dsub_rn(q[0], q[1]),
+                 o1 = __dsub_rn(q[2], q[3]);
+    const double s00 = __dadd_rn(e0, e1), s01 = __dadd_rn(o0, o1), s10 = __dsub_rn(e0, e1), s11 = __dsub_rn(o0, o1);
+    auto z_sum = [&](uint32_t p) {
+        const uint32_t word = g.tword[p];
+        const double even = (word >> 26) & 1u ? s10 : s00, odd = (word >> 26) & 1u ? s11 : s01;
+        return flip_if((word >> 25) & 1u ? odd : even, (signs >> p) & 1u);
+    };
+#pragma unroll
+    for (uint32_t p = 0; p < kPauliHeldTerms; ++p) {
+        if (p >= held) break;  // (uniform over the CTA, as the next)
+        if (p >= regular) reg[p] = __dadd_rn(reg[p], z_sum(p));
+    }
+    for (uint32_t p = held; p < zs; ++p) add(p, z_sum(p));
 }
 
 // Per term: this CTA's sum in a fixed order (lanes, then warps), written to
 // slot_of(t) as (re, im) of the pair sum before the i^popcount(x & z)
 // factor, with the term's visit weight; the accumulators are cleared.
 template <typename SLOT>
-__device__ __forceinline__ void group_write(GroupShared& g, double (&reg)[kRegularTerms], double* __restrict__ acc,
-                                            const GroupTerm* __restrict__ terms, uint32_t nterms, SLOT slot_of) {
-#pragma unroll
-    for (uint32_t p = 0; p < kRegularTerms; ++p) {
-        if (p < g.regular) acc[p * kGroupThreads + threadIdx.x] = reg[p];
-        reg[p] = 0.0;
-    }
+__device__ __forceinline__ void group_write(GroupShared& g, double (&reg)[kPauliHeldTerms], double* __restrict__ acc,
+                                            const GroupTerm* __restrict__ terms, uint32_t nterms, uint32_t paired,
+                                            SLOT slot_of) {
+    const uint32_t held = g.held;
     for (uint32_t p = 0; p < nterms; ++p) {
         const uint32_t t = g.place[p];
-        double r = acc[p * kGroupThreads + threadIdx.x];
-        acc[p * kGroupThreads + threadIdx.x] = 0.0;
+        double r = 0.0;
+        if (p < held) {
+#pragma unroll
+            for (uint32_t i = 0; i < kPauliHeldTerms; ++i) r = i == p ? reg[i] : r;
+        } else if ((threadIdx.x & paired) == 0) {
+            double& sum = acc[((p - held) * kGroupThreads + threadIdx.x) >> paired];
+            r = sum;
+            sum = 0.0;
+        }
         for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
         __syncthreads();
         if ((threadIdx.x & 31) == 0) g.red[threadIdx.x >> 5] = r;
@@ -428,13 +470,15 @@ __device__ __forceinline__ void group_write(GroupShared& g, double (&reg)[kRegul
         if (threadIdx.x == 0) {
             double sum = 0.0;
             for (int w = 0; w < kGroupThreads / 32; ++w) sum += g.red[w];
-            double* p = slot_of(terms[t].out);
+            double* out = slot_of(terms[t].out);
             const uint32_t mode = g.tmode[t];
             const double w = static_cast<double>(g.tweight[t]);
-            p[0] = mode == 0 ? sum : mode == 1 ? w * sum : 0.0;
-            p[1] = mode == 2 ? -w * sum : 0.0;
+            out[0] = mode == 0 ? sum : mode == 1 ? w * sum : 0.0;
+            out[1] = mode == 2 ? -w * sum : 0.0;
         }
     }
+#pragma unroll
+    for (uint32_t i = 0; i < kPauliHeldTerms; ++i) reg[i] = 0.0;
 }
 
 // Coset representative: the coset number deposited on the free (non-pivot)
@@ -450,54 +494,67 @@ __device__ __forceinline__ uint64_t deposit_bits(uint64_t v, uint64_t mask) {
     return r;
 }
 
+// This thread's first amplitude in the coset of representative 0.  The span
+// is linear over XOR in the chunk's number, so its others, and those of other
+// cosets, are an XOR away.
+__device__ __forceinline__ uint64_t group_base(const GroupShared& g, uint32_t c) {
+    return (g.sspan[threadIdx.x >> c] << c) | (threadIdx.x & ((1u << c) - 1));
+}
+
 template <typename A>
 __device__ __forceinline__ void group_gather(const A* __restrict__ st, uint64_t rep, A* buf, const GroupShared& g,
-                                             uint32_t c, uint32_t tile_amps) {
-    const uint32_t lowmask = (1u << c) - 1;
-    for (uint32_t L = threadIdx.x; L < tile_amps; L += kGroupThreads) {
-        const uint64_t m = ((rep ^ g.sspan[L >> c]) << c) | (L & lowmask);
-        cp_async_amp(buf + L, st + m);
-    }
+                                             uint64_t base, uint32_t c, uint32_t tile_amps) {
+    const uint64_t first = base ^ (rep << c);
+#pragma unroll
+    for (uint32_t i = 0; i < kMaxOwn; ++i)
+        if ((i << kOwnShift) < tile_amps) cp_async_amp(buf + (threadIdx.x | (i << kOwnShift)), st + (first ^ g.off[i]));
     asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
-// Cosets are processed with two shared-memory buffers: the next coset's
-// amplitudes are gathered with cp.async while this one is reduced.
+// Cosets are processed with `stages` (two or three) shared-memory buffers: the
+// amplitudes of the stages - 1 cosets ahead are gathered with cp.async while
+// this one is reduced.
 template <typename A>
 __global__ void __launch_bounds__(kGroupThreads, 2)
     k_pauli_group(const A* __restrict__ st, uint32_t c, uint32_t d, const uint64_t* __restrict__ span,
-                  uint64_t free_mask, const GroupTerm* __restrict__ terms, uint32_t nterms, uint64_t ncosets,
+                  uint64_t free_mask, const GroupTerm* __restrict__ terms, uint32_t nterms, uint32_t held, uint32_t paired, uint32_t stages, uint64_t ncosets,
                   uint32_t pitch, double* __restrict__ partials) {
     extern __shared__ __align__(16) unsigned char gsm[];
     __shared__ GroupShared g;
     const uint32_t tile_amps = 1u << (c + d);
-    A* buf0 = reinterpret_cast<A*>(gsm);
-    A* buf1 = buf0 + tile_amps;
-    double* acc = reinterpret_cast<double*>(buf1 + tile_amps);
-    const uint32_t sig = group_setup(g, acc, c, d, span, terms, nterms);
-    double reg[kRegularTerms] = {};
+    A* const tiles = reinterpret_cast<A*>(gsm);
+    double* acc = reinterpret_cast<double*>(tiles + stages * tile_amps);
+    const uint32_t sig = group_setup(g, acc, held, paired, c, d, span, terms, nterms);
+    const uint64_t base = group_base(g, c);
+    double reg[kPauliHeldTerms] = {};
     // Moving gridDim.x cosets on is a masked add on the free bits.
     const uint64_t rstep = deposit_bits(gridDim.x, free_mask);
     auto advance = [&](uint64_t r) { return ((r | ~free_mask) + rstep) & free_mask; };
-    uint64_t rep = deposit_bits(blockIdx.x, free_mask);
-    if (blockIdx.x < ncosets) group_gather(st, rep, buf0, g, c, tile_amps);
-    A* cur = buf0;
-    A* nxt = buf1;
-    for (uint64_t cs = blockIdx.x; cs < ncosets; cs += gridDim.x) {
-        const uint64_t rep_next = advance(rep);
-        if (cs + gridDim.x < ncosets) group_gather(st, rep_next, nxt, g, c, tile_amps);
+    uint64_t rep = deposit_bits(blockIdx.x, free_mask), ahead = rep;  // of the tile reduced, of the one gathered
+    uint64_t at = blockIdx.x;                                         // the latter's number
+    uint32_t fill = 0, cur = 0;                                       // their buffers
+    auto gather = [&]() {  // (an empty group past the end keeps the count)
+        if (at < ncosets) group_gather(st, ahead, tiles + fill * tile_amps, g, base, c, tile_amps);
         else asm volatile("cp.async.commit_group;\n" ::: "memory");
+        ahead = advance(ahead);
+        at += gridDim.x;
+        fill = fill + 1 == stages ? 0 : fill + 1;
+    };
+    for (uint32_t i = 0; i + 1 < stages; ++i) gather();
+    for (uint64_t cs = blockIdx.x; cs < ncosets; cs += gridDim.x) {
+        // The buffer that is filled now was reduced from in the round before: with
+        // three, every thread is past that at this round's barrier.
+        if (stages == 2) gather();
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         __syncthreads();
-        group_tile(g, reg, acc, cur, rep, tile_amps, nterms, sig);
-        __syncthreads();  // this buffer is the target of the gather after next
-        rep = rep_next;
-        A* tmp = cur;
-        cur = nxt;
-        nxt = tmp;
+        if (stages == 3) gather();
+        group_tile(g, reg, acc, tiles + cur * tile_amps, rep, tile_amps, nterms, paired, sig);
+        if (stages == 2) __syncthreads();
+        rep = advance(rep);
+        cur = cur + 1 == stages ? 0 : cur + 1;
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    group_write(g, reg, acc, terms, nterms, [&](uint32_t out) {
+    group_write(g, reg, acc, terms, nterms, paired, [&](uint32_t out) {
         return partials + 2 * (static_cast<uint64_t>(out) * pitch + blockIdx.x);
     });
 }
@@ -512,15 +569,16 @@ template <typename A>
 __global__ void __launch_bounds__(kGroupThreads, 2)
     k_pauli_group_batch(const A* __restrict__ st, uint32_t n, uint32_t c, uint32_t d,
                         const uint64_t* __restrict__ span, uint64_t free_mask, const GroupTerm* __restrict__ terms,
-                        uint32_t nterms, uint64_t bindings, uint32_t per, double* __restrict__ partials) {
+                        uint32_t nterms, uint32_t held, uint32_t paired, uint64_t bindings, uint32_t per,
+                        double* __restrict__ partials) {
     extern __shared__ __align__(16) unsigned char gsm[];
     __shared__ GroupShared g;
     const uint32_t tile_amps = 1u << (c + d);
     A* buf0 = reinterpret_cast<A*>(gsm);
     A* buf1 = buf0 + tile_amps;
     double* acc = reinterpret_cast<double*>(buf1 + tile_amps);
-    const uint32_t sig = group_setup(g, acc, c, d, span, terms, nterms);
-    double reg[kRegularTerms] = {};
+    const uint32_t sig = group_setup(g, acc, held, paired, c, d, span, terms, nterms);
+    double reg[kPauliHeldTerms] = {};
     const uint64_t ncosets = uint64_t{1} << (n - c - d);
     const uint32_t slot = blockIdx.x % per;
     const uint64_t b0 = blockIdx.x / per, bstep = gridDim.x / per;
@@ -530,7 +588,7 @@ __global__ void __launch_bounds__(kGroupThreads, 2)
     const uint64_t mine = ncosets > slot ? (ncosets - slot + per - 1) / per : 0;
     const uint64_t nb = (bindings - b0 + bstep - 1) / bstep;
     auto write = [&](uint64_t b) {
-        group_write(g, reg, acc, terms, nterms, [&](uint32_t out) {
+        group_write(g, reg, acc, terms, nterms, paired, [&](uint32_t out) {
             return partials + 2 * ((static_cast<uint64_t>(out) * bindings + b) * per + slot);
         });
     };
@@ -545,20 +603,21 @@ __global__ void __launch_bounds__(kGroupThreads, 2)
     };
     uint64_t b = 0, rep = 0;
     item(0, b, rep);
-    group_gather(st + (b << n), rep, buf0, g, c, tile_amps);
+    const uint64_t base = group_base(g, c);
+    group_gather(st + (b << n), rep, buf0, g, base, c, tile_amps);
     A* cur = buf0;
     A* nxt = buf1;
     for (uint64_t f = 0; f < items; ++f) {
         uint64_t bn = 0, repn = 0;
         if (f + 1 < items) {
             item(f + 1, bn, repn);
-            group_gather(st + (bn << n), repn, nxt, g, c, tile_amps);
+            group_gather(st + (bn << n), repn, nxt, g, base, c, tile_amps);
         } else {
             asm volatile("cp.async.commit_group;\n" ::: "memory");
         }
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         __syncthreads();
-        group_tile(g, reg, acc, cur, rep, tile_amps, nterms, sig);
+        group_tile(g, reg, acc, cur, rep, tile_amps, nterms, paired, sig);
         __syncthreads();  // this buffer is the target of the gather after next
         if ((f + 1) % mine == 0) write(b);
         b = bn;
@@ -594,22 +653,33 @@ __global__ void k_batch_group_finish(const double* __restrict__ partials, uint64
 
 }  // namespace
 
-// Dynamic shared memory of a group: two tile buffers and the accumulators.
-static size_t group_smem(uint32_t tile_qubits, uint32_t nterms, int precision) {
-    return 2 * (size_t{1} << tile_qubits) * (precision == MB2_C64 ? sizeof(float2) : sizeof(double2)) +
-           size_t{nterms} * kGroupThreads * sizeof(double);
-}
+// The shared memory of a group that lets two CTAs share an SM: of its tile
+// buffers, and of the sums that no register holds.  Three buffers where they
+// leave room for that (at most `most`); where one sum for each thread does
+// not, one for each pair of threads (paired).
+struct GroupMemory {
+    uint32_t stages, paired;
+    size_t bytes;
+    GroupMemory(uint32_t most, uint32_t tile_qubits, uint32_t nterms, uint32_t held, int precision) {
+        const size_t tile = (size_t{1} << tile_qubits) * (precision == MB2_C64 ? sizeof(float2) : sizeof(double2));
+        const size_t sums = size_t{nterms - held} * kGroupThreads * sizeof(double);
+        auto two_fit = [](size_t dynamic) { return 2 * (dynamic + sizeof(GroupShared) + 1024) <= kSmemPerSm; };
+        stages = most == 3 && two_fit(3 * tile + sums) ? 3 : 2;
+        paired = two_fit(stages * tile + sums) ? 0 : 1;
+        bytes = stages * tile + (sums >> paired);
+    }
+};
 
 int launch_pauli_group(const void* amps, uint32_t n, uint32_t c, uint32_t d, const uint64_t* dev_span,
-                       uint64_t free_mask, const void* dev_terms, uint32_t nterms, double* dev_partials,
+                       uint64_t free_mask, const void* dev_terms, uint32_t nterms, uint32_t held, double* dev_partials,
                        uint32_t grid, uint32_t pitch, void* stream, int precision) {
     if (nterms == 0) return MB2_OK;
-    if (nterms > kMaxGroupTerms || c + d > kPauliTileQubits || d > kPauliMaxSpan) return MB2_ERR_INVALID;
+    if (nterms > kMaxGroupTerms || held > nterms || c + d > kPauliTileQubits || d > kPauliMaxSpan) return MB2_ERR_INVALID;
     const auto s = static_cast<cudaStream_t>(stream);
     const uint64_t ncosets = uint64_t{1} << (n - c - d);
     // Two buffers of 2^(c+d) amplitudes, of which each thread owns two or four.
     if (c + d < kPauliMinTileQubits || grid > pitch) return MB2_ERR_INVALID;
-    const size_t smem = group_smem(c + d, nterms, precision);
+    const GroupMemory mem(3, c + d, nterms, held, precision);
     static const bool attr = [] {  // once, thread-safe (concurrent callers wait for it)
         return cudaFuncSetAttribute(k_pauli_group<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     128 * 1024) == cudaSuccess &&
@@ -619,23 +689,23 @@ int launch_pauli_group(const void* amps, uint32_t n, uint32_t c, uint32_t d, con
     if (!attr) return launch_status();
     const auto* terms = static_cast<const GroupTerm*>(dev_terms);
     if (precision == MB2_C64)
-        k_pauli_group<float2><<<grid, kGroupThreads, smem, s>>>(static_cast<const float2*>(amps), c, d, dev_span,
-                                                           free_mask, terms, nterms, ncosets, pitch, dev_partials);
+        k_pauli_group<float2><<<grid, kGroupThreads, mem.bytes, s>>>(static_cast<const float2*>(amps), c, d, dev_span,
+                                                           free_mask, terms, nterms, held, mem.paired, mem.stages, ncosets, pitch, dev_partials);
     else
-        k_pauli_group<double2><<<grid, kGroupThreads, smem, s>>>(static_cast<const double2*>(amps), c, d, dev_span,
-                                                            free_mask, terms, nterms, ncosets, pitch, dev_partials);
+        k_pauli_group<double2><<<grid, kGroupThreads, mem.bytes, s>>>(static_cast<const double2*>(amps), c, d, dev_span,
+                                                            free_mask, terms, nterms, held, mem.paired, mem.stages, ncosets, pitch, dev_partials);
     note_launches(1);
     return launch_status();
 }
 
 int launch_pauli_group_batch(const void* amps, uint32_t n, uint32_t c, uint32_t d, const uint64_t* dev_span,
-                             uint64_t free_mask, const void* dev_terms, uint32_t nterms, uint64_t bindings,
+                             uint64_t free_mask, const void* dev_terms, uint32_t nterms, uint32_t held, uint64_t bindings,
                              uint32_t per, double* dev_partials, int sm_count, void* stream, int precision) {
     if (nterms == 0) return MB2_OK;
-    if (nterms > kMaxGroupTerms || c + d > kPauliTileQubits || d > kPauliMaxSpan || c + d > n || per == 0 ||
+    if (nterms > kMaxGroupTerms || held > nterms || c + d > kPauliTileQubits || d > kPauliMaxSpan || c + d > n || per == 0 ||
         c + d < kPauliMinTileQubits)
         return MB2_ERR_INVALID;
-    const size_t smem = group_smem(c + d, nterms, precision);
+    const GroupMemory mem(2, c + d, nterms, held, precision);
     static const bool attr = [] {  // once, thread-safe
         return cudaFuncSetAttribute(k_pauli_group_batch<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     128 * 1024) == cudaSuccess &&
@@ -650,11 +720,11 @@ int launch_pauli_group_batch(const void* amps, uint32_t n, uint32_t c, uint32_t 
     const auto s = static_cast<cudaStream_t>(stream);
     const auto* terms = static_cast<const GroupTerm*>(dev_terms);
     if (precision == MB2_C64)
-        k_pauli_group_batch<float2><<<grid, kGroupThreads, smem, s>>>(static_cast<const float2*>(amps), n, c, d, dev_span,
-                                                                 free_mask, terms, nterms, bindings, per, dev_partials);
+        k_pauli_group_batch<float2><<<grid, kGroupThreads, mem.bytes, s>>>(static_cast<const float2*>(amps), n, c, d, dev_span,
+                                                                 free_mask, terms, nterms, held, mem.paired, bindings, per, dev_partials);
     else
-        k_pauli_group_batch<double2><<<grid, kGroupThreads, smem, s>>>(static_cast<const double2*>(amps), n, c, d,
-                                                                  dev_span, free_mask, terms, nterms, bindings, per,
+        k_pauli_group_batch<double2><<<grid, kGroupThreads, mem.bytes, s>>>(static_cast<const double2*>(amps), n, c, d,
+                                                                  dev_span, free_mask, terms, nterms, held, mem.paired, bindings, per,
                                                                   dev_partials);
     note_launches(1);
     return launch_status();

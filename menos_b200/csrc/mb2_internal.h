@@ -552,6 +552,13 @@ constexpr uint32_t kMaxGroupTerms = 16;
 constexpr uint32_t kPauliTileQubits = 11;
 constexpr uint32_t kPauliMinTileQubits = 10;  // smaller states: one streaming pass per term
 constexpr uint32_t kPauliMaxSpan = 8;
+// The terms whose sums registers hold, at most kPauliHeldTerms of a group's: Z
+// strings, and pairs (tile indexes dl apart) that differ in the highest bit of
+// a full tile's index.
+constexpr uint32_t kPauliHeldTerms = 8;
+MB2_HD inline constexpr bool pauli_can_hold(bool z_string, uint32_t dl, uint32_t tile_qubits) {
+    return z_string || (tile_qubits == kPauliTileQubits && (dl >> (kPauliTileQubits - 1)) != 0);
+}
 struct PauliGroupTerm {
     uint64_t x, z;
     uint32_t kx;   // coordinates of x >> c in the group's basis
@@ -563,6 +570,7 @@ struct PauliGroupPlan {
     uint32_t c = 0, d = 0;
     uint64_t free_mask = 0;  // high bits (above c) that index the cosets
     uint32_t span_off = 0, term_off = 0, nterms = 0;
+    uint32_t held = 0;  // terms whose sums the kernel keeps in registers
 };
 struct PauliPlan {
     std::vector<PauliGroupPlan> groups;
@@ -571,7 +579,7 @@ struct PauliPlan {
 };
 PauliPlan plan_pauli_groups(const uint64_t* x, const uint64_t* z, uint32_t num_terms, uint32_t n);
 int launch_pauli_group(const void* amps, uint32_t n, uint32_t c, uint32_t d, const uint64_t* dev_span,
-                       uint64_t free_mask, const void* dev_terms, uint32_t nterms, double* dev_partials,
+                       uint64_t free_mask, const void* dev_terms, uint32_t nterms, uint32_t held, double* dev_partials,
                        uint32_t grid, uint32_t pitch, void* stream, int precision);
 // One streaming pass per term (partials only), for terms that share no read.
 int launch_expectation_partials(const void* amps, uint32_t n, const uint64_t* dev_x, const uint64_t* dev_z,

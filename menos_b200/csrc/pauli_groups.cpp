@@ -154,6 +154,7 @@ PauliPlan plan_pauli_groups(const uint64_t* x, const uint64_t* z, uint32_t num_t
             pt.xl = static_cast<uint32_t>(x[t] & ((uint64_t{1} << c) - 1));
             pt.out = t;
             plan.terms.push_back(pt);
+            if (gp.held < kPauliHeldTerms && pauli_can_hold(pt.x == 0, (pt.kx << c) | pt.xl, c + gp.d)) ++gp.held;
         }
         plan.groups.push_back(gp);
     }
