@@ -371,6 +371,17 @@ int mb2_trajectories_monitored(mb2_context* ctx, uint32_t num_qubits, const mb2_
                                double* standard_error, uint64_t shots, const uint32_t* targets,
                                uint32_t num_targets, uint64_t* outcomes, uint64_t* counts, uint64_t* num_outcomes,
                                mb2_boundary_fn boundary, void* user);
+/* How many trajectories such a run holds on the device at once, and the bytes
+ * it takes there at most: their states (one more while they are allocated),
+ * draws, values and the kernels' scratch.  monitored: whether a boundary is
+ * given.  A device that refuses that much is asked for one trajectory's share
+ * (as monitored).  Has no counterpart in the reference. */
+int mb2_trajectories_bytes(uint32_t num_qubits, const mb2_op* ops, uint32_t num_ops, uint64_t trajectories,
+                           uint32_t num_terms, int32_t monitored, uint64_t* batch, uint64_t* bytes);
+/* The device bytes that drawing and counting `shots` shots take beside the
+ * state and the walk's scratch (mb2_sample, mb2_dm_sample); 16 bytes a shot
+ * where the device refuses that much.  Has no counterpart in the reference. */
+uint64_t mb2_draw_bytes(uint64_t shots);
 
 /* ---- batched parameter sweep ------------------------------------------- */
 /* One circuit structure under many parameter bindings, in one device job:

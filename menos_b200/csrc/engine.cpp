@@ -300,27 +300,37 @@ struct ExpectPlan {
 }  // namespace
 
 namespace mb2 {
+namespace {
+uint64_t up256(uint64_t v) { return (v + 255) & ~uint64_t{255}; }
+
+// A gate's share of a tiled program, at most: a phase record and a store
+// record of a mapped tile, a few gate words and pass padding (432 bytes) and
+// its matrix (16 * 4^k, staged or global-only); blocks never outnumber gates.
+uint64_t program_bound(const mb2_op& gate) { return 432 + (16ull << (2 * gate.num_qubits)); }
+
+// Drawing and counting shots (device_counts): uniforms, per-shot basis states,
+// and the sort's scratch or the counts'.
+uint64_t draw_bytes(uint64_t shots) {
+    return 2 * up256(8 * shots) +
+           std::max<uint64_t>(uniforms_scratch_bytes(shots), up256(8 * shots) + runs_scratch_bytes(shots));
+}
+
+// ExpectPlan's bytes, at most: masks, partials, results, the groups' span
+// vectors (at most 2^kPauliMaxSpan per group) and terms.
+uint64_t expect_bound(uint64_t terms) {
+    return terms == 0 ? 0
+                      : 2 * up256(8 * terms) + up256(16 * kExpBlocks * terms + 16 * terms) +
+                            up256(8 * terms << kPauliMaxSpan) + sizeof(PauliGroupTerm) * terms;
+}
+}  // namespace
+
 uint64_t scratch_bound(uint32_t n, const mb2_op* ops, uint32_t num_ops, uint64_t shots, uint32_t terms) {
-    auto up = [](uint64_t v) { return (v + 255) & ~uint64_t{255}; };
-    // The sweep's upload (mb2_apply_program_monitored): per block at most a
-    // phase record and a store record of a mapped tile, a few gate words and
-    // pass padding (432 bytes) and its matrix (16 * 4^k, staged or
-    // global-only); blocks never outnumber ops.
+    // The sweep's upload (mb2_apply_program_monitored).
     uint64_t program = 4 * 256;
     for (uint32_t i = 0; i < num_ops; ++i)
-        if (ops[i].opcode != MB2_MEASURE) program += 432 + (16ull << (2 * ops[i].num_qubits));
-    // The sampler (device_counts): uniforms, per-shot basis, the walk's
-    // scratch, and the sort's or the counts'.
-    const uint64_t sample =
-        shots == 0 ? 0
-                   : 2 * up(8 * shots) + sample_scratch_bytes(n, shots) +
-                         std::max<uint64_t>(uniforms_scratch_bytes(shots), up(8 * shots) + runs_scratch_bytes(shots));
-    // The expectation (mb2_expectation): masks, partials, results, the
-    // groups' span vectors (at most 2^kPauliMaxSpan per group) and terms.
-    const uint64_t t = terms;
-    const uint64_t expect = terms == 0 ? 0
-                                       : 2 * up(8 * t) + up(16 * kExpBlocks * t + 16 * t) +
-                                             up(8 * t << kPauliMaxSpan) + sizeof(PauliGroupTerm) * t;
+        if (ops[i].opcode != MB2_MEASURE) program += program_bound(ops[i]);
+    const uint64_t sample = shots == 0 ? 0 : draw_bytes(shots) + sample_scratch_bytes(n, shots);
+    const uint64_t expect = expect_bound(terms);
     const uint64_t need = std::max({program, sample, expect});
     uint64_t rounded = uint64_t{1} << 20;  // ensure_scratch's power-of-two growth
     while (rounded < need) rounded <<= 1;
@@ -1208,10 +1218,9 @@ int device_counts(mb2_state* s, uint32_t n, uint64_t shots, uint64_t seed, const
                   size_t walk_bytes, WALK walk) {
     if (shots > uint64_t{1} << 40) return fail(s->ctx, MB2_ERR_RESOURCE, "too many shots");
     const size_t al_u = (shots * 8 + 255) & ~size_t{255};
-    const size_t other = std::max(mb2::uniforms_scratch_bytes(shots), al_u + mb2::runs_scratch_bytes(shots));
     // Where the device has no room for the sort (a state that nearly fills
     // it), the uniforms are sorted and the outcomes counted on the host.
-    const int room = ensure_scratch(s, 2 * al_u + walk_bytes + other);
+    const int room = ensure_scratch(s, walk_bytes + mb2::draw_bytes(shots));
     if (room != MB2_OK && room != MB2_ERR_RESOURCE) return room;
     const bool on_device = room == MB2_OK;
     if (!on_device)
@@ -1628,6 +1637,32 @@ int mb2_trajectories(mb2_context* ctx, uint32_t n, const mb2_op* ops, uint32_t n
                                       term_means, standard_error, shots, targets, num_targets, outcomes, counts,
                                       num_outcomes, nullptr, nullptr);
 }
+
+int mb2_trajectories_bytes(uint32_t n, const mb2_op* ops, uint32_t num_ops, uint64_t trajectories, uint32_t num_terms,
+                           int32_t monitored, uint64_t* batch, uint64_t* bytes) {
+    if (n < 1 || n > 34 || (ops == nullptr && num_ops != 0) || trajectories == 0 || batch == nullptr || bytes == nullptr)
+        return MB2_ERR_INVALID;
+    // What the plan uploads, at most: each run of gates a program of its own in
+    // three parts, each channel its operators and their products.
+    uint64_t upload = 0, channels = 0;
+    for (uint32_t i = 0; i < num_ops; ++i) {
+        if (ops[i].opcode == MB2_MEASURE) continue;
+        if (ops[i].num_qubits > MB2_MAX_OP_QUBITS) return MB2_ERR_INVALID;
+        if (ops[i].opcode == MB2_CHANNEL) {
+            upload += 2 * mb2::up256(uint64_t{ops[i].reserved} * (16ull << (2 * ops[i].num_qubits)));
+            ++channels;
+        } else {
+            upload += 3 * 256 + mb2::program_bound(ops[i]);
+        }
+    }
+    *batch = trajectory_batch(n, trajectories, monitored != 0);
+    const uint64_t states = *batch + (*batch > 1 ? 1 : 0);  // the one state is held until the batch's are
+    *bytes = states * (uint64_t{16} << n) +
+             TrajLayout(n, *batch, channels, num_terms, upload, mb2::expect_bound(num_terms)).bytes;
+    return MB2_OK;
+}
+
+uint64_t mb2_draw_bytes(uint64_t shots) { return shots == 0 ? 0 : mb2::draw_bytes(shots); }
 
 int mb2_trajectories_monitored(mb2_context* ctx, uint32_t n, const mb2_op* ops, uint32_t num_ops,
                                uint64_t trajectories, uint64_t seed, const uint64_t* x_masks,

@@ -431,8 +431,9 @@ private:
                          DeviceCost{device_bytes, e.h2d_bytes, d2h, launches}};
         // Host work in the CPU dense engine's time components, as the
         // reference's CUDA estimate reports it: the passes the host prepares
-        // (plan and block build per pass) and, for counts, the per-shot
-        // uniforms (the walk itself runs on the device).
+        // (plan and block build per pass) and, for counts, the shots (counted
+        // on the host unless every qubit is read into its own clbit; drawn and
+        // walked on the device).
         auto& dense = est.time.counts[static_cast<std::size_t>(Engine::Dense)];
         dense[0] = static_cast<double>(e.passes + 1);
         if (request.want_counts) dense[2] = static_cast<double>(request.shots);

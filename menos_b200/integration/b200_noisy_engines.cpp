@@ -298,8 +298,12 @@ public:
             launches += 2;
             d2h += 16 * terms;
         }
-        const uint64_t device_bytes = 16 * pow2(2 * n) + (uint64_t{1} << 20) + 16 * request.shots + h2d;
-        if (device_bytes > free_device_bytes())
+        // Drawing and counting on the device, or where there is no room for
+        // that the walk's 16 bytes a shot.
+        const uint64_t free_bytes = free_device_bytes(), base = 16 * pow2(2 * n) + (uint64_t{1} << 20) + h2d;
+        uint64_t device_bytes = base + (request.want_counts ? mb2_draw_bytes(request.shots) : 16 * request.shots);
+        if (device_bytes > free_bytes) device_bytes = base + 16 * request.shots;
+        if (device_bytes > free_bytes)
             return CostEstimate{false, 0, 0, "density_matrix_b200 needs " + std::to_string(device_bytes) +
                                                  " device bytes", {}};
         CostEstimate est{true, host, work, "", DeviceCost{device_bytes, h2d, d2h, launches}};
@@ -372,6 +376,28 @@ public:
     }
 };
 
+// The first MiB beside a state is nobody's charge: every state has that much
+// staging (masks, partial sums, encoded programs).
+constexpr uint64_t kUnchargedBytes = uint64_t{1} << 20;
+
+// What a trajectory run holds on the device: mb2_trajectories runs them in
+// batches, whose states and scratch are far more than one state where a state
+// is small.
+struct TrajectoryRun {
+    uint64_t batch, state_bytes, bytes;
+    [[nodiscard]] uint64_t charge() const {
+        return std::max(state_bytes, bytes > kUnchargedBytes ? bytes - kUnchargedBytes : 0);
+    }
+};
+
+TrajectoryRun trajectory_run(uint32_t n, const Ops& ops, uint64_t trajectories, uint64_t terms, bool monitored) {
+    TrajectoryRun run{1, 16 * pow2(n), 0};
+    check(mb2_trajectories_bytes(n, ops.ops.data(), static_cast<uint32_t>(ops.ops.size()), trajectories,
+                                 static_cast<uint32_t>(terms), monitored ? 1 : 0, &run.batch, &run.bytes),
+          "trajectory bytes");
+    return run;
+}
+
 class B200TrajectoryEngine : public SimulationEngine {
 public:
     [[nodiscard]] std::string_view name() const override { return "trajectory_b200"; }
@@ -407,18 +433,28 @@ public:
             passes += channel ? 2.0 : 1.0;
             per += pow2(static_cast<uint32_t>(n + k));
             if (channel) per += pow2(static_cast<uint32_t>(n + k)) + states;
-            launches += channel ? 5 : 1;
+            launches += channel ? (n <= 12 ? 4 : 8) : 1;
         }
         const uint64_t terms = request.want_expectation ? request.observable->terms.size() : 0;
         per += terms * states;
         uint64_t work = request.trajectories * per;
         if (request.want_counts) work += request.trajectories * states;
-        const uint64_t device_bytes = 16 * states + (uint64_t{1} << 20);
-        if (device_bytes > free_device_bytes())
+        // A batch of trajectories, or where there is no room for one, one at a
+        // time.
+        const Ops ops = to_mb2(*request.operations);
+        const uint64_t free_bytes = free_device_bytes();
+        TrajectoryRun run = trajectory_run(n, ops, request.trajectories, terms, false);
+        if (run.charge() + kUnchargedBytes > free_bytes) run = TrajectoryRun{1, 16 * states, 0};
+        const uint64_t device_bytes = run.charge() + kUnchargedBytes;
+        if (device_bytes > free_bytes)
             return CostEstimate{false, 0, 0, "trajectory_b200 needs " + std::to_string(device_bytes) + " device bytes",
                                 {}};
+        // Every launch but the terms' and the shots' serves a whole batch.
+        const uint64_t batches = (request.trajectories + run.batch - 1) / run.batch;
+        const uint64_t outputs = (terms != 0 ? 2 : 0) + (request.want_counts ? 5 : 0);
         CostEstimate est{true, 16 * request.shots, work, "",
-                         DeviceCost{device_bytes, 0, 16 * (terms + request.shots), request.trajectories * launches}};
+                         DeviceCost{device_bytes, 0, 16 * (terms + request.shots),
+                                    batches * launches + request.trajectories * outputs}};
         auto& tr = est.time.counts[static_cast<std::size_t>(Engine::Trajectory)];
         tr[0] = static_cast<double>(request.trajectories) * passes;
         tr[1] = static_cast<double>(work);
@@ -455,8 +491,9 @@ public:
         double standard_error = 0.0;
         std::vector<uint64_t> outcomes(std::max<uint64_t>(shots, 1)), counts(outcomes.size());
         uint64_t distinct = outcomes.size();
-        // The state the run holds on the device, charged to the Device space.
-        const common::MemoryLedger::Charge charge(16 * pow2(n), common::MemoryLedger::Space::Device);
+        // What the run holds on the device, charged to the Device space.
+        const uint64_t held = trajectory_run(n, ops, trajectories, num_terms, request.monitor != nullptr).charge();
+        const common::MemoryLedger::Charge charge(held, common::MemoryLedger::Space::Device);
         MonitorBridge bridge{request.monitor, nullptr};
         const int rc = mb2_trajectories_monitored(
             b200_context(), n, ops.ops.data(), static_cast<uint32_t>(ops.ops.size()), trajectories, request.seed,
@@ -469,7 +506,7 @@ public:
         check(rc, "trajectories");
         EngineExecutionResult result;
         result.statistical = true;
-        result.actual_bytes = 16 * pow2(n);
+        result.actual_bytes = held;
         if (request.want_counts) result.counts = histogram(outcomes, counts, shots == 0 ? 0 : distinct,
                                                            request.bitstring_width);
         if (request.want_expectation) {
