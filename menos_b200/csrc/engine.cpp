@@ -2220,11 +2220,11 @@ int mb2_debug_schedule(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_opti
     try {
         blocks = mb2::build_blocks(ops, num_ops, o.fuse_gates != 0, static_cast<uint32_t>(o.fusion_width));
         uint32_t m = tile_width(o.tile_qubits > 0 ? static_cast<uint32_t>(o.tile_qubits) : 0, num_qubits, blocks);
+        bool tc = false;
         if (c64) {
-            m = o.tile_qubits > 0 ? std::min<uint32_t>(static_cast<uint32_t>(o.tile_qubits), mb2::kMaxTileQubitsC64)
-                                  : std::min<uint32_t>(mb2::kDefaultTileQubitsC64, num_qubits);
-            for (const mb2::Block& b : blocks) m = std::max(m, b.k);
-            m = std::max(m, mb2::kMinTileQubits);
+            const C64Choice ch = c64_choice(o, num_qubits, mb2::kDefaultTileQubitsC64, blocks);
+            m = ch.m;
+            tc = ch.tc;
         }
         if ((!c64 && o.per_gate != 0) || num_qubits < mb2::kMinTileQubits || blocks.empty()) {
             for (uint32_t i = 0; i < blocks.size(); ++i) {
@@ -2234,7 +2234,7 @@ int mb2_debug_schedule(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_opti
         } else {
             const uint32_t low = o.low_qubits < 0 ? 0u : (o.low_qubits == 0 ? mb2::kDefaultFixedLow
                                                                              : static_cast<uint32_t>(o.low_qubits));
-            const mb2::TileProgram prog = mb2::plan_tile_program(blocks, num_qubits, m, low, nullptr, c64);
+            const mb2::TileProgram prog = mb2::plan_tile_program(blocks, num_qubits, m, low, nullptr, c64, !tc);
             order = prog.order;
             order_pass = prog.order_pass;
         }
@@ -2352,20 +2352,42 @@ int measure_costs(mb2_state* st, mb2_state* small, uint32_t m, double* fixed, do
     return MB2_OK;
 }
 
-// Seconds for one pass of blocks [b0, b1) over 2^n amplitudes: the fixed
-// cost, the memory time and the blocks' compute, added -- a pass with dense
-// blocks is bound by FP64 latency at the resident warps, so its loads and
-// stores overlap its arithmetic only in part (measured: a 28-qubit brick pass
-// of 8 U3s takes about its DRAM time plus its FP64 time at the measured rate).
-double pass_seconds(const mb2_tuning& t, bool c64, const std::vector<mb2::Block>& blocks, size_t b0, size_t b1,
-                    uint32_t n) {
+// Seconds for one pass over 2^n amplitudes whose compute is worth `dense1`
+// dense one-qubit blocks and `diag` diagonals: the fixed cost, the memory time
+// and the compute, added -- a pass with dense blocks is bound by FP64 latency
+// at the resident warps, so its loads and stores overlap its arithmetic only
+// in part (measured: a 28-qubit brick pass of 8 U3s takes about its DRAM time
+// plus its FP64 time at the measured rate).
+struct PassCompute {
+    double dense1 = 0.0, diag = 0.0;
+};
+double pass_seconds(const mb2_tuning& t, bool c64, const PassCompute& work, uint32_t n) {
     const double mem = c64 ? t.pass_s_per_amp_c64 : t.pass_s_per_amp;
-    const double dense1 = c64 ? t.dense1_s_per_amp_c64 : t.dense1_s_per_amp;
-    const double diag = c64 ? t.diag_s_per_amp_c64 : t.diag_s_per_amp;
-    double compute = 0.0;
-    for (size_t i = b0; i < b1; ++i)  // a dense k-qubit block sums 2^k terms per amplitude
-        compute += blocks[i].diagonal ? diag : dense1 * static_cast<double>(uint64_t{1} << (blocks[i].k - 1));
+    const double compute = work.dense1 * (c64 ? t.dense1_s_per_amp_c64 : t.dense1_s_per_amp) +
+                           work.diag * (c64 ? t.diag_s_per_amp_c64 : t.diag_s_per_amp);
     return (c64 ? t.pass_s_fixed_c64 : t.pass_s_fixed) + (mem + compute) * static_cast<double>(uint64_t{1} << n);
+}
+
+// A block by itself: a dense k-qubit block sums 2^k terms per amplitude.
+PassCompute block_compute(const mb2::Block& b) {
+    PassCompute c;
+    (b.diagonal ? c.diag : c.dense1) = b.diagonal ? 1.0 : static_cast<double>(uint64_t{1} << (b.k - 1));
+    return c;
+}
+
+// A planned pass, by what its kernel does for each block: permutations are
+// the tile's map and cost nothing, a real block on its matrix's two diagonals
+// half of a one-qubit block.
+PassCompute planned_compute(const mb2::TileProgram& prog, const mb2::TilePass& pass) {
+    PassCompute c;
+    for (uint32_t i = 0; i < pass.prog_count; ++i) {
+        const mb2::TileInstr& g = prog.instrs[pass.prog_begin + i];
+        if (g.op == mb2::TOP_DIAG) c.diag += 1.0;
+        else if (g.op == mb2::TOP_G2 && g.kind == mb2::TK_CROSS) c.dense1 += 0.5;
+        else if (g.op == mb2::TOP_G1 || g.op == mb2::TOP_G2 || g.op == mb2::TOP_SMEM)
+            c.dense1 += static_cast<double>(uint64_t{1} << (g.k - 1));
+    }
+    return c;
 }
 
 }  // namespace
@@ -2448,25 +2470,32 @@ int mb2_estimate_sweep_time(mb2_context* ctx, const mb2_op* ops, uint32_t num_op
         const std::vector<mb2::Block> blocks = mb2::build_blocks(ops, num_ops, o.fuse_gates != 0, static_cast<uint32_t>(o.fusion_width));
         double total = 0.0;
         if (o.per_gate != 0 || num_qubits < mb2::kMinTileQubits || blocks.empty()) {
-            for (size_t i = 0; i < blocks.size(); ++i) total += pass_seconds(t, c64, blocks, i, i + 1, num_qubits);
+            for (const mb2::Block& b : blocks) total += pass_seconds(t, c64, block_compute(b), num_qubits);
         } else {
-            const uint32_t req = o.tile_qubits > 0 ? static_cast<uint32_t>(o.tile_qubits)
-                                                   : (c64 ? t.tile_qubits_c64 : t.tile_qubits);
-            uint32_t m = c64 ? std::min<uint32_t>(std::max<uint32_t>(req, mb2::kMinTileQubits), mb2::kMaxTileQubitsC64)
-                             : tile_width(req, num_qubits, blocks);
-            for (const mb2::Block& b : blocks) m = std::max(m, b.k);
+            // The sweep's own plan; in the tensor-core form every block is part of a
+            // phase's matrix, and counted as it is in the block list.
+            uint32_t m;
+            bool tc = false;
+            if (c64) {
+                const C64Choice ch = c64_choice(o, num_qubits, t.tile_qubits_c64, blocks);
+                m = ch.m;
+                tc = ch.tc;
+            } else {
+                m = tile_width(o.tile_qubits > 0 ? static_cast<uint32_t>(o.tile_qubits) : t.tile_qubits, num_qubits, blocks);
+            }
             m = std::min(m, num_qubits);
-            // Pass i applies the next `gates` blocks of the program's order.
             const mb2::TileProgram prog = mb2::plan_tile_program(blocks, num_qubits, m, mb2::kDefaultFixedLow,
-                                                                 nullptr, c64);
-            std::vector<mb2::Block> ordered;
-            ordered.reserve(prog.order.size());
-            for (uint32_t i : prog.order) ordered.push_back(blocks[i]);
-            size_t b0 = 0;
+                                                                 nullptr, c64, !tc);
+            size_t done = 0;
             for (const mb2::TilePass& p : prog.passes) {
-                const size_t b1 = std::min(ordered.size(), b0 + p.gates);
-                total += pass_seconds(t, c64, ordered, b0, b1, num_qubits);
-                b0 = b1;
+                PassCompute work;
+                if (!tc) work = planned_compute(prog, p);
+                for (size_t end = std::min(prog.order.size(), done + p.gates); tc && done < end; ++done) {
+                    const PassCompute one = block_compute(blocks[prog.order[done]]);
+                    work.dense1 += one.dense1;
+                    work.diag += one.diag;
+                }
+                total += pass_seconds(t, c64, work, num_qubits);
             }
         }
         *seconds = total;
