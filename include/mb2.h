@@ -580,6 +580,11 @@ int mb2_debug_staged_bytes(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_
  * no counterpart in the reference. */
 int mb2_debug_room(mb2_context* ctx, uint64_t bytes);
 
+/* The sampler's sort by itself: `count` (up to 2^32) words of the generator's
+ * state, tempered, as ascending uniforms in out.  Lets tests give it words
+ * that a seed does not.  Has no counterpart in the reference. */
+int mb2_debug_sort_words(mb2_context* ctx, const uint64_t* words, uint64_t count, double* out);
+
 /* The complex64 tensor-core step alone, on the context's device: 256 rows of
  * 16 complex64 amplitudes (rows: 256 * 32 floats, interleaved) times the
  * 16x16 complex matrix (row-major, interleaved doubles) as the tile pass

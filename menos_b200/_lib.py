@@ -157,6 +157,7 @@ SIGNATURES = {
                                      _VP, _VP]),
     "mb2_debug_staged_bytes": (C.c_int, [C.POINTER(MB2Op), C.c_uint32, C.POINTER(SweepOptions), C.c_uint32, C.c_int32,
                                          C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]),
+    "mb2_debug_sort_words": (C.c_int, [_VP, _VP, C.c_uint64, _VP]),
     "mb2_debug_room": (C.c_int, [_VP, C.c_uint64]),
     "mb2_copy_out": (C.c_int, [_VP, _VP, C.c_uint64]),
     "mb2_copy_in": (C.c_int, [_VP, _VP, C.c_uint64]),

@@ -2206,6 +2206,31 @@ int mb2_debug_tc_probe(mb2_context* ctx, const float* rows, const double* matrix
     return MB2_OK;
 }
 
+int mb2_debug_sort_words(mb2_context* ctx, const uint64_t* words, uint64_t count, double* out) {
+    if (ctx == nullptr || words == nullptr || out == nullptr || count == 0 || count > uint64_t{1} << 32)
+        return MB2_ERR_INVALID;
+    MB2_CUDA(ctx, cudaSetDevice(ctx->device));
+    const size_t scratch = (mb2::uniforms_scratch_bytes(count) + 255) & ~size_t{255};
+    cudaStream_t stream = nullptr;
+    MB2_CUDA(ctx, cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+    unsigned char* dev = nullptr;
+    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&dev), scratch + count * 8, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dev, words, count * 8, cudaMemcpyHostToDevice, stream);
+    auto* u = reinterpret_cast<double*>(dev + scratch);
+    int rc = MB2_OK;
+    if (e == cudaSuccess) {
+        rc = mb2::launch_sort_words(reinterpret_cast<const uint64_t*>(dev), count, dev, u, stream);
+        if (rc != MB2_OK) rc = fail(ctx, rc, std::string("sort launch: ") + mb2::last_cuda_error_string());
+    }
+    if (e == cudaSuccess && rc == MB2_OK) e = cudaMemcpyAsync(out, u, count * 8, cudaMemcpyDeviceToHost, stream);
+    if (dev != nullptr) cudaFreeAsync(dev, stream);
+    const cudaError_t se = cudaStreamSynchronize(stream);
+    cudaStreamDestroy(stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "sort");
+    if (se != cudaSuccess) return cuda_fail(ctx, se, "sort");
+    return rc;
+}
+
 int mb2_debug_schedule(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_options* opts, uint32_t num_qubits,
                        uint32_t* pass, uint32_t* k, uint32_t* qubits, double* matrices, uint64_t* num_blocks,
                        uint64_t* matrix_len, int32_t precision) {

@@ -1,7 +1,7 @@
 """Sampling from the seed to the counts on the device: the generator and the
-sort at the sizes where their kernels change shape (a twist is 312 words, a
-CTA sorts up to 4096 keys in shared memory, runs are counted in tiles of
-1024), sums that cross binades inside one chunk, and the short walk over a
+sort at the sizes where their kernels change shape (a twist is 312 words, runs
+are counted in tiles of 1024; where one CTA's sort ends:
+test_gpu_counts_branches.py), sums that cross binades inside one chunk, and the short walk over a
 density matrix's diagonal.  Counts are whole numbers: identical, always."""
 import numpy as np
 import pytest
