@@ -322,6 +322,7 @@ int launch_tile_pass(void* amps, uint32_t n, const TilePass& pass, const uint32_
     L.smem = L.stages * (size_t{1} << pass.m) * sizeof(double2) + staged;
     L.sm_count = sm_count;
     L.heavy = pass.heavy;
+    L.mapped = pass.mapped;
     // A batch adds the bindings above the n qubits: ntiles counts every
     // binding's tiles, and n grows to the bits the binding index occupies.
     L.ntiles = (uint64_t{1} << n) >> pass.m;

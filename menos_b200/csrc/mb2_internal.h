@@ -176,6 +176,7 @@ struct TilePass {
     uint32_t param_lo = 0;
     uint32_t param_len = 0;
     bool heavy = false;  // has two-qubit dense/monomial, kDiagK or kSmem words
+    bool mapped = false; // reads or leaves the tile through a map (kPhaseMap, store_rec), or has kCross words
     bool mid = false;    // heavy, but only through general dense two-qubit words (kGen2)
     // Tensor-core form (complex64, tile_tc.cpp): the pass's composed phase
     // matrices are tcdata[tc_begin, tc_begin + tc_phases * kTcOperandWords).
@@ -390,6 +391,7 @@ struct TileLaunch {
     int grid = 0;       // set by the instance launcher
     int sm_count = 0;
     bool heavy = false;  // the pass needs the full kernel variant (see TilePass::heavy)
+    bool mapped = false;  // ... the one with the tile's map (TilePass::mapped)
     uint32_t threads = 0;
     size_t smem = 0;
     void* stream = nullptr;

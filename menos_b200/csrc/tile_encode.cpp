@@ -109,6 +109,7 @@ void encode_compact(TileProgram& prog) {
             return is_param(g) ? pass.sdata_count + (g.data - pass.param_lo) : g.data;
         };
         auto& w = prog.words;
+        bool with_map = false;
         bool heavy = false, heavy_other = false;  // other: beyond general dense 2q
         TileMap map;
         // Slot byte offset of place v, in this program's slots.
@@ -253,6 +254,7 @@ void encode_compact(TileProgram& prog) {
                         packed |= static_cast<uint32_t>(g.pos[s]) << (4 * s);
                     }
                     const bool mapped = !map.identity();
+                    with_map = with_map || mapped;
                     const uint32_t settle = mapped && g.kind != 0 ? cop::kPhaseSettle : 0u;
                     w.push_back((mapped ? cop::kPhaseMap : cop::kPhase) |
                                 ((static_cast<uint32_t>(g.nthread) | settle | (controls() << 4)) << 8) | (packed << 16));
@@ -325,6 +327,7 @@ void encode_compact(TileProgram& prog) {
                 case TOP_G2: {
                     if (g.kind == TK_CROSS) {
                         static constexpr uint32_t kPair[4][4] = {{9, 0, 1, 2}, {9, 9, 3, 4}, {9, 9, 9, 5}, {9, 9, 9, 9}};
+                        with_map = true;
                         w.push_back(header(cop::kCross + kPair[g.pos[0]][g.pos[1]], 0, 0, off));
                         break;
                     }
@@ -361,6 +364,7 @@ void encode_compact(TileProgram& prog) {
         pass.heavy = heavy;
         pass.mid = heavy && !heavy_other;
         pass.store_rec = 0;
+        pass.mapped = with_map || !map.identity();
         if (!map.identity()) {
             // The canonical mapping reads the tile through the map: thread bits
             // are tile bits 0.., the register bits the four above them.

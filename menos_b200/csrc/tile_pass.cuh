@@ -195,6 +195,12 @@ __device__ __forceinline__ void gen2_if(double2 (&a)[kNA], const double* md) {
     if constexpr (FULL) g2<P0, P1, TK_GEN>(a, md, 0u);
 }
 
+// Real cross blocks, in the instances that have them.
+template <int P0, int P1, bool MAP>
+__device__ __forceinline__ void cross2_if(double2 (&a)[kNA], const double* md) {
+    if constexpr (MAP) cross2<P0, P1>(a, md);
+}
+
 // cp.async of one 16-byte amplitude, global -> shared (L2 only, no L1).
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
@@ -214,7 +220,14 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // allocator's layout at the merge).  The launcher picks the lean variant for
 // passes without them (the encoder writes single-qubit monomial gates as
 // general 2x2 products, exact up to zero signs).
-template <int MT, bool FULL, typename SYNC>
+//
+// MAP = false compiles out what a pass with X, CX, SWAP or real cross blocks
+// has (TilePass::mapped): the branches on a phase's map and its outside
+// controls, the store record, kCross.  Passes without such blocks paid 1 to 2 %
+// for them: 24 qubits, 16 layers of RY and CZ, 5.45 ms without the maps, 5.54
+// with, 5.43 here; 26 qubits, 10 brick layers, 18.7, 18.9, 18.7; dense
+// two-qubit layers at 27 qubits (FULL) 19.2, 19.4, 18.7.
+template <int MT, bool FULL, bool MAP, typename SYNC>
 __device__ __forceinline__ void compute_tile(double2* __restrict__ tile, const uint32_t* __restrict__ sw,
                                              uint32_t nwords, const double* __restrict__ sd, uint32_t nsdata,
                                              uint32_t pshift, const double* __restrict__ gdata, uint32_t tid,
@@ -227,13 +240,13 @@ __device__ __forceinline__ void compute_tile(double2* __restrict__ tile, const u
     while (pc < nwords) {
         const uint32_t w0 = sw[pc];
         const uint32_t op0 = w0 & 0xffu;
-        if (op0 == cop::kPhase || op0 == cop::kPhaseMap) {
+        if (op0 == cop::kPhase || (MAP && op0 == cop::kPhaseMap)) {
             // The phase record (cop::kPhase): this thread's tile bits from
             // the nibble table, the register bits' slot byte offsets as words.
             // With a map of the tile (cop::kPhaseMap) the slot comes from a
             // table of its own: a pass's X, CX and SWAP blocks cost these
             // lookups in the phases behind them and no move of an amplitude.
-            const bool mapped = op0 == cop::kPhaseMap;
+            const bool mapped = MAP && op0 == cop::kPhaseMap;
             const uint32_t* rec = sw + pc;
             const uint32_t nctl = mapped ? (w0 >> 12) & 7u : 0u;
             pc += mapped ? cop::phase_map_words(MT) + nctl : cop::phase_words(MT);
@@ -298,12 +311,12 @@ __device__ __forceinline__ void compute_tile(double2* __restrict__ tile, const u
                     MB2_CASE4(cop::kReal1, (g1<P, TK_REAL>(a, md, 0u)))
                     MB2_CASE12(cop::kGen2, (gen2_if<P0, P1, FULL>(a, md)))
                     MB2_CASE12(cop::kMono2, if constexpr (FULL) g2<P0, P1, TK_MONO>(a, md, sw[pc++]))
-                    case cop::kCross + 0: cross2<0, 1>(a, md); break;
-                    case cop::kCross + 1: cross2<0, 2>(a, md); break;
-                    case cop::kCross + 2: cross2<0, 3>(a, md); break;
-                    case cop::kCross + 3: cross2<1, 2>(a, md); break;
-                    case cop::kCross + 4: cross2<1, 3>(a, md); break;
-                    case cop::kCross + 5: cross2<2, 3>(a, md); break;
+                    case cop::kCross + 0: cross2_if<0, 1, MAP>(a, md); break;
+                    case cop::kCross + 1: cross2_if<0, 2, MAP>(a, md); break;
+                    case cop::kCross + 2: cross2_if<0, 3, MAP>(a, md); break;
+                    case cop::kCross + 3: cross2_if<1, 2, MAP>(a, md); break;
+                    case cop::kCross + 4: cross2_if<1, 3, MAP>(a, md); break;
+                    case cop::kCross + 5: cross2_if<2, 3, MAP>(a, md); break;
                     case cop::kU3Run0123:
                         g1<0, TK_U3>(a, md, 0u);
                         g1<1, TK_U3>(a, md + 8, 0u);
@@ -453,7 +466,7 @@ __device__ __forceinline__ void compute_tile(double2* __restrict__ tile, const u
 // outside the tile (nmask); moving gridDim.x tiles on is the masked add
 // ((base | ~nmask) + step) & nmask, step = deposit(gridDim.x).
 // The pass over this CTA's share of the tiles: tiles cta, cta + nctas, ...
-template <int MT, typename IDX, bool FULL>
+template <int MT, typename IDX, bool FULL, bool MAP>
 __device__ __forceinline__ void tile_pass_body(double2* __restrict__ st, uint32_t n, uint32_t m_rt, uint64_t smask,
                                                uint64_t gmask, const uint32_t* __restrict__ words, uint32_t nwords,
                                                const double* __restrict__ sdata, uint32_t nsdata,
@@ -553,12 +566,12 @@ __device__ __forceinline__ void tile_pass_body(double2* __restrict__ st, uint32_
             for (uint64_t g = gmask; g != 0; g &= g - 1, ++r)
                 gbits |= static_cast<uint32_t>((static_cast<uint64_t>(cbase) >> (__ffsll(static_cast<long long>(g)) - 1)) & 1u) << r;
         }
-        compute_tile<MT, FULL>(tile, sw, nwords, sd, nsdata, 0u, gdata, tid, m, gbits, [] { __syncthreads(); });
+        compute_tile<MT, FULL, MAP>(tile, sw, nwords, sd, nsdata, 0u, gdata, tid, m, gbits, [] { __syncthreads(); });
 
         // Store: canonical mapping, -0.0 normalised; where the pass left the
         // tile mapped, through the store record.
         const IDX b0 = cbase + off_lo;
-        if (store_rec != 0) {
+        if (MAP && store_rec != 0) {
             const uint32_t* rec = sw + store_rec;
             const uint16_t* pt = reinterpret_cast<const uint16_t*>(rec + 2);
             uint32_t z0 = static_cast<uint32_t>(pt[tid & 15u]) ^ static_cast<uint32_t>(pt[16 + ((tid >> 4) & 15u)]);
@@ -581,14 +594,14 @@ __device__ __forceinline__ void tile_pass_body(double2* __restrict__ st, uint32_
     }
 }
 
-template <int MAXT, int MINB, int MT, typename IDX, bool FULL>
+template <int MAXT, int MINB, int MT, typename IDX, bool FULL, bool MAP>
 __global__ void __launch_bounds__(MAXT, MINB)
     k_tile_pass(double2* __restrict__ st, uint32_t n, uint32_t m_rt, uint64_t smask, uint64_t gmask,
                 const uint32_t* __restrict__ words, uint32_t nwords, const double* __restrict__ sdata,
                 uint32_t nsdata, const double* __restrict__ gdata, uint64_t ntiles, const double* __restrict__ pdata,
                 uint32_t pstride, uint32_t param_lo, uint32_t param_len, uint32_t bshift, uint32_t store_rec,
                 uint32_t stages) {
-    tile_pass_body<MT, IDX, FULL>(st, n, m_rt, smask, gmask, words, nwords, sdata, nsdata, gdata, ntiles, pdata,
+    tile_pass_body<MT, IDX, FULL, MAP>(st, n, m_rt, smask, gmask, words, nwords, sdata, nsdata, gdata, ntiles, pdata,
                                   pstride, param_lo, param_len, bshift, store_rec, stages, blockIdx.x, gridDim.x);
 }
 
@@ -604,13 +617,13 @@ __global__ void __launch_bounds__(MAXT, 1) k_tile_pass_jobs(const TileJob* __res
         else hi = mid;
     }
     const TileJob& J = jobs[lo];
-    tile_pass_body<MT, uint64_t, FULL>(static_cast<double2*>(J.st), J.n, m_rt, J.smask, J.gmask, J.words, J.nwords, J.sdata, J.nsdata,
+    tile_pass_body<MT, uint64_t, FULL, true>(static_cast<double2*>(J.st), J.n, m_rt, J.smask, J.gmask, J.words, J.nwords, J.sdata, J.nsdata,
                                        J.gdata, J.ntiles, nullptr, 0, 0, 0, 0, J.store_rec, 2, blockIdx.x - J.cta_begin,
                                        J.nctas);
 }
 
 // Launches one instance; the shared-memory limit is raised once per instance.
-template <int MAXT, int MINB, int MT, typename IDX, bool FULL>
+template <int MAXT, int MINB, int MT, typename IDX, bool FULL, bool MAP>
 int launch_instance(const TileLaunch& L) {
     // The dynamic limit is what the static shared memory leaves of the
     // per-block maximum; it is raised once, by whichever thread launches
@@ -618,9 +631,9 @@ int launch_instance(const TileLaunch& L) {
     // initialisation is thread-safe and every thread sees it complete).
     static const size_t dyn_max = [] {
         cudaFuncAttributes fa{};
-        if (cudaFuncGetAttributes(&fa, k_tile_pass<MAXT, MINB, MT, IDX, FULL>) != cudaSuccess) return size_t{0};
+        if (cudaFuncGetAttributes(&fa, k_tile_pass<MAXT, MINB, MT, IDX, FULL, MAP>) != cudaSuccess) return size_t{0};
         const size_t v = kTileSmemMax - fa.sharedSizeBytes;
-        if (cudaFuncSetAttribute(k_tile_pass<MAXT, MINB, MT, IDX, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(k_tile_pass<MAXT, MINB, MT, IDX, FULL, MAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(v)) != cudaSuccess)
             return size_t{0};
         return v;
@@ -628,7 +641,7 @@ int launch_instance(const TileLaunch& L) {
     if (dyn_max == 0) return launch_status();
     if (L.smem > dyn_max) return MB2_ERR_INVALID;
     launch_behind(
-        k_tile_pass<MAXT, MINB, MT, IDX, FULL>, L.grid, L.threads, L.smem, static_cast<cudaStream_t>(L.stream),
+        k_tile_pass<MAXT, MINB, MT, IDX, FULL, MAP>, L.grid, L.threads, L.smem, static_cast<cudaStream_t>(L.stream),
         static_cast<double2*>(L.amps), L.n_all, L.m, L.smask, L.gmask, L.words, L.nwords, L.sdata, L.nsdata, L.gdata,
         L.ntiles, L.pdata, L.pstride, L.param_lo, L.param_len, L.bshift, L.store_rec, L.stages);
     return launch_status();

@@ -36,6 +36,13 @@ constexpr size_t kMaxBlocksPerPass = 300;
 // as they are.
 constexpr size_t kMaxAhead = 512;
 
+// States up to which a program's passes run one kernel (TilePass::mapped): one
+// and two kernels, ms: a sampled density matrix of 10 and 11 qubits (20 and 22
+// here; its passes are of both kinds) 0.601 0.634, 1.184 1.208; 10 brick layers
+// and a CX ladder at 20 qubits 0.316 0.318, at 22 1.039 1.049, at 23 2.115
+// 2.110, at 24 4.46 4.43; 5 layers at 26 10.48 10.28.
+constexpr uint32_t kOneKernelQubits = 22;
+
 // A pass's instruction words and small-matrix data are staged in shared memory
 // (kMaxStagedBytes): a bound on what each block adds, whatever order the
 // pass's blocks come in.
@@ -922,6 +929,14 @@ TileProgram plan_tile_program(const std::vector<Block>& all, uint32_t n, uint32_
         prog.passes.push_back(pass);
     }
     encode_compact(prog);
+    // Short passes all run the kernel with the map where one of them needs it:
+    // going from one kernel to the other costs more than the 1 % that the map
+    // costs the rest (kOneKernelQubits).
+    if (n <= kOneKernelQubits) {
+        bool any = false;
+        for (const TilePass& p : prog.passes) any = any || p.mapped;
+        for (TilePass& p : prog.passes) p.mapped = any;
+    }
     return prog;
 }
 
