@@ -380,7 +380,7 @@ int launch_c64_instance(const TileLaunch& L) {
     if (dyn_max == 0) return launch_status();
     if (L.smem > dyn_max) return MB2_ERR_INVALID;
     launch_behind(
-        k_tile_pass_c64<MAXT, MINB, MT, IDX, V>, L.grid, L.threads, L.smem, static_cast<cudaStream_t>(L.stream),
+        L.n_all, k_tile_pass_c64<MAXT, MINB, MT, IDX, V>, L.grid, L.threads, L.smem, static_cast<cudaStream_t>(L.stream),
         static_cast<float2*>(L.amps), L.n_all, L.m, L.smask, L.words, L.nwords, L.sdata, L.nsdata, L.gdata, L.ntiles,
         L.pdata, L.pstride, L.param_lo, L.param_len, L.bshift, L.store_rec, L.stages);
     return launch_status();
