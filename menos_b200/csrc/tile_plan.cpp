@@ -406,6 +406,8 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
     }
     const bool tc = tc_blocks != nullptr && std::find(tc_blocks->begin(), tc_blocks->end(), 0) == tc_blocks->end();
     const Staged staged_of{mt, mapped, true, tc};
+    std::vector<size_t> stages(nb);  // (looked at for every candidate below)
+    for (uint32_t i = 0; i < nb; ++i) stages[i] = staged_of(blocks[i], moves[i] != 0);
     for (uint32_t i = 0; i < nb; ++i)
         for (uint32_t t = 0; t < blocks[i].k; ++t) lists[blocks[i].q[t]].push_back(i);
     std::vector<uint32_t> head(n, 0);
@@ -436,9 +438,9 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
             const uint32_t i = lists[x][h[x]];
             if ((blocks[i].mask() & ~s) != 0 || !at_head(h, i)) continue;
             if (limit && (count >= kMaxBlocksPerPass ||
-                          (count > 0 && staged + staged_of(blocks[i], moves[i] != 0) > kMaxStagedBytes)))
+                          (count > 0 && staged + stages[i] > kMaxStagedBytes)))
                 break;
-            staged += staged_of(blocks[i], moves[i] != 0);
+            staged += stages[i];
             ++count;
             if (out) out->push_back(i);
             for (uint32_t t = 0; t < blocks[i].k; ++t) {
