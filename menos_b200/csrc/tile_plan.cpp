@@ -234,7 +234,7 @@ bool is_exact_move(const Block& b) {
 // instead of 28 (a CX's control, one bit for a whole tile when it lies
 // outside, need not be in it either).
 std::vector<PassSel> select_passes(const std::vector<Block>& blocks, uint32_t n, uint32_t m, uint32_t fixed_low,
-                                   const std::vector<uint8_t>* parametric) {
+                                   const std::vector<uint8_t>* parametric, const std::vector<int8_t>& kinds) {
     std::vector<PassSel> passes;
     uint32_t widest = 1;
     for (const Block& b : blocks) widest = std::max(widest, b.k);
@@ -251,15 +251,14 @@ std::vector<PassSel> select_passes(const std::vector<Block>& blocks, uint32_t n,
     const size_t nb = blocks.size();
     auto is_param = [&](size_t i) { return parametric != nullptr && ((*parametric)[i] & kParamBlock) != 0; };
     std::vector<uint8_t> moves(nb), done(nb, 0);
-    std::vector<int8_t> kinds(nb, -1);
-    bool mapped = false;
+    bool mapped = false, any = false;
     for (size_t i = 0; i < nb; ++i) {
         moves[i] = !is_param(i) && is_exact_move(blocks[i]);
-        if (!is_param(i)) kinds[i] = static_cast<int8_t>(move_kind(blocks[i]));
+        any = any || moves[i];
         mapped = mapped || kinds[i] >= 0;
     }
     std::vector<uint64_t> moves_from(nb + 1, 0);  // qubits of the exact moves from block i on
-    for (size_t i = nb; i-- > 0;) moves_from[i] = moves_from[i + 1] | (moves[i] ? blocks[i].mask() : 0);
+    for (size_t i = any ? nb : 0; i-- > 0;) moves_from[i] = moves_from[i + 1] | (moves[i] ? blocks[i].mask() : 0);
     const Staged staged_of{mt, mapped, false};
     for (size_t first = 0; first < nb;) {
         uint64_t smask = 0, dmask = 0;  // the tile's qubits so far; the diagonals' operands
@@ -382,12 +381,13 @@ void thread_bit_order(uint32_t m, const uint32_t* reg, uint32_t nreg, uint8_t* t
 // next set from the ready dense blocks, so the kernel changes phase rarely.
 // Exact permutations need no registers either, but end the phase they come
 // in (the amplitudes' places change), so they wait until no other block of
-// the pass is ready.  Not in a program that is rewritten for the tensor cores
-// (tc_blocks: which blocks can be): there they are part of a phase's matrix
-// like any other block, and waiting would spread them over more phases
-// (81 layouts instead of 75 for a 26-qubit RY/RZ + CX ansatz, unfused).
+// the pass is ready.  Not in a pass that is rewritten for the tensor cores
+// (tc_blocks: which blocks can be, in a program for them): there they are part
+// of a phase's matrix like any other block, and waiting would spread them over
+// more phases (81 layouts instead of 75 for a 26-qubit RY/RZ + CX ansatz,
+// unfused).
 std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, uint32_t n, uint32_t m,
-                                             uint32_t fixed_low, const std::vector<uint8_t>* parametric,
+                                             uint32_t fixed_low, const std::vector<int8_t>& kinds,
                                              const std::vector<uint8_t>* tc_blocks) {
     std::vector<PassSel> passes;
     uint32_t widest = 1;
@@ -397,17 +397,16 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
     const uint32_t fixed = std::min(fixed_low, mt - widest);
     const uint32_t nb = static_cast<uint32_t>(blocks.size());
     std::vector<std::vector<uint32_t>> lists(n);
-    std::vector<uint8_t> moves(nb, 0);
+    std::vector<uint8_t> moves(nb, 0), none(nb, 0);
     bool mapped = false;
     for (uint32_t i = 0; i < nb; ++i) {
-        const bool move = !(parametric != nullptr && ((*parametric)[i] & kParamBlock) != 0) && move_kind(blocks[i]) >= 0;
-        moves[i] = move && tc_blocks == nullptr;
-        mapped = mapped || move;
+        moves[i] = kinds[i] >= 0;
+        mapped = mapped || moves[i];
     }
     const bool tc = tc_blocks != nullptr && std::find(tc_blocks->begin(), tc_blocks->end(), 0) == tc_blocks->end();
     const Staged staged_of{mt, mapped, true, tc};
     std::vector<size_t> stages(nb);  // (looked at for every candidate below)
-    for (uint32_t i = 0; i < nb; ++i) stages[i] = staged_of(blocks[i], moves[i] != 0);
+    for (uint32_t i = 0; i < nb; ++i) stages[i] = staged_of(blocks[i], moves[i] && tc_blocks == nullptr);
     for (uint32_t i = 0; i < nb; ++i)
         for (uint32_t t = 0; t < blocks[i].k; ++t) lists[blocks[i].q[t]].push_back(i);
     std::vector<uint32_t> head(n, 0);
@@ -489,7 +488,12 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
         PassSel sel;
         sel.smask = s;
         std::vector<uint8_t> in_pass(nb, 0);
-        for (uint32_t i : members) in_pass[i] = 1;
+        bool simt = tc_blocks == nullptr;
+        for (uint32_t i : members) {
+            in_pass[i] = 1;
+            simt = simt || !(*tc_blocks)[i];
+        }
+        const std::vector<uint8_t>& waits = simt ? moves : none;
         std::vector<uint32_t> ph = head, sim, grown;
         std::vector<uint8_t> sim_in, grown_in;
         // Runs every member that register set `regs` can take (diagonals and
@@ -511,7 +515,7 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
                         if (hh[x] >= lists[x].size()) continue;
                         const uint32_t i = lists[x][hh[x]];
                         const Block& b = blocks[i];
-                        if (!in[i] || b.diagonal != diag || moves[i] || !at_head(hh, i) ||
+                        if (!in[i] || b.diagonal != diag || waits[i] || !at_head(hh, i) ||
                             !(b.diagonal || b.k > 2 || (b.mask() & ~regs) == 0))
                             continue;
                         in[i] = 0;
@@ -538,7 +542,7 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
                 if (hh[y] >= lists[y].size()) continue;
                 const uint32_t i = lists[y][hh[y]];
                 const Block& b = blocks[i];
-                if (!in[i] || moves[i] || !at_head(hh, i) || !(b.diagonal || b.k > 2 || (b.mask() & ~regs) == 0)) continue;
+                if (!in[i] || waits[i] || !at_head(hh, i) || !(b.diagonal || b.k > 2 || (b.mask() & ~regs) == 0)) continue;
                 in[i] = 0;
                 if (!b.diagonal && b.k <= 2) ++dense;
                 for (uint32_t t = 0; t < b.k; ++t) {
@@ -560,11 +564,11 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
             // blocks use, then the lowest).
             uint64_t cand = 0;
             for (uint32_t i : members)
-                if (in_pass[i] && !blocks[i].diagonal && blocks[i].k <= 2 && !moves[i]) cand |= blocks[i].mask();
+                if (in_pass[i] && !blocks[i].diagonal && blocks[i].k <= 2 && !waits[i]) cand |= blocks[i].mask();
             // Nothing but permutations ready: those that are.
             bool ready = false;
             for (uint32_t i : members)
-                ready = ready || (in_pass[i] && !blocks[i].diagonal && blocks[i].k <= 2 && !moves[i] && at_head(ph, i));
+                ready = ready || (in_pass[i] && !blocks[i].diagonal && blocks[i].k <= 2 && !waits[i] && at_head(ph, i));
             if (!ready) {
                 bool any = false;
                 for (bool again = true; again;) {
@@ -572,7 +576,7 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
                     for (uint32_t x = 0; x < n; ++x) {
                         if (!((s >> x) & 1u) || ph[x] >= lists[x].size()) continue;
                         const uint32_t i = lists[x][ph[x]];
-                        if (!in_pass[i] || !moves[i] || !at_head(ph, i)) continue;
+                        if (!in_pass[i] || !waits[i] || !at_head(ph, i)) continue;
                         in_pass[i] = 0;
                         again = any = true;
                         sel.gates.push_back(i);
@@ -600,7 +604,7 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
                     const uint64_t runs = grown_runs + count_from(regs | (uint64_t{1} << x), x, sim, sim_in);
                     uint32_t uses = 0;
                     for (uint32_t i : members)
-                        if (in_pass[i] && !blocks[i].diagonal && blocks[i].k <= 2 && !moves[i] &&
+                        if (in_pass[i] && !blocks[i].diagonal && blocks[i].k <= 2 && !waits[i] &&
                             ((blocks[i].mask() >> x) & 1u) && at_head(ph, i))
                             ++uses;
                     const uint64_t score = (runs << 16) | uses;
@@ -630,6 +634,7 @@ TileProgram plan_tile_program(const std::vector<Block>& all, uint32_t n, uint32_
     std::vector<uint8_t> part_flags, last;
     std::vector<uint32_t> origin;
     for (size_t i = 0; i < all.size() && split; ++i) {
+        if (origin.empty() && (all[i].k != 2 || all[i].diagonal)) continue;
         Block first, second;
         const uint8_t flags = all_parametric ? (*all_parametric)[i] : uint8_t{0};
         const bool two = !(flags & kParamBlock) && move_kind(all[i]) < 0 && split_block(all[i], first, second);
@@ -668,9 +673,14 @@ TileProgram plan_tile_program(const std::vector<Block>& all, uint32_t n, uint32_
     if (mt < kRegQubits) throw std::invalid_argument("state too small for the tile kernel");
     if (commuting && !split)
         for (const Block& b : all) prog.tc_blocks.push_back(tc_convertible(b));
+    std::vector<int8_t> kinds(blocks.size());  // move_kind; parametric blocks have none
+    for (size_t i = 0; i < blocks.size(); ++i)
+        kinds[i] = parametric != nullptr && ((*parametric)[i] & kParamBlock) != 0
+                       ? int8_t{-1}
+                       : static_cast<int8_t>(move_kind(blocks[i]));
     const std::vector<PassSel> sels =
-        commuting ? select_passes_commuting(blocks, n, mt, fixed_low, parametric, split ? nullptr : &prog.tc_blocks)
-                  : select_passes(blocks, n, mt, fixed_low, parametric);
+        commuting ? select_passes_commuting(blocks, n, mt, fixed_low, kinds, split ? nullptr : &prog.tc_blocks)
+                  : select_passes(blocks, n, mt, fixed_low, parametric, kinds);
     prog.c64 = commuting;
     prog.param_offsets.assign(all.size(), 0);
     auto param_flags = [&](uint32_t bi) -> uint8_t { return parametric ? (*parametric)[bi] : uint8_t{0}; };
@@ -683,14 +693,20 @@ TileProgram plan_tile_program(const std::vector<Block>& all, uint32_t n, uint32_
     };
     // The caller's blocks in an order of whole blocks that the parts' order
     // amounts to: one is listed when it is complete and every earlier block on
-    // its qubits is.  Returns how many that made.
-    std::vector<std::vector<uint32_t>> waiting(n);  // per qubit, latest block first
-    for (uint32_t i = static_cast<uint32_t>(all.size()); i-- > 0;)
+    // its qubits is.  Returns how many that made.  (Where no block is in parts,
+    // the order they are planned in is that order.)
+    std::vector<std::vector<uint32_t>> waiting(whole ? 0 : n);  // per qubit, latest block first
+    for (uint32_t i = whole ? 0 : static_cast<uint32_t>(all.size()); i-- > 0;)
         for (uint32_t t = 0; t < all[i].k; ++t) waiting[all[i].q[t]].push_back(i);
-    std::vector<uint8_t> ready(all.size(), 0);
+    std::vector<uint8_t> ready(whole ? 0 : all.size(), 0);
     std::vector<uint32_t> look;
     auto complete = [&](uint32_t i) {
         uint32_t listed = 0;
+        if (whole) {
+            prog.order.push_back(i);
+            prog.order_pass.push_back(static_cast<uint32_t>(prog.passes.size()));
+            return uint32_t{1};
+        }
         ready[i] = 1;
         look.assign(1, i);
         while (!look.empty()) {
@@ -744,7 +760,7 @@ TileProgram plan_tile_program(const std::vector<Block>& all, uint32_t n, uint32_
             std::vector<uint32_t> r(first);
             for (size_t j = from; j < sel.gates.size() && r.size() < kRegQubits; ++j) {
                 const Block& b = blocks[sel.gates[j]];
-                if (!(param_flags(sel.gates[j]) & kParamBlock) && move_kind(b) >= 0) break;  // the phase ends there
+                if (kinds[sel.gates[j]] >= 0) break;  // the phase ends there
                 if (b.diagonal || b.k > 2) continue;
                 bool fits = true;
                 uint32_t extra = 0;
@@ -782,7 +798,7 @@ TileProgram plan_tile_program(const std::vector<Block>& all, uint32_t n, uint32_
             if (whole || last[sel.gates[j]]) pass.gates += complete(origin_of(sel.gates[j]));
             TileInstr g{};
             g.k = static_cast<uint8_t>(b.k);
-            const int move = param_flags(sel.gates[j]) & kParamBlock ? -1 : move_kind(b);
+            const int move = kinds[sel.gates[j]];
             if (move >= 0) {
                 close_phase();
                 g.op = TOP_MOVE;
