@@ -331,6 +331,7 @@ int launch_tile_pass(void* amps, uint32_t n, const TilePass& pass, const uint32_
         L.ntiles *= batch->bindings;
         while ((uint64_t{1} << (L.n_all - n)) < batch->bindings) ++L.n_all;
     }
+    L.behind = pass.behind && (uint64_t{sizeof(double2)} << L.n_all) <= kBehindBytes;
     const int rc = pass.m == 11 ? launch_tile_m11(L) : pass.m == 12 ? launch_tile_m12(L) : launch_tile_generic(L);
     note_launches(1);
     return rc;

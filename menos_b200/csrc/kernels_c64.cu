@@ -380,7 +380,7 @@ int launch_c64_instance(const TileLaunch& L) {
     if (dyn_max == 0) return launch_status();
     if (L.smem > dyn_max) return MB2_ERR_INVALID;
     launch_behind(
-        L.n_all, k_tile_pass_c64<MAXT, MINB, MT, IDX, V>, L.grid, L.threads, L.smem, static_cast<cudaStream_t>(L.stream),
+        L.behind, k_tile_pass_c64<MAXT, MINB, MT, IDX, V>, L.grid, L.threads, L.smem, static_cast<cudaStream_t>(L.stream),
         static_cast<float2*>(L.amps), L.n_all, L.m, L.smask, L.words, L.nwords, L.sdata, L.nsdata, L.gdata, L.ntiles,
         L.pdata, L.pstride, L.param_lo, L.param_len, L.bshift, L.store_rec, L.stages);
     return launch_status();
@@ -432,6 +432,7 @@ int launch_tile_pass_c64(void* amps, uint32_t n, const TilePass& pass, const uin
         L.ntiles *= batch->bindings;
         while ((uint64_t{1} << (L.n_all - n)) < batch->bindings) ++L.n_all;
     }
+    L.behind = pass.behind && (uint64_t{sizeof(float2)} << L.n_all) <= kBehindBytes;
     const uint64_t cap = static_cast<uint64_t>(sm_count) * (pass.m == kMaxTileQubitsC64 ? 1u : 2u);
     L.grid = static_cast<int>(L.ntiles < cap ? L.ntiles : cap);
     int rc;

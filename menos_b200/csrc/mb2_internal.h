@@ -176,6 +176,7 @@ struct TilePass {
     uint32_t param_lo = 0;
     uint32_t param_len = 0;
     bool heavy = false;  // has two-qubit dense/monomial, kDiagK or kSmem words
+    bool behind = true;  // no pass of the program keeps it from being launched behind another (launch_next.cuh)
     bool mapped = false; // reads or leaves the tile through a map (kPhaseMap, store_rec), or has kCross words
     bool mid = false;    // heavy, but only through general dense two-qubit words (kGen2)
     // Tensor-core form (complex64, tile_tc.cpp): the pass's composed phase
@@ -369,6 +370,8 @@ int launch_tile_pass(void* amps, uint32_t n, const TilePass& pass, const uint32_
                      const double* dev_sdata, const double* dev_gdata, int sm_count, void* stream,
                      const BatchLayout* batch = nullptr);
 // One tile-pass launch, as the instances (kernels_tile_*.cu) take it.
+// States up to which passes are launched behind one another.
+constexpr uint64_t kBehindBytes = uint64_t{64} << 20;
 struct TileLaunch {
     void* amps = nullptr;
     uint32_t n_all = 0;  // index bits, bindings included
@@ -392,6 +395,7 @@ struct TileLaunch {
     int sm_count = 0;
     bool heavy = false;  // the pass needs the full kernel variant (see TilePass::heavy)
     bool mapped = false;  // ... the one with the tile's map (TilePass::mapped)
+    bool behind = false;  // launched behind the pass before it (launch_next.cuh)
     uint32_t threads = 0;
     size_t smem = 0;
     void* stream = nullptr;

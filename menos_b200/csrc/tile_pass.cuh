@@ -641,7 +641,7 @@ int launch_instance(const TileLaunch& L) {
     if (dyn_max == 0) return launch_status();
     if (L.smem > dyn_max) return MB2_ERR_INVALID;
     launch_behind(
-        L.n_all, k_tile_pass<MAXT, MINB, MT, IDX, FULL, MAP>, L.grid, L.threads, L.smem, static_cast<cudaStream_t>(L.stream),
+        L.behind, k_tile_pass<MAXT, MINB, MT, IDX, FULL, MAP>, L.grid, L.threads, L.smem, static_cast<cudaStream_t>(L.stream),
         static_cast<double2*>(L.amps), L.n_all, L.m, L.smask, L.gmask, L.words, L.nwords, L.sdata, L.nsdata, L.gdata,
         L.ntiles, L.pdata, L.pstride, L.param_lo, L.param_len, L.bshift, L.store_rec, L.stages);
     return launch_status();

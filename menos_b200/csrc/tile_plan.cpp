@@ -955,6 +955,9 @@ TileProgram plan_tile_program(const std::vector<Block>& all, uint32_t n, uint32_
         for (const TilePass& p : prog.passes) any = any || p.mapped;
         for (TilePass& p : prog.passes) p.mapped = any;
     }
+    bool full = false;
+    for (const TilePass& p : prog.passes) full = full || p.heavy;
+    for (TilePass& p : prog.passes) p.behind = commuting || !full;
     return prog;
 }
 
