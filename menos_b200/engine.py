@@ -266,9 +266,10 @@ class DeviceState:
         """An array for copy_out, its pages touched: the system hands out a
         new array's pages at the first write to each, which inside the copy
         costs more than the copy.  Called while the device is at work, it
-        costs nothing."""
+        costs nothing.  (A small array's pages are the allocator's own.)"""
         out = np.empty(1 << self.n, np.complex128 if self.precision == C128 else np.complex64)
-        out.view(np.uint8)[::4096] = 0
+        if out.nbytes > 1 << 16:
+            out.view(np.uint8)[::4096] = 0
         return out
 
     def copy_out(self, out: Optional[np.ndarray] = None) -> np.ndarray:
