@@ -1192,12 +1192,14 @@ int histogram(mb2_context* ctx, uint32_t n, const std::vector<uint64_t>& basis, 
     for (size_t i = 1; i < oc.size() && ordered; ++i) ordered = oc[i - 1].first < oc[i].first;
     if (!ordered) std::sort(oc.begin(), oc.end());
     uint64_t d = 0;
+    for (size_t i = 0; i < oc.size(); ++i) d += i == 0 || oc[i].first != oc[i - 1].first ? 1 : 0;
+    if (d > *num_outcomes) return fail(ctx, MB2_ERR_INVALID, "outcome capacity too small");  // nothing written
+    d = 0;
     for (const auto& [o, c] : oc) {
         if (d > 0 && outcomes[d - 1] == o) {
             counts[d - 1] += c;
             continue;
         }
-        if (d >= *num_outcomes) return fail(ctx, MB2_ERR_INVALID, "outcome capacity too small");
         outcomes[d] = o;
         counts[d] = c;
         ++d;
@@ -1205,6 +1207,13 @@ int histogram(mb2_context* ctx, uint32_t n, const std::vector<uint64_t>& basis, 
     *num_outcomes = d;
     return MB2_OK;
 }
+
+// Up to this many shots are drawn, sorted and counted on the host: a call on
+// the device is nine launches and a second synchronisation more.  Device and
+// host, us: 100 shots of a 4-qubit state 84, 50, of a 20-qubit one 200, 167, of
+// a 2-qubit density matrix 75, 38; 3000 shots 102 88, 227 223, 95 86; 4096
+// shots 111 105, 252 267, 108 101; 8192 shots 119 177, 257 344, 109 163.
+constexpr uint64_t kFewShots = 3000;
 
 // `shots` draws from `seed` as counts of the measured outcomes, the state on
 // the device from the uniforms to the counts: walk(draw, u, sort, scratch,
@@ -1218,11 +1227,15 @@ int device_counts(mb2_state* s, uint32_t n, uint64_t shots, uint64_t seed, const
                   size_t walk_bytes, WALK walk) {
     if (shots > uint64_t{1} << 40) return fail(s->ctx, MB2_ERR_RESOURCE, "too many shots");
     const size_t al_u = (shots * 8 + 255) & ~size_t{255};
-    // Where the device has no room for the sort (a state that nearly fills
-    // it), the uniforms are sorted and the outcomes counted on the host.
-    const int room = ensure_scratch(s, walk_bytes + mb2::draw_bytes(shots));
-    if (room != MB2_OK && room != MB2_ERR_RESOURCE) return room;
-    const bool on_device = room == MB2_OK;
+    // Few shots, or where the device has no room for the sort (a state that
+    // nearly fills it): the uniforms are sorted and the outcomes counted on the
+    // host.
+    bool on_device = shots > kFewShots;
+    if (on_device) {
+        const int room = ensure_scratch(s, walk_bytes + mb2::draw_bytes(shots));
+        if (room != MB2_OK && room != MB2_ERR_RESOURCE) return room;
+        on_device = room == MB2_OK;
+    }
     if (!on_device)
         if (int e = ensure_scratch(s, 2 * al_u + walk_bytes); e != MB2_OK) return e;
     auto* base = static_cast<unsigned char*>(s->scratch);

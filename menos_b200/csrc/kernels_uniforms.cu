@@ -137,16 +137,6 @@ __global__ void __launch_bounds__(kSortThreads) k_bucket_sort(uint64_t* __restri
         u[begin + i] = static_cast<double>(v[i]) * (1.0 / 9007199254740992.0);
 }
 
-// A single bucket: at most kSortMean words, sorted in place as uniforms.
-__global__ void __launch_bounds__(kSortThreads) k_sort_few(const uint64_t* words, uint32_t shots, double* u) {
-    __shared__ uint64_t sh[kSortMean];
-    for (uint32_t i = threadIdx.x; i < shots; i += kSortThreads) sh[i] = mt_key(words[i]);
-    __syncthreads();
-    sort_cta(sh, shots);
-    for (uint32_t i = threadIdx.x; i < shots; i += kSortThreads)
-        u[i] = static_cast<double>(sh[i]) * (1.0 / 9007199254740992.0);
-}
-
 // Runs of equal basis states (non-decreasing): the runs that begin in each
 // tile of kRleTile shots, then each run's state and first shot at its rank.
 __global__ void __launch_bounds__(kRleThreads) k_run_count(const uint64_t* __restrict__ basis, uint64_t shots,
@@ -212,11 +202,6 @@ size_t uniforms_scratch_bytes(uint64_t shots) {
 int launch_sort_words(const uint64_t* words, uint64_t shots, void* scratch, double* dev_u, void* stream) {
     const auto s = static_cast<cudaStream_t>(stream);
     const uint32_t bits = bucket_bits(shots);
-    if (bits == 0) {
-        k_sort_few<<<1, kSortThreads, 0, s>>>(words, static_cast<uint32_t>(shots), dev_u);
-        note_launches(1);
-        return launch_status();
-    }
     const uint64_t nb = uint64_t{1} << bits;
     auto* p = static_cast<unsigned char*>(scratch) + al(mt_room(shots) * 8);
     auto* keys = reinterpret_cast<uint64_t*>(p);

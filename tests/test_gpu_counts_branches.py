@@ -1,8 +1,8 @@
 """Branches of the sampling path that ordinary states and calls do not take:
 no room on the device for the draws' sort and the counts, an infinite
-amplitude, a sort bucket beyond what shared memory holds, and the sizes where
-one CTA's sort ends (512 words, sorted in one piece; buckets of at most 512 on
-average above, up to 1024 each in shared memory)."""
+amplitude, a sort bucket beyond what shared memory holds; and the sizes where
+its rules turn (3000 shots, up to which the host draws and counts; buckets of
+at most 512 words on average, up to 1024 each sorted in shared memory)."""
 import ctypes as C
 
 import numpy as np
@@ -22,8 +22,8 @@ def identity(n):
 
 
 @pytest.mark.parametrize("n", [3, 13])
-@pytest.mark.parametrize("shots", [511, 512, 513, 1024, 1025])
-def test_counts_where_one_sort_ends(ctx, oracle, n, shots):
+@pytest.mark.parametrize("shots", [1, 2999, 3000, 3001, 4096, 4097])
+def test_counts_where_the_device_takes_over(ctx, oracle, n, shots):
     s = rand_state(n, np.random.default_rng(shots))
     st = dev_state(ctx, s)
     for seed in (1, 2 ** 63):
@@ -74,6 +74,14 @@ def mt_key(x):
     x = x ^ ((x << np.uint64(17)) & np.uint64(0x71D67FFFEDA60000))
     x = x ^ ((x << np.uint64(37)) & np.uint64(0xFFF7EEE000000000))
     return (x ^ (x >> np.uint64(43))) >> np.uint64(11)
+
+
+@pytest.mark.parametrize("count", [1, 2, 511, 512, 513, 1024, 1025, 70000])
+def test_sort_sizes(ctx, count):
+    words = np.random.default_rng(count).integers(0, 2 ** 64, count, np.uint64)
+    out = np.zeros(count)
+    assert lib().mb2_debug_sort_words(ctx.h, words.ctypes.data, count, out.ctypes.data) == 0
+    assert np.array_equal(out, np.sort(mt_key(words).astype(np.float64) * 2.0 ** -53))
 
 
 @pytest.mark.parametrize("crowd", [0, 1023, 1024, 1025, 3000, 4096])
