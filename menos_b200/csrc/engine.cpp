@@ -1597,7 +1597,9 @@ struct TrajChannel {
 };
 
 // The most trajectories run at once, and the most memory their states take
-// together (a larger state runs alone).
+// together (a larger state runs alone).  256 trajectories of 10 qubits with 16
+// at once 16.1 ms, 64 7.7, 256 5.8; 128 of 14 qubits 27.2, 9.6, 6.7: more than
+// 64 would gain a third for four times the memory that a small run holds.
 constexpr uint64_t kTrajBatch = 64;
 constexpr uint64_t kTrajBatchBytes = uint64_t{256} << 20;
 uint64_t trajectory_batch(uint32_t n, uint64_t trajectories, bool monitored) {

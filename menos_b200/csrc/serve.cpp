@@ -203,7 +203,9 @@ void run_small_batch(mb2_server* s, cudaStream_t stream, std::vector<Request>& b
     std::vector<uint32_t> tile(B, 0);
     std::vector<bool> ok(B, true);
     // Plans and draws: host work of half a millisecond a request, spread over a
-    // few threads (vectors of bool share bytes, hence the plain flags).
+    // few threads (vectors of bool share bytes, hence the plain flags).  A burst
+    // of 128 requests of 12 to 16 qubits on 16 cores with up to 2 threads a
+    // batch 15.6 ms, 8 11.8, 16 11.7; bursts of 40 and 8 within 7 % of each other.
     std::vector<uint8_t> planned(B, 0);
     std::vector<std::vector<double>> uniforms(B);
     auto prepare = [&](size_t i) {
