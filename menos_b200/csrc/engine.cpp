@@ -614,7 +614,7 @@ int mb2_apply_program_monitored(mb2_state* s, const mb2_op* ops, uint32_t num_op
                                                                          : static_cast<uint32_t>(o.low_qubits));
         // complex64 results are not bitwise the reference's: commuting
         // blocks may be reordered into fewer passes.
-        prog = mb2::plan_tile_program(blocks, s->n, m, low, nullptr, c64, !tc);
+        prog = mb2::plan_tile_program(blocks, s->n, m, low, nullptr, c64, !tc, s->n <= m);
         if (tc) mb2::make_tensor_core_program(prog, blocks, mb2::tc_max_phases(m));
     } catch (const std::exception& e) {
         return fail(s->ctx, MB2_ERR_INVALID, e.what());
@@ -656,6 +656,10 @@ int mb2_apply_program_monitored(mb2_state* s, const mb2_op* ops, uint32_t num_op
         if (err != 0) return fail(s->ctx, MB2_ERR_CUDA, "tensor-core pass: a bounded wait ran out");
         return MB2_OK;
     };
+    // A monitored sweep waits for each pass: there is none to launch one behind,
+    // and saying so takes the launch longer (12 qubits, 11 passes: 143 -> 150 us).
+    if (boundary != nullptr)
+        for (mb2::TilePass& pass : prog.passes) pass.behind = false;
     for (const mb2::TilePass& pass : prog.passes) {
         int rc;
         if (pass.tc) {
@@ -2117,7 +2121,7 @@ mb2::TileProgram debug_plan(const std::vector<mb2::Block>& blocks, const mb2_swe
     m = std::min(std::max(m, mb2::kMinTileQubits), num_qubits);
     const uint32_t low = o.low_qubits < 0 ? 0u : (o.low_qubits == 0 ? mb2::kDefaultFixedLow
                                                                      : static_cast<uint32_t>(o.low_qubits));
-    mb2::TileProgram prog = mb2::plan_tile_program(blocks, num_qubits, m, low, nullptr, c64, !tc);
+    mb2::TileProgram prog = mb2::plan_tile_program(blocks, num_qubits, m, low, nullptr, c64, !tc, num_qubits <= m);
     if (tc) mb2::make_tensor_core_program(prog, blocks, mb2::tc_max_phases(m));
     return prog;
 }
@@ -2274,7 +2278,7 @@ int mb2_debug_schedule(const mb2_op* ops, uint32_t num_ops, const mb2_sweep_opti
         } else {
             const uint32_t low = o.low_qubits < 0 ? 0u : (o.low_qubits == 0 ? mb2::kDefaultFixedLow
                                                                              : static_cast<uint32_t>(o.low_qubits));
-            const mb2::TileProgram prog = mb2::plan_tile_program(blocks, num_qubits, m, low, nullptr, c64, !tc);
+            const mb2::TileProgram prog = mb2::plan_tile_program(blocks, num_qubits, m, low, nullptr, c64, !tc, num_qubits <= m);
             order = prog.order;
             order_pass = prog.order_pass;
         }
@@ -2525,7 +2529,7 @@ int mb2_estimate_sweep_time(mb2_context* ctx, const mb2_op* ops, uint32_t num_op
             }
             m = std::min(m, num_qubits);
             const mb2::TileProgram prog = mb2::plan_tile_program(blocks, num_qubits, m, mb2::kDefaultFixedLow,
-                                                                 nullptr, c64, !tc);
+                                                                 nullptr, c64, !tc, num_qubits <= m);
             size_t done = 0;
             for (const mb2::TilePass& p : prog.passes) {
                 PassCompute work;

@@ -338,10 +338,14 @@ constexpr uint8_t kParamM00Real = 4;   // ... entry (0,0) is real in every bindi
 // split: two-qubit blocks that are a permutation and a one-qubit gate run as
 // the two (off for a commuting program that make_tensor_core_program rewrites,
 // which takes permutations as it takes other blocks).
+// latency: they stay whole all the same, for one state of one tile: its sweep is
+// one CTA's chain of phases, and the parts' work is less but their phases are
+// more (12 layers of the fused RY/RZ + CX ansatz on 12 qubits 381 us whole, 426
+// in parts, planning included; on 13 qubits, four tiles, parts are the faster).
 TileProgram plan_tile_program(const std::vector<Block>& blocks, uint32_t n, uint32_t m,
                               uint32_t fixed_low = kDefaultFixedLow,
                               const std::vector<uint8_t>* parametric = nullptr, bool commuting = false,
-                              bool split = true);
+                              bool split = true, bool latency = false);
 
 // ---- device launches (kernels_*.cu) ----------------------------------------
 struct DevCtx;  // forward (engine.cpp)

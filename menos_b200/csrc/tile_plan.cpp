@@ -627,13 +627,13 @@ std::vector<PassSel> select_passes_commuting(const std::vector<Block>& blocks, u
 }
 
 TileProgram plan_tile_program(const std::vector<Block>& all, uint32_t n, uint32_t m, uint32_t fixed_low,
-                              const std::vector<uint8_t>* all_parametric, bool commuting, bool split) {
+                              const std::vector<uint8_t>* all_parametric, bool commuting, bool split, bool latency) {
     // The blocks as they are planned: origin[i] the caller's block that part i
     // belongs to, last[i] whether it completes it.
     std::vector<Block> parts;
     std::vector<uint8_t> part_flags, last;
     std::vector<uint32_t> origin;
-    for (size_t i = 0; i < all.size() && split; ++i) {
+    for (size_t i = 0; i < all.size() && split && !latency; ++i) {
         if (origin.empty() && (all[i].k != 2 || all[i].diagonal)) continue;
         Block first, second;
         const uint8_t flags = all_parametric ? (*all_parametric)[i] : uint8_t{0};
