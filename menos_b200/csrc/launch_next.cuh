@@ -6,15 +6,17 @@
 // program that a pass stages was uploaded before the sweep's first pass.
 //
 // What it saves is the gap between two launches, about 1.6 us a pass.  Beside
-// long passes the waiting CTAs cost more than that, and where passes of the
-// lean and the full complex128 kernels follow one another, whose CTAs differ in
-// size, far more: so only passes over at most 64 MiB of states are, and in
-// complex128 only those of programs without full ones (TileLaunch::behind).
+// long passes the waiting CTAs cost more than that, and where complex128 passes
+// without and with blocks of three or more qubits follow one another, whose
+// CTAs differ in size and last milliseconds, far more: so only passes over at
+// most 64 MiB of states are, and not where those meet (TileLaunch::behind).
 // Behind one another and plainly, ms, complex128: 20 brick layers at 14, 16
 // and 18 qubits 0.377 0.389, 0.442 0.455, 0.511 0.530, at 24 8.81 8.87; 6 at 28
 // 54.30 53.90; a sampled density matrix of 11 qubits 1.22 1.26; layers of H and
-// four blocks of four qubits (lean, then full passes) at 18 qubits 1.04 1.01, at
-// 22 5.07 4.93, at 26 75.8 71.5.  Complex64: the RY/RZ + CX ansatz of 10 layers
+// four blocks of four qubits (passes without, then with them) at 18 qubits 1.04
+// 1.01, at 22 5.07 4.93 (plainly only where they meet 4.88), at 26 75.8 71.5;
+// the fused RY/RZ + CX ansatz of 12 layers (lean and full passes, no such
+// blocks) at 16 qubits 0.517 0.551.  Complex64: the RY/RZ + CX ansatz of 10 layers
 // at 23 qubits 2.21 2.24; layers of H and CCX (the full kernel) at 20 1.07
 // 1.11, with CX at 26 94.9 88.0.
 #pragma once

@@ -176,7 +176,8 @@ struct TilePass {
     uint32_t param_lo = 0;
     uint32_t param_len = 0;
     bool heavy = false;  // has two-qubit dense/monomial, kDiagK or kSmem words
-    bool behind = true;  // no pass of the program keeps it from being launched behind another (launch_next.cuh)
+    bool wide = false;   // has blocks of three or more qubits, applied from shared memory (kSmem)
+    bool behind = true;  // may be launched behind the pass before it (launch_next.cuh)
     bool mapped = false; // reads or leaves the tile through a map (kPhaseMap, store_rec), or has kCross words
     bool mid = false;    // heavy, but only through general dense two-qubit words (kGen2)
     // Tensor-core form (complex64, tile_tc.cpp): the pass's composed phase

@@ -934,6 +934,7 @@ TileProgram plan_tile_program(const std::vector<Block>& all, uint32_t n, uint32_
                 map = TileMap();
             }
             g.op = TOP_SMEM;
+            pass.wide = true;
             for (uint32_t t = 0; t < b.k; ++t) g.pos[t] = static_cast<uint8_t>(local_pos(sel.smask, b.q[t]));
             if (param_flags(sel.gates[j]) & kParamBlock)
                 throw std::invalid_argument("parametric blocks wider than 2 qubits are not batched");
@@ -955,9 +956,8 @@ TileProgram plan_tile_program(const std::vector<Block>& all, uint32_t n, uint32_
         for (const TilePass& p : prog.passes) any = any || p.mapped;
         for (TilePass& p : prog.passes) p.mapped = any;
     }
-    bool full = false;
-    for (const TilePass& p : prog.passes) full = full || p.heavy;
-    for (TilePass& p : prog.passes) p.behind = commuting || !full;
+    for (size_t i = 1; i < prog.passes.size() && !commuting; ++i)
+        prog.passes[i].behind = prog.passes[i].wide == prog.passes[i - 1].wide;
     return prog;
 }
 
