@@ -274,23 +274,26 @@ __device__ __forceinline__ uint32_t group_setup(GroupShared& g, double* acc, uin
         g.cpar[t][w] = bits;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        // Kinds: 0 regular pairs, 1 Z strings, 2 other pairs.
-        auto kind = [&](uint32_t t) {
-            return g.tmode[t] == 0 ? 1u : pauli_can_hold(false, g.tdl[t], c + d) ? 0u : 2u;
-        };
-        uint32_t n = 0;
-        for (uint32_t t = 0; t < nterms && n < kPauliHeldTerms; ++t)
-            if (kind(t) == 0) g.place[n++] = t;
-        g.regular = n;
-        for (uint32_t t = 0; t < nterms; ++t)
-            if (kind(t) == 1) g.place[n++] = t;
-        g.zs = n;
-        g.held = held;
-        uint32_t past = 0;  // regular pairs past the registers' go with the others
-        for (uint32_t t = 0; t < nterms; ++t)
-            if (kind(t) == 2 || (kind(t) == 0 && past++ >= g.regular)) g.place[n++] = t;
-        g.tword[nterms] = 0;
+    if (threadIdx.x < 32) {
+        // The places, by one warp: a lane a term (kMaxGroupTerms <= 32).
+        const uint32_t t = threadIdx.x, below = (1u << t) - 1u;
+        const bool term = t < nterms, z = term && g.tmode[t] == 0;
+        const bool pair = term && !z && pauli_can_hold(false, g.tdl[t], c + d);
+        const uint32_t pairs = __ballot_sync(0xffffffffu, pair), zs = __ballot_sync(0xffffffffu, z);
+        const uint32_t first = __popc(pairs) < static_cast<int>(kPauliHeldTerms) ? __popc(pairs) : kPauliHeldTerms;
+        const bool regular = pair && __popc(pairs & below) < static_cast<int>(kPauliHeldTerms);
+        // (Regular pairs past the registers' go with the others.)
+        const uint32_t others = __ballot_sync(0xffffffffu, term && !z && !regular);
+        if (term)
+            g.place[regular ? __popc(pairs & below)
+                    : z     ? first + __popc(zs & below)
+                            : first + __popc(zs) + __popc(others & below)] = t;
+        if (t == 0) {
+            g.regular = first;
+            g.zs = first + __popc(zs);
+            g.held = held;
+            g.tword[nterms] = 0;
+        }
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < ((nterms - held) * kGroupThreads) >> paired; i += kGroupThreads) acc[i] = 0.0;
